@@ -141,7 +141,7 @@ typedef struct {
   int sweep_heavy;           /* single-vector sweeps: vertices with more entries than this
                                 get a whole warp (0 = 16)                              */
   int dense_tail;            /* largest number of final-level vertices whose substitution
-                                is replaced by a dense triangular product (0 = 4096,
+                                is replaced by a dense triangular product (0 = 2048,
                                 -1 = none; at most 8192 and n/4)                       */
   int sweep_stride;          /* 1 = one value per vertex in the one-vector sweep vectors;
                                 0 = one 32-byte sector per vertex (faster: values that
@@ -318,7 +318,8 @@ int acg_time_kernels_batch(acg_solver* h, int precision, int nrhs, int reps, acg
  * each levels[i] = L: fwd_ms[i] is the forward sweep over the tasks of levels
  * 0..L and bwd_ms[i] the backward sweep over the tasks of levels >= L (the
  * swept head; the dense tail's levels are never swept), each per launch with
- * nrhs right-hand sides; fwd_tasks[i] / bwd_tasks[i] are those tasks.  Levels
+ * nrhs right-hand sides; fwd_tasks[i] / bwd_tasks[i] are those tasks.  A level
+ * inside a block of merged levels counts with the whole block.  Levels
  * are clamped to [0, levels - 1]; times are differences of two timings, and a
  * prefix shorter than the timing noise reads 0.  The differences between points show what
  * each range of levels costs.  Diagnostic only: it uses the batch buffers, so a
@@ -369,7 +370,7 @@ int acg_serve_close(acg_server* s);
  * y_dev = LDLsolver(ldli, r_dev), as acg_ldlsolve computes it, for vectors
  * already in device memory, without allocating: every piece of scratch comes
  * from one fixed device array inside the library (ACG_NOALLOC_MAX_N vertices
- * at most, about 6.4 MB, reserved on each GPU that loads the library until
+ * at most, about 8.5 MB, reserved on each GPU that loads the library until
  * the process exits).  Meant for callers that must not allocate while they
  * solve: a serving loop whose device memory is a fixed pool sized at start-up,
  * a host runtime whose own allocator owns the GPU's memory, or a caller that

@@ -245,13 +245,16 @@ __global__ void __launch_bounds__(kSweepThreads, kb_sweep_min_blocks<T, CPL>())
     const SweepTask r2 = load_task(tasks, t + 2 * W, ntasks);
     SweepEntries<T, kBatchEntryUnroll> e1;
     load_entries<T, true, false, kBatchEntryUnroll>(e1, r1, lane, idx, coef, coef, coef);
-    const int gw = e0.gw;  // 32 for a heavy task, 8 for a light one (uniform per warp)
+    const bool active = e0.active(lane);
+    const int gw = e0.gw();  // 32 for a heavy task, 8 for a light one (uniform per warp)
     const int k0 = e0.k0 - (gw == 32 ? lane : gl);  // first entry of this lane's vertex
     T acc[CPL];
 #pragma unroll
     for (int j = 0; j < CPL; ++j) acc[j] = T(0);
     Row<T, CPL> a;
-    if (e0.active && (gw == 8 || lane < 8)) {
+#pragma unroll
+    for (int j = 0; j < CPL; ++j) a.v[j] = T(0);
+    if (active && e0.kind() != kRowFinal && (gw == 8 || lane < 8)) {
       if (kForward) {
         ld_stream_row<CPL>(a.v, aux + (size_t)e0.v * kp + gl * CPL, pol);
       } else {
@@ -261,25 +264,19 @@ __global__ void __launch_bounds__(kSweepThreads, kb_sweep_min_blocks<T, CPL>())
         for (int j = 0; j < CPL; ++j) a.v[j] = g * a.v[j];
       }
     }
-    int rounds = e0.active ? (e0.k1 - k0 + gw - 1) / gw : 0;
+    int rounds = active ? (e0.k1 - k0 + gw - 1) / gw : 0;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) rounds = max(rounds, __shfl_xor_sync(0xffffffffu, rounds, o));
+    int nid = e0.id[0];
+    T nc = e0.c[0];
     for (int j = 0; j < rounds; ++j) {
-      int myid;
-      T myc;
-      if (j < kBatchEntryUnroll) {
-        myid = e0.id[0];
-        myc = e0.c[0];
-#pragma unroll
-        for (int q = 1; q < kBatchEntryUnroll; ++q)
-          if (q == j) {
-            myid = e0.id[q];
-            myc = e0.c[q];
-          }
-      } else {
-        const int k = e0.k0 + j * gw;
-        myid = (e0.active && k < e0.k1) ? __ldg(&idx[k]) : -1;
-        myc = (e0.active && k < e0.k1) ? __ldg(&coef[k]) : T(0);
+      const int myid = nid;
+      const T myc = nc;
+      {  // the next round's entry, on its way while this round's rows are
+        const int k = e0.k0 + (j + 1) * gw;
+        const bool more = active && k < e0.k1;
+        nid = more ? __ldg(&idx[k]) : -1;
+        nc = more ? __ldg(&coef[k]) : T(0);
       }
 #pragma unroll
       for (int l0 = 0; l0 < 8; l0 += EB) {
@@ -348,19 +345,23 @@ __global__ void __launch_bounds__(kSweepThreads, kb_sweep_min_blocks<T, CPL>())
         acc[q] += __shfl_xor_sync(0xffffffffu, acc[q], 16);
       }
     }
-    if (e0.active && (gw == 8 || lane < 8)) {
+    if (active && (gw == 8 || lane < 8)) {
       T res[CPL];
 #pragma unroll
       for (int q = 0; q < CPL; ++q) res[q] = a.v[q] + acc[q];
-      st_row<CPL>(out + (size_t)e0.v * kp + gl * CPL, res);
+      st_row<CPL>(out + (size_t)e0.slot() * kp + gl * CPL, res);
       if (mark) {
-        // the vertex's row of the other sweep's vector is dead from here on
+        // the same slot of the other sweep's vector is dead from here on
         // (forward: y, read by no one until the backward rewrites it;
-        // backward: s, whose only reader was this task): mark it pending
-        // for the next sweep instead of a separate pass over the vector
+        // backward: s, whose reader was this task or one it waited for): mark
+        // it pending for the next sweep instead of a separate pass over the
+        // vector.  The other sweep uses the work slots of the block's other
+        // end, so a plain row of a block marks its vertex's work slot too.
 #pragma unroll
         for (int q = 0; q < CPL; ++q) res[q] = pending_value<T>();
-        st_stream_row<CPL>(mark + (size_t)e0.v * kp + gl * CPL, res, pol);
+        st_stream_row<CPL>(mark + (size_t)e0.slot() * kp + gl * CPL, res, pol);
+        if (e0.kind() == kRowPlain && e0.delta)
+          st_stream_row<CPL>(mark + (size_t)(e0.v + e0.delta) * kp + gl * CPL, res, pol);
       }
     }
     e0 = e1;
@@ -1178,16 +1179,29 @@ __global__ void __launch_bounds__(kVecThreads) kb_gather_in(int n, int kp, const
   }
 }
 
+// Marks the work rows [n, nslots) of the batched sweep vectors pending.
+template <typename T>
+__device__ __forceinline__ void mark_work_rows(int n, int nslots, int kp, T* s, T* y) {
+  const T pv = pending_value<T>();
+  const size_t S = (size_t)gridDim.x * blockDim.x;
+  for (size_t i = (size_t)n * kp + blockIdx.x * blockDim.x + threadIdx.x; i < (size_t)nslots * kp; i += S) {
+    s[i] = pv;
+    y[i] = pv;
+  }
+}
+
 // bm = b - mean; r = bm (as T); x0 = 0; s, y pending; per-column |b| and reset.
 template <typename T>
 __global__ void __launch_bounds__(kVecThreads) kb_center(int n, int kp, double* __restrict__ bm, T* __restrict__ r,
                                                          T* __restrict__ x0, T* __restrict__ s_out, T* __restrict__ y_out,
-                                                         PcgState* st, BatchShared* bs, double* partials, LoopCtl ctl) {
+                                                         PcgState* st, BatchShared* bs, double* partials, LoopCtl ctl,
+                                                         int nslots) {
   const size_t N = (size_t)n * kp;
   const size_t i0 = blockIdx.x * blockDim.x + threadIdx.x;
   const int c = (int)(i0 % kp);
   const double mu = st[c].mean;
   const T pend = pending_value<T>();
+  if (s_out) mark_work_rows(n, nslots, kp, s_out, y_out);
   double acc[2] = {0.0, 0.0};
   for (size_t i = i0; i < N; i += (size_t)gridDim.x * blockDim.x) {
     const double v = bm[i] - mu;
@@ -1354,8 +1368,10 @@ template <typename T>
 __global__ void __launch_bounds__(kVecThreads) kb_outer_prep(int n, int kp, const double* __restrict__ r64,
                                                              T* __restrict__ rin, T* __restrict__ x0,
                                                              T* __restrict__ s_out, T* __restrict__ y_out, PcgState* st,
-                                                             BatchShared* bs, double* partials, LoopCtl inner_ctl) {
+                                                             BatchShared* bs, double* partials, LoopCtl inner_ctl,
+                                                             int nslots) {
   const size_t N = (size_t)n * kp;
+  mark_work_rows(n, nslots, kp, s_out, y_out);
   const size_t i0 = blockIdx.x * blockDim.x + threadIdx.x;
   const int c = (int)(i0 % kp);
   const bool act = !st[c].outer_done;

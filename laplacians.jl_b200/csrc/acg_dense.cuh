@@ -34,7 +34,7 @@ constexpr int kDenseRows = 64;
 constexpr int kDenseChunk = 256;
 constexpr int kDenseSub = 64;
 constexpr int kDenseThreads = 256;
-constexpr int kDenseDefaultK = 4096;  // largest tail chosen automatically
+constexpr int kDenseDefaultK = 2048;  // largest tail chosen automatically
 constexpr int kDenseMaxK = 8192;      // largest tail accepted
 constexpr int kDenseMinLevels = 8;    // fewer tail levels than this: no dense tail
 

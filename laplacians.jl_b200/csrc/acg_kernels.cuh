@@ -23,6 +23,8 @@
 
 #include <climits>
 
+#include "acg_plan.h"
+
 namespace acg {
 
 constexpr int kMaxPartialBlocks = 2048;
@@ -347,7 +349,8 @@ __global__ void __launch_bounds__(kThinThreads, 1) k_thin(int l0, int l1, const 
 // it, so the value is its own ready flag.  Warps take tasks round-robin in
 // level order (task t by warp t mod W); a task's inputs come from strictly
 // earlier tasks, so with all warps co-resident (cooperative launch) the
-// earliest unfinished task can always proceed.  Each wait polls the L2 copy
+// earliest unfinished task can always proceed.  The tasks are the rows of the
+// sweep plan (acg_plan.h), which merges levels into blocks.  Each wait polls the L2 copy
 // with relaxed GPU-scope loads and gives up after spin_limit polls (a launch
 // argument, kSpinLimit unless the solver's options set another), raising
 // PcgState::sweep_error instead of hanging.
@@ -414,22 +417,31 @@ __device__ __forceinline__ T wait_value(const T* p, PcgState* st, int poll_mode,
   return is_pending(x) ? wait_value_slow(p, st, poll_mode, spin_limit) : x;
 }
 
-// A task record (32 bytes): {first vertex, (count << 1) | heavy, p[0..4]} with
-// p[i] = ptr[first + i], so a lane finds its entry range without another
-// dependent load.  A heavy task is one vertex on 32 lanes, a light task up to
-// 4 consecutive vertices of one level on 8 lanes each.
+// A task record (32 bytes): {first vertex, kind << 4 | count << 1 | heavy,
+// p[0..4], delta}: the task's rows are p[i]..p[i+1], so a lane finds its entry
+// range without another dependent load.  A heavy task is one row on 32 lanes,
+// a light task up to 4 rows of consecutive vertices on 8 lanes each.  The
+// kinds (SweepRowKind) say whether a row adds the vertex's own term and where
+// its value goes: slot v, or v + delta for a block's work values.  A plain
+// row with a delta is a block's first level, whose work slot is unused.
 struct alignas(16) SweepTask {
-  int v, cnt_heavy;
-  int p[6];
+  int v, info;
+  int p[5];
+  int delta;
 };
 
 template <typename T, int U = kEntryUnroll>
 struct SweepEntries {
-  int v, k0, k1, gw;
-  bool active;
+  int v, k0, k1, info, delta;
   int id[U];
   T c[U];
   T a, own;
+  __device__ __forceinline__ int gw() const { return (info & 1) ? 32 : 8; }  // uniform: one task per warp
+  __device__ __forceinline__ int kind() const { return info >> 4; }
+  __device__ __forceinline__ bool active(int lane) const {
+    return ((info & 1) ? 0 : (lane >> 3)) < ((info >> 1) & 7);
+  }
+  __device__ __forceinline__ int slot() const { return kind() == kRowWork ? v + delta : v; }
 };
 
 __device__ __forceinline__ SweepTask load_task(const SweepTask* __restrict__ tasks, int t, int ntasks) {
@@ -437,12 +449,12 @@ __device__ __forceinline__ SweepTask load_task(const SweepTask* __restrict__ tas
   if (t < ntasks) {
     const int4* q = reinterpret_cast<const int4*>(tasks + t);
     const int4 x = __ldg(q), y = __ldg(q + 1);
-    r.v = x.x; r.cnt_heavy = x.y; r.p[0] = x.z; r.p[1] = x.w;
-    r.p[2] = y.x; r.p[3] = y.y; r.p[4] = y.z; r.p[5] = y.w;
+    r.v = x.x; r.info = x.y; r.p[0] = x.z; r.p[1] = x.w;
+    r.p[2] = y.x; r.p[3] = y.y; r.p[4] = y.z; r.delta = y.w;
   } else {
-    r.v = 0; r.cnt_heavy = 0;
+    r.v = 0; r.info = 0; r.delta = 0;
 #pragma unroll
-    for (int i = 0; i < 6; ++i) r.p[i] = 0;
+    for (int i = 0; i < 5; ++i) r.p[i] = 0;
   }
   return r;
 }
@@ -451,29 +463,85 @@ template <typename T, bool kForward, bool kLoadAux = true, int U = kEntryUnroll>
 __device__ __forceinline__ void load_entries(SweepEntries<T, U>& e, const SweepTask& r, int lane,
                                              const int* __restrict__ idx, const T* __restrict__ coef,
                                              const T* __restrict__ aux, const T* __restrict__ sfwd, int vs = 1) {
-  const bool heavy = r.cnt_heavy & 1;
-  const int cnt = r.cnt_heavy >> 1;
+  const bool heavy = r.info & 1;
+  const int cnt = (r.info >> 1) & 7;
   const int sub = heavy ? 0 : (lane >> 3);
   const int gw = heavy ? 32 : 8;
   const int gl = heavy ? lane : (lane & 7);
-  e.active = sub < cnt;
-  e.gw = gw;
+  const bool active = sub < cnt;
   e.v = r.v + sub;
+  e.info = r.info;
+  e.delta = r.delta;
   int k0 = 0, k1 = 0;
 #pragma unroll
   for (int i = 0; i < 4; ++i)
     if (i == sub) { k0 = r.p[i]; k1 = r.p[i + 1]; }
-  if (!e.active) k0 = k1 = 0;
+  if (!active) k0 = k1 = 0;
   e.k0 = k0 + gl;
   e.k1 = k1;
-  e.a = (kLoadAux && e.active) ? __ldg(&aux[e.v]) : T(0);
-  e.own = (kLoadAux && !kForward && e.active) ? __ldg(&sfwd[(size_t)e.v * vs]) : T(0);
+  const bool term = kLoadAux && active && e.kind() != kRowFinal;
+  e.a = term ? __ldg(&aux[e.v]) : T(0);
+  e.own = (!kForward && term) ? __ldg(&sfwd[(size_t)e.v * vs]) : T(0);
 #pragma unroll
   for (int j = 0; j < U; ++j) {
     const int k = e.k0 + j * gw;
     e.id[j] = k < k1 ? __ldg(&idx[k]) : -1;
     e.c[j] = k < k1 ? __ldg(&coef[k]) : T(0);
   }
+}
+
+// acc += c[j] * out[id[j]] over a lane's entries in turn (id < 0: none), waiting
+// for the values still pending.  The loads of all entries are issued before any is
+// checked.  FP32: inputs seen pending are polled again together (all polls of
+// a round in flight), not one wait after another; bounded like every wait.
+// Single-vector mixed solve on the 1M grid: 39.5 -> 36.9 ms.  FP64 keeps the
+// waits one by one: with joint polls, 256 graphs in one FP64 launch (many
+// graphs, thousands of tasks per level) went from 146.7 to 156.3 ms.
+template <typename T, int U>
+__device__ __forceinline__ void gather_entries(T& acc, const int (&id)[U], const T (&c)[U], const T* out, int vs,
+                                               PcgState* st, int poll_mode, unsigned spin_limit) {
+  T xv[U];
+#pragma unroll
+  for (int j = 0; j < U; ++j) xv[j] = id[j] >= 0 ? ld_relaxed(&out[(size_t)id[j] * vs]) : T(0);
+  unsigned pend = 0;
+  if constexpr (sizeof(T) == 4) {
+#pragma unroll
+    for (int j = 0; j < U; ++j)
+      if (id[j] >= 0 && is_pending(xv[j])) pend |= 1u << j;
+  } else {
+#pragma unroll
+    for (int j = 0; j < U; ++j)
+      if (id[j] >= 0 && is_pending(xv[j])) xv[j] = wait_value_slow(&out[(size_t)id[j] * vs], st, poll_mode, spin_limit);
+  }
+  unsigned int sleep_ns = 32;
+  for (unsigned int spins = 1; pend; ++spins) {
+    if (poll_mode == 0) {
+      if (spins >= 64) __nanosleep(64);
+    } else if (poll_mode == 2) {
+      if (spins >= 4) {
+        __nanosleep(sleep_ns);
+        if (sleep_ns < 1024) sleep_ns <<= 1;
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < U; ++j)
+      if ((pend >> j) & 1u) xv[j] = ld_relaxed(&out[(size_t)id[j] * vs]);
+    unsigned still = 0;
+#pragma unroll
+    for (int j = 0; j < U; ++j)
+      if (((pend >> j) & 1u) && is_pending(xv[j])) still |= 1u << j;
+    pend = still;
+    if (pend && (((spins & 1023u) == 0 && *((volatile int*)&st->sweep_error)) || spins >= spin_limit)) {
+      atomicExch(&st->sweep_error, 1);
+#pragma unroll
+      for (int j = 0; j < U; ++j)
+        if ((pend >> j) & 1u) xv[j] = T(0);
+      break;
+    }
+  }
+#pragma unroll
+  for (int j = 0; j < U; ++j)
+    if (id[j] >= 0) acc += c[j] * xv[j];
 }
 
 // Warp w runs tasks w, w+W, w+2W, ... (W warps in the grid).  Task records
@@ -499,61 +567,24 @@ __global__ void __launch_bounds__(kSweepThreads) k_sweep(int ntasks, const Sweep
     const SweepTask r2 = load_task(tasks, t + 2 * W, ntasks);
     SweepEntries<T> e1;
     load_entries<T, kForward>(e1, r1, lane, idx, coef, aux, sfwd, vs);
-    const int gw = e0.gw;  // uniform across the warp: one task per warp
+    const int gw = e0.gw();
     T acc = T(0);
-    // issue the loads of all prefetched entries before checking any of them
-    T xv[kEntryUnroll];
+    // a row longer than the prefetched entries goes on in chunks of the same
+    // size: one value round trip per chunk, not per round of entries
+    for (int k = e0.k0; k < e0.k1;) {
+      gather_entries<T, kEntryUnroll>(acc, e0.id, e0.c, out, vs, st, poll_mode, spin_limit);
+      k += kEntryUnroll * gw;
+      if (k >= e0.k1) break;
 #pragma unroll
-    for (int j = 0; j < kEntryUnroll; ++j) xv[j] = e0.id[j] >= 0 ? ld_relaxed(&out[(size_t)e0.id[j] * vs]) : T(0);
-    // FP32: inputs seen pending are polled again together (all polls of a
-    // round in flight), not one wait after another; bounded like every wait.
-    // Single-vector mixed solve on the 1M grid: 39.5 -> 36.9 ms.  FP64 keeps
-    // the waits one by one: with joint polls, 256 graphs in one FP64 launch
-    // (many graphs, thousands of tasks per level) went from 146.7 to 156.3 ms.
-    unsigned pend = 0;
-    if constexpr (sizeof(T) == 4) {
-#pragma unroll
-      for (int j = 0; j < kEntryUnroll; ++j)
-        if (e0.id[j] >= 0 && is_pending(xv[j])) pend |= 1u << j;
-    } else {
-#pragma unroll
-      for (int j = 0; j < kEntryUnroll; ++j)
-        if (e0.id[j] >= 0 && is_pending(xv[j])) xv[j] = wait_value_slow(&out[(size_t)e0.id[j] * vs], st, poll_mode, spin_limit);
-    }
-    unsigned int sleep_ns = 32;
-    for (unsigned int spins = 1; pend; ++spins) {
-      if (poll_mode == 0) {
-        if (spins >= 64) __nanosleep(64);
-      } else if (poll_mode == 2) {
-        if (spins >= 4) {
-          __nanosleep(sleep_ns);
-          if (sleep_ns < 1024) sleep_ns <<= 1;
-        }
-      }
-#pragma unroll
-      for (int j = 0; j < kEntryUnroll; ++j)
-        if ((pend >> j) & 1u) xv[j] = ld_relaxed(&out[(size_t)e0.id[j] * vs]);
-      unsigned still = 0;
-#pragma unroll
-      for (int j = 0; j < kEntryUnroll; ++j)
-        if (((pend >> j) & 1u) && is_pending(xv[j])) still |= 1u << j;
-      pend = still;
-      if (pend && (((spins & 1023u) == 0 && *((volatile int*)&st->sweep_error)) || spins >= spin_limit)) {
-        atomicExch(&st->sweep_error, 1);
-#pragma unroll
-        for (int j = 0; j < kEntryUnroll; ++j)
-          if ((pend >> j) & 1u) xv[j] = T(0);
-        break;
+      for (int j = 0; j < kEntryUnroll; ++j) {
+        const int kk = k + j * gw;
+        e0.id[j] = kk < e0.k1 ? __ldg(&idx[kk]) : -1;
+        e0.c[j] = kk < e0.k1 ? __ldg(&coef[kk]) : T(0);
       }
     }
-#pragma unroll
-    for (int j = 0; j < kEntryUnroll; ++j)
-      if (e0.id[j] >= 0) acc += e0.c[j] * xv[j];
-    for (int k = e0.k0 + kEntryUnroll * gw; k < e0.k1; k += gw)
-      acc += __ldg(&coef[k]) * wait_value(&out[(size_t)__ldg(&idx[k]) * vs], st, poll_mode, spin_limit);
     __syncwarp();  // reconverge after the divergent waits before the shuffles
     acc = group_sum_w(acc, gw);
-    if (e0.active && (lane & (gw - 1)) == 0) st_relaxed(&out[(size_t)e0.v * vs], kForward ? e0.a + acc : e0.a * e0.own + acc);
+    if (e0.active(lane) && (lane & (gw - 1)) == 0) st_relaxed(&out[(size_t)e0.slot() * vs], kForward ? e0.a + acc : e0.a * e0.own + acc);
     e0 = e1;
     r1 = r2;
   }
@@ -607,7 +638,7 @@ __global__ void __launch_bounds__(kTailThreads, 1) k_tail(int NL, int V0, int NV
     // the first task of this warp came through the pipeline; further tasks of
     // a level (more than 32 of them is excluded by the host) never occur
     if (w < cur.y) {
-      const int gw = e0.gw;
+      const int gw = e0.gw();
       T acc = T(0);
       T xv[kEntryUnroll];
 #pragma unroll
@@ -622,7 +653,7 @@ __global__ void __launch_bounds__(kTailThreads, 1) k_tail(int NL, int V0, int NV
         acc += __ldg(&coef[k]) * (id >= V0 ? sv[id - V0] : out[id]);
       }
       acc = group_sum_w(acc, gw);
-      if (e0.active && (lane & (gw - 1)) == 0) {
+      if (e0.active(lane) && (lane & (gw - 1)) == 0) {
         const T res = kForward ? e0.a + acc : e0.a * e0.own + acc;
         sv[e0.v - V0] = res;
         out[e0.v] = res;
@@ -640,11 +671,22 @@ constexpr size_t tail_smem_bytes(int nv, int nl) {
 }
 
 template <typename T>
-__global__ void k_fill_pending(int n, T* a, T* b, int vs = 1) {
+__global__ void k_fill_pending(size_t n, T* a, T* b, int vs = 1) {
   const T pv = pending_value<T>();
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    a[(size_t)i * vs] = pv;
-    if (b) b[(size_t)i * vs] = pv;
+  for (size_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    a[i * vs] = pv;
+    if (b) b[i * vs] = pv;
+  }
+}
+
+// Marks the work slots [n, nslots) of the one-vector sweep vectors pending
+// (the kernels that mark the n values of s and y).
+template <typename T>
+__device__ __forceinline__ void mark_work_slots(int n, int nslots, T* s, T* y, int vs) {
+  const T pv = pending_value<T>();
+  for (int i = n + blockIdx.x * blockDim.x + threadIdx.x; i < nslots; i += gridDim.x * blockDim.x) {
+    s[(size_t)i * vs] = pv;
+    y[(size_t)i * vs] = pv;
   }
 }
 

@@ -188,9 +188,11 @@ __global__ void __launch_bounds__(kVecThreads) k_spmv_pq(int n, const int* __res
 template <typename T>
 __global__ void __launch_bounds__(kVecThreads) k_update(int n, T* x3, const T* __restrict__ p, const T* __restrict__ q,
                                                         T* __restrict__ r, T* __restrict__ s_out, T* __restrict__ y_out,
-                                                        PcgState* st, double* partials, LoopCtl ctl, int vs) {
+                                                        PcgState* st, double* partials, LoopCtl ctl, int vs,
+                                                        int nslots) {
   if (st->done) return;
   const T pend = pending_value<T>();
+  mark_work_slots(n, nslots, s_out, y_out, vs);
   const double al = st->alpha;
   const T* xc = x3 + (size_t)st->xcur * n;
   T* xn = x3 + (size_t)st->xnext * n;
@@ -271,9 +273,10 @@ __global__ void __launch_bounds__(kVecThreads) k_gather_in(int n, const int* __r
 template <typename T>
 __global__ void __launch_bounds__(kVecThreads) k_center(int n, double* __restrict__ bm, T* __restrict__ r, T* __restrict__ x0,
                                                         T* __restrict__ s_out, T* __restrict__ y_out, PcgState* st,
-                                                        double* partials, LoopCtl ctl, int vs) {
+                                                        double* partials, LoopCtl ctl, int vs, int nslots) {
   const double mu = st->mean;
   const T pend = pending_value<T>();
+  if (s_out) mark_work_slots(n, nslots, s_out, y_out, vs);
   double acc[2] = {0.0, 0.0};
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     const double v = bm[i] - mu;
@@ -361,9 +364,11 @@ __global__ void __launch_bounds__(kVecThreads) k_scatter_out(int n, const int* _
 template <typename T>
 __global__ void __launch_bounds__(kVecThreads) k_outer_prep(int n, const double* __restrict__ r64, T* __restrict__ rin,
                                                             T* __restrict__ x0, T* __restrict__ s_out, T* __restrict__ y_out,
-                                                            PcgState* st, double* partials, LoopCtl inner_ctl, int vs) {
+                                                            PcgState* st, double* partials, LoopCtl inner_ctl, int vs,
+                                                           int nslots) {
   const double inv = 1.0 / st->scale;
   const T pend = pending_value<T>();
+  mark_work_slots(n, nslots, s_out, y_out, vs);
   double acc[2] = {0.0, 0.0};
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     const T v = (T)(r64[i] * inv);

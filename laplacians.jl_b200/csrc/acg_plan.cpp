@@ -1,0 +1,336 @@
+#include "acg_plan.h"
+
+#include <algorithm>
+#include <cmath>
+#include <thread>
+
+namespace acg {
+namespace {
+
+constexpr int kMaxBlockLevels = 256;
+// a row's own cost in entries: its task record, its right-hand side and store
+constexpr double kRowCost = 4.0;
+
+// A block of levels [l0, l1); rows of M_B (its vertices in level order) when it
+// has several levels.
+struct Block {
+  int l0, l1;
+  std::vector<int> vert;       // vertices, level by level
+  std::vector<int> ptr, idx;   // M_B by row, internal vertex ids ascending
+  std::vector<double> val;
+};
+
+struct Shared {
+  const SweepDag& d;
+  const SweepCost* cost;
+  std::vector<int> lev, mark;
+  std::vector<int> where;  // a vertex's row in the block being grown
+  std::vector<double> acc;
+  std::vector<double> level_cost;  // rows and entries of a level, both directions averaged
+};
+
+// Greedy blocks over the levels [la, lb): from each level on, the length with
+// the largest saving in hand-overs.
+void partition(Shared& s, int la, int lb, std::vector<Block>& out) {
+  const SweepDag& d = s.d;
+  const auto& runs = *d.level_runs;
+  const double A = s.cost->entries_per_hop;
+  std::vector<int> cols;
+  int stamp_at = -1;
+  for (int l = la; l < lb;) {
+    Block b;
+    b.l0 = l;
+    b.ptr.push_back(0);
+    double inner = 0.0, all = 0.0, best = 0.0;
+    size_t best_verts = 0, first = 0;
+    int best_len = 1, longest = 0;
+    for (int len = 1; l + len <= lb && len <= kMaxBlockLevels; ++len) {
+      const int L = l + len - 1;
+      size_t last = 0;
+      all += s.level_cost[L];
+      // more entries than the block's levels are worth: no gain from here on
+      const double most = A * len + all;
+      bool over = false;
+      for (const auto& r : runs[L]) {
+        for (int v = r.first; v < r.second && !over; ++v) {
+          ++last;
+          stamp_at = v;
+          cols.clear();
+          cols.push_back(v);
+          s.mark[v] = stamp_at;
+          s.acc[v] = 1.0;
+          for (int k = (*d.fptr)[v + 1] - 1; k >= (*d.fptr)[v]; --k) {
+            const int u = (*d.fidx)[k];
+            if (s.lev[u] < l) break;  // inputs ascend by level
+            const double c = (*d.fc)[k];
+            inner += 1.0;
+            const int ru = s.where[u];
+            for (int e = b.ptr[ru]; e < b.ptr[ru + 1]; ++e) {
+              const int w = b.idx[e];
+              if (s.mark[w] != stamp_at) {
+                s.mark[w] = stamp_at;
+                s.acc[w] = 0.0;
+                cols.push_back(w);
+              }
+              s.acc[w] += c * b.val[e];
+            }
+          }
+          std::sort(cols.begin(), cols.end());
+          s.where[v] = (int)b.vert.size();
+          b.vert.push_back(v);
+          for (int w : cols) {
+            b.idx.push_back(w);
+            b.val.push_back(s.acc[w]);
+            s.mark[w] = -1;
+          }
+          b.ptr.push_back((int)b.idx.size());
+          longest = std::max(longest, (int)cols.size());
+          over = (double)b.idx.size() > most;
+        }
+        if (over) break;
+      }
+      if (over) break;
+      if (len == 1) first = last;
+      if (len >= 2) {
+        const double ends = 0.5 * (double)(first + last);
+        const double work = all - inner;
+        const double fin = (double)b.idx.size() - ends + kRowCost * ((double)b.vert.size() - ends);
+        const double rounds = std::floor((double)(longest - 1) / s.cost->row_entries);
+        // a level costs a hand-over and its entries; the block two hand-overs
+        const double gain = (len - 2) - (work + fin - all) / A - s.cost->row_round * rounds;
+        if (gain > best) {
+          best = gain;
+          best_len = len;
+          best_verts = b.vert.size();
+        } else if ((best == 0.0 && len >= 4) || gain < best - std::max(2.0, 0.25 * best)) {
+          break;
+        }
+      }
+    }
+    b.l1 = l + best_len;
+    if (best_len == 1) {
+      b.vert.clear();
+      b.ptr.clear();
+      b.idx.clear();
+      b.val.clear();
+    } else {
+      b.vert.resize(best_verts);
+      b.idx.resize(b.ptr[best_verts]);
+      b.val.resize(b.ptr[best_verts]);
+      b.ptr.resize(best_verts + 1);
+      b.idx.shrink_to_fit();
+      b.val.shrink_to_fit();
+    }
+    out.push_back(std::move(b));
+    l = out.back().l1;
+  }
+}
+
+// The vertex ranges of levels [l0, l1), one per graph (a graph's vertices are
+// numbered level by level, so consecutive levels join up).
+std::vector<std::pair<int, int>> ranges(const SweepDag& d, int l0, int l1) {
+  std::vector<std::pair<int, int>> out;
+  for (int l = l0; l < l1; ++l)
+    for (const auto& r : (*d.level_runs)[l])
+      if (r.second > r.first) out.push_back(r);
+  std::sort(out.begin(), out.end());
+  size_t w = 0;
+  for (size_t i = 0; i < out.size(); ++i) {
+    if (w && out[w - 1].second == out[i].first)
+      out[w - 1].second = out[i].second;
+    else
+      out[w++] = out[i];
+  }
+  out.resize(w);
+  return out;
+}
+
+}  // namespace
+
+SweepPlan build_sweep_plan(const SweepDag& d, const SweepCost& cost, bool merge) {
+  Shared s{d, &cost, std::vector<int>(d.n, 0), std::vector<int>(d.n, -1), std::vector<int>(d.n, 0),
+           std::vector<double>(d.n, 0.0), std::vector<double>(d.nlev, 0.0)};
+  const auto& runs = *d.level_runs;
+  const int head = std::min(d.tail_level, d.nlev);
+  for (int l = 0; l < d.nlev; ++l)
+    for (const auto& r : runs[l]) {
+      for (int v = r.first; v < r.second; ++v) s.lev[v] = l;
+      const double in = (*d.fptr)[r.second] - (*d.fptr)[r.first], outs = (*d.bptr)[r.second] - (*d.bptr)[r.first];
+      s.level_cost[l] += 0.5 * (in + outs) + kRowCost * (r.second - r.first);
+    }
+  // Blocks: stretches of levels of about equal cost are partitioned by their
+  // own thread (the stretches depend on the graph alone).
+  std::vector<Block> blocks;
+  // A DAG that fills in fast is merged less: the rows of M_B may hold at most
+  // six times the factor's entries (or 32M), else the blocks are cut again with
+  // dearer entries.
+  const size_t most = std::max((size_t)6 * d.fidx->size(), (size_t)32 << 20);
+  SweepCost c = cost;
+  s.cost = &c;
+  for (int round = 0; merge && round < 6; ++round, c.entries_per_hop *= 0.25) {
+    blocks.clear();
+    double total = 0.0;
+    for (int l = 0; l < head; ++l) total += s.level_cost[l];
+    const int stretches = std::max(1, std::min(8, (int)(total / 1e6)));
+    std::vector<int> cut{0};
+    double sum = 0.0;
+    for (int l = 0; l < head; ++l) {
+      sum += s.level_cost[l];
+      if ((int)cut.size() < stretches && sum >= total * (double)cut.size() / stretches) cut.push_back(l + 1);
+    }
+    cut.push_back(head);
+    std::vector<std::vector<Block>> parts(cut.size() - 1);
+    std::vector<std::thread> pool;
+    for (size_t i = 1; i < parts.size(); ++i)
+      pool.emplace_back([&, i]() { partition(s, cut[i], cut[i + 1], parts[i]); });
+    partition(s, cut[0], cut[1], parts[0]);
+    for (auto& t : pool) t.join();
+    size_t held = 0;
+    for (auto& p : parts)
+      for (auto& b : p) {
+        held += b.idx.size();
+        blocks.push_back(std::move(b));
+      }
+    if (held <= most) break;
+    if (round == 5) merge = false;
+  }
+  if (!merge) {
+    blocks.clear();
+    for (int l = 0; l < head; ++l) blocks.push_back(Block{l, l + 1, {}, {}, {}, {}});
+  }
+  SweepPlan plan;
+  plan.blocks = (int)blocks.size();
+  plan.nslots = d.n;
+
+  // slots of the blocks' work values
+  std::vector<int> delta(d.n, 0);
+  for (const Block& b : blocks) {
+    if (b.l1 - b.l0 < 2) continue;
+    for (const auto& r : ranges(d, b.l0, b.l1)) {
+      for (int v = r.first; v < r.second; ++v) delta[v] = plan.nslots - r.first;
+      plan.nslots += r.second - r.first;
+    }
+  }
+  auto add_entry = [](SweepRows& R, int slot, double c) {
+    R.idx.push_back(slot);
+    R.coef.push_back(c);
+  };
+  auto add_run = [](SweepRows& R, int v0, int count, int kind, int del) {
+    R.runs.push_back(SweepRun{v0, count, kind, del, (int)R.ptr.size() - 1});
+  };
+  SweepRows &F = plan.fwd, &B = plan.bwd;
+  F.ptr.push_back(0);
+  B.ptr.push_back(0);
+  F.upto.assign(d.nlev, 0);
+  B.upto.assign(d.nlev, 0);
+
+  // ---- forward: blocks upwards, then the dense tail's rows (head inputs only)
+  for (const Block& b : blocks) {
+    const bool multi = b.l1 - b.l0 > 1;
+    for (const auto& r : ranges(d, b.l0, b.l0 + 1)) {
+      add_run(F, r.first, r.second - r.first, kRowPlain, multi ? delta[r.first] : 0);
+      for (int v = r.first; v < r.second; ++v) {
+        for (int k = (*d.fptr)[v]; k < (*d.fptr)[v + 1]; ++k) add_entry(F, (*d.fidx)[k], (*d.fc)[k]);
+        F.ptr.push_back((int)F.idx.size());
+      }
+    }
+    F.upto[b.l0] = (int)F.runs.size();
+    if (!multi) continue;
+    const auto rest = ranges(d, b.l0 + 1, b.l1);
+    for (const auto& r : rest) {
+      add_run(F, r.first, r.second - r.first, kRowWork, delta[r.first]);
+      for (int v = r.first; v < r.second; ++v) {
+        for (int k = (*d.fptr)[v]; k < (*d.fptr)[v + 1]; ++k) {
+          if (s.lev[(*d.fidx)[k]] >= b.l0) break;
+          add_entry(F, (*d.fidx)[k], (*d.fc)[k]);
+        }
+        F.ptr.push_back((int)F.idx.size());
+      }
+    }
+    for (size_t i = 0; i < b.vert.size(); ++i) s.where[b.vert[i]] = (int)i;
+    for (const auto& r : rest) {
+      add_run(F, r.first, r.second - r.first, kRowFinal, delta[r.first]);
+      for (int v = r.first; v < r.second; ++v) {
+        const int row = s.where[v];
+        for (int e = b.ptr[row]; e < b.ptr[row + 1]; ++e) {
+          const int u = b.idx[e];
+          add_entry(F, s.lev[u] == b.l0 ? u : u + delta[u], b.val[e]);
+        }
+        F.ptr.push_back((int)F.idx.size());
+      }
+    }
+    for (int l = b.l0 + 1; l < b.l1; ++l) F.upto[l] = (int)F.runs.size();
+  }
+  if (head < d.nlev) {
+    for (const auto& r : ranges(d, head, d.nlev)) {
+      add_run(F, r.first, r.second - r.first, kRowPlain, 0);
+      for (int v = r.first; v < r.second; ++v) {
+        for (int k = (*d.fptr)[v]; k < (*d.fptr)[v + 1]; ++k) add_entry(F, (*d.fidx)[k], (*d.fc)[k]);
+        F.ptr.push_back((int)F.idx.size());
+      }
+    }
+    for (int l = head; l < d.nlev; ++l) F.upto[l] = (int)F.runs.size();
+  }
+
+  // ---- backward: blocks downwards; a block's last level is its first step
+  std::vector<int> tptr, tidx;
+  std::vector<double> tval;
+  for (auto it = blocks.rbegin(); it != blocks.rend(); ++it) {
+    const Block& b = *it;
+    const int top = b.l1 - 1;
+    const bool multi = top > b.l0;
+    for (const auto& r : ranges(d, top, b.l1)) {
+      add_run(B, r.first, r.second - r.first, kRowPlain, multi ? delta[r.first] : 0);
+      for (int v = r.first; v < r.second; ++v) {
+        for (int k = (*d.bptr)[v]; k < (*d.bptr)[v + 1]; ++k) add_entry(B, (*d.bidx)[k], (*d.bc)[k]);
+        B.ptr.push_back((int)B.idx.size());
+      }
+    }
+    B.upto[top] = (int)B.runs.size();
+    if (!multi) continue;
+    const auto rest = ranges(d, b.l0, top);
+    for (const auto& r : rest) {
+      add_run(B, r.first, r.second - r.first, kRowWork, delta[r.first]);
+      for (int v = r.first; v < r.second; ++v) {
+        for (int k = (*d.bptr)[v]; k < (*d.bptr)[v + 1]; ++k) {
+          if (s.lev[(*d.bidx)[k]] < b.l1) break;
+          add_entry(B, (*d.bidx)[k], (*d.bc)[k]);
+        }
+        B.ptr.push_back((int)B.idx.size());
+      }
+    }
+    // columns of M_B, targets descending (as the plain entries)
+    const int m = (int)b.vert.size();
+    for (int i = 0; i < m; ++i) s.where[b.vert[i]] = i;
+    tptr.assign(m + 1, 0);
+    for (int u : b.idx) tptr[s.where[u] + 1]++;
+    for (int i = 0; i < m; ++i) tptr[i + 1] += tptr[i];
+    tidx.resize(b.idx.size());
+    tval.resize(b.idx.size());
+    {
+      std::vector<int> pos(tptr.begin(), tptr.end() - 1);
+      for (int i = m - 1; i >= 0; --i)
+        for (int e = b.ptr[i]; e < b.ptr[i + 1]; ++e) {
+          const int c = s.where[b.idx[e]];
+          tidx[pos[c]] = b.vert[i];
+          tval[pos[c]] = b.val[e];
+          ++pos[c];
+        }
+    }
+    for (const auto& r : rest) {
+      add_run(B, r.first, r.second - r.first, kRowFinal, delta[r.first]);
+      for (int v = r.first; v < r.second; ++v) {
+        const int c = s.where[v];
+        for (int e = tptr[c]; e < tptr[c + 1]; ++e) {
+          const int u = tidx[e];
+          add_entry(B, s.lev[u] == top ? u : u + delta[u], tval[e]);
+        }
+        B.ptr.push_back((int)B.idx.size());
+      }
+    }
+    for (int l = b.l0; l < top; ++l) B.upto[l] = (int)B.runs.size();
+  }
+  return plan;
+}
+
+}  // namespace acg

@@ -19,6 +19,7 @@
 
 #include "../../include/acgpu.h"
 #include "acg_internal.h"
+#include "acg_plan.h"
 #include "acg_batch.cuh"
 #include "acg_dense.cuh"
 #include "acg_group.cuh"
@@ -81,6 +82,30 @@ struct SweepStep {
   size_t smem;  // thin runs: dynamic shared memory bytes
 };
 
+// A sweep plan (acg_plan.h) on the device: its rows' entries, and the task
+// tables of the one-vector sweeps (k_sweep) and of the batched ones (kb_sweep).
+struct DevSweep {
+  int nslots = 0;                    // values of a sweep vector: n + the blocks' work slots
+  int64_t nnz_f = 0, nnz_b = 0;
+  DevBuf<int> f_idx, b_idx;
+  DevBuf<double> f_c64, b_c64;
+  DevBuf<float> f_c32, b_c32;
+  int ntasks_f = 0, ntasks_b = 0, ntasks_fb = 0, ntasks_bb = 0;
+  DevBuf<SweepTask> tasks_f, tasks_b, tasks_fb, tasks_bb;
+  // per level l: the batched forward table's tasks up to the last one level l
+  // needs, and the backward table's (which walks levels downwards) likewise
+  std::vector<int> tfb_upto, tbb_from;
+  template <typename T>
+  const T* coef(bool fwd) const {
+    if constexpr (sizeof(T) == 8) return fwd ? f_c64.p : b_c64.p;
+    else return fwd ? f_c32.p : b_c32.p;
+  }
+  size_t bytes() const {
+    return 4 * (f_idx.n + b_idx.n) + 8 * (f_c64.n + b_c64.n) + 4 * (f_c32.n + b_c32.n) +
+           sizeof(SweepTask) * (tasks_f.n + tasks_b.n + tasks_fb.n + tasks_bb.n);
+  }
+};
+
 // Graph capture and device (de)allocation are serialised across threads: an
 // allocation or free on one thread while another thread captures a stream can
 // invalidate that capture.  Graph launches do not take this lock.
@@ -91,7 +116,6 @@ struct SolverImpl {
   cudaStream_t stream = nullptr;
   int n = 0;
   int64_t nnz_l = 0, nnz_f = 0;
-  int64_t nnz_fsweep = 0, nnz_bsweep = 0;  // entries the forward / backward sweeps walk
   int nlev = 0;
   int vl_spmv = 8;
   int thin_max_width = 2048;
@@ -105,15 +129,21 @@ struct SolverImpl {
   // narrow tail of the DAG run by one CTA (k_tail): levels [nlev - tail_nl, nlev)
   int tail_nl = 0, tail_v0 = 0, tail_nv = 0;
   int tail_tf0 = 0;                // forward: sync-free tasks [0, tail_tf0), the tail after
-  int tail_tb0 = 0;                // backward: the tail first, then sync-free tasks [tail_tb0, ntasks_b)
+  int tail_tb0 = 0;                // backward: the tail first, then the sync-free tasks from tail_tb0 on
   DevBuf<int2> tail_lvl_f, tail_lvl_b;
-  int ntasks_f = 0, ntasks_b = 0;
   int sweep_blocks[2] = {0, 0};    // co-resident grid of k_sweep per value type
   int poll_mode = 0;
   unsigned spin_limit = kSpinLimit;  // polls before a sweep wait gives up
   double min_inner_tol = 2e-5;       // mixed precision: floor of an inner solve's tolerance
   cudaEvent_t order_ev = nullptr;    // device entry points: after the legacy stream's work
-  DevBuf<SweepTask> tasks_f, tasks_b;
+  // sweep plans: [0] one vector, [1] batches (whose entries cost more, so their
+  // blocks are smaller); the per-level engine and the one-CTA tail need one
+  // level per block and have plan 0 alone.  So does a group: some of its
+  // members' PCG amplify a change of rounding to 1e-9 of x at tol 1e-8 (weights
+  // of 1/distance), and a group's results stay those of its levels in turn.
+  DevSweep sweep[2];
+  bool two_plans = false;
+  const DevSweep& batch_sweep() const { return sweep[two_plans ? 1 : 0]; }
 
   DevBuf<int> perm, lvl_off_d;
   DevBuf<int> iperm;               // external vertex -> internal (the batched gather and scatter)
@@ -167,11 +197,6 @@ struct SolverImpl {
   DevBuf<double> dt_M64, dt_part;        // dt_part: partial tiles (chunks x K x columns, as T)
   DevBuf<float> dt_M32;
   size_t dt_part_cols = 0;               // columns dt_part holds
-  int ntasks_bb = 0, ntasks_fb = 0;      // task tables of the batched sweeps
-  DevBuf<SweepTask> tasks_bb, tasks_fb;
-  // per level l: the forward table's tasks of levels <= l, and the backward
-  // table's tasks of levels >= l (the backward table walks levels downwards)
-  std::vector<int> tfb_upto, tbb_from;
   cudaGraphExec_t bexec[2][2][4] = {};  // [slot][precision][log2(kp/8)]
 
   // asynchronous batched solves (acg_solve_async): two slots, each with its
@@ -311,7 +336,6 @@ template <typename T, bool kForward>
 void enqueue_syncfree(cudaStream_t s, const SolverImpl& S, const T* aux, const T* sfwd, T* out, PcgState* st,
                       int t0, int t1, int vs) {
   if (t1 <= t0) return;
-  const TypedArrays<T> A = arrays_of<T>(S);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(S.sweep_blocks[plan_index<T>()]);
   cfg.blockDim = dim3(kSweepThreads);
@@ -321,19 +345,21 @@ void enqueue_syncfree(cudaStream_t s, const SolverImpl& S, const T* aux, const T
   at[0].val.cooperative = 1;
   cfg.attrs = at;
   cfg.numAttrs = 1;
-  const SweepTask* tasks = (kForward ? S.tasks_f.p : S.tasks_b.p) + t0;
-  ACG_CUDA(cudaLaunchKernelEx(&cfg, k_sweep<T, kForward>, t1 - t0, tasks, kForward ? A.fi : A.bi,
-                              kForward ? A.fc : A.bc, aux, sfwd, out, st, S.poll_mode, vs, S.spin_limit));
+  const DevSweep& P = S.sweep[0];
+  const SweepTask* tasks = (kForward ? P.tasks_f.p : P.tasks_b.p) + t0;
+  ACG_CUDA(cudaLaunchKernelEx(&cfg, k_sweep<T, kForward>, t1 - t0, tasks,
+                              (const int*)(kForward ? P.f_idx.p : P.b_idx.p), P.coef<T>(kForward), aux, sfwd, out, st,
+                              S.poll_mode, vs, S.spin_limit));
 }
 
 // The narrow tail of the DAG in one CTA.
 template <typename T, bool kForward>
 void enqueue_tail(cudaStream_t s, const SolverImpl& S, const T* aux, const T* sfwd, T* out, const PcgState* st) {
-  const TypedArrays<T> A = arrays_of<T>(S);
+  const DevSweep& P = S.sweep[0];
   const size_t smem = tail_smem_bytes<T>(S.tail_nv, S.tail_nl);
   k_tail<T, kForward><<<1, kTailThreads, smem, s>>>(
-      S.tail_nl, S.tail_v0, S.tail_nv, kForward ? S.tail_lvl_f.p : S.tail_lvl_b.p, kForward ? S.ntasks_f : S.ntasks_b,
-      kForward ? S.tasks_f.p : S.tasks_b.p, kForward ? A.fi : A.bi, kForward ? A.fc : A.bc, aux, sfwd, out, st);
+      S.tail_nl, S.tail_v0, S.tail_nv, kForward ? S.tail_lvl_f.p : S.tail_lvl_b.p, kForward ? P.ntasks_f : P.ntasks_b,
+      kForward ? P.tasks_f.p : P.tasks_b.p, kForward ? P.f_idx.p : P.b_idx.p, P.coef<T>(kForward), aux, sfwd, out, st);
 }
 
 // The dense tail step of a sweep on kp-column vectors (kp = 1, or 8 * CPL):
@@ -374,7 +400,7 @@ void enqueue_forward(cudaStream_t s, const SolverImpl& S, const T* r, T* sv, Pcg
       enqueue_syncfree<T, true>(s, S, r, (const T*)nullptr, sv, st, 0, S.tail_tf0, vs);
       enqueue_tail<T, true>(s, S, r, (const T*)nullptr, sv, st);
     } else {
-      enqueue_syncfree<T, true>(s, S, r, (const T*)nullptr, sv, st, 0, S.ntasks_f, vs);
+      enqueue_syncfree<T, true>(s, S, r, (const T*)nullptr, sv, st, 0, S.sweep[0].ntasks_f, vs);
     }
     if (S.dt_K && dense)
       enqueue_dense<T, 0>(s, S, true, sv, (T*)nullptr, part ? part : reinterpret_cast<T*>(S.dt_part.p), &st->done,
@@ -395,9 +421,9 @@ void enqueue_backward(cudaStream_t s, const SolverImpl& S, const T* sv, T* y, Pc
                           &st->done, vs);
     if (S.tail_nl > 0) {
       enqueue_tail<T, false>(s, S, g, sv, y, st);
-      enqueue_syncfree<T, false>(s, S, g, sv, y, st, S.tail_tb0, S.ntasks_b, vs);
+      enqueue_syncfree<T, false>(s, S, g, sv, y, st, S.tail_tb0, S.sweep[0].ntasks_b, vs);
     } else {
-      enqueue_syncfree<T, false>(s, S, g, sv, y, st, 0, S.ntasks_b, vs);
+      enqueue_syncfree<T, false>(s, S, g, sv, y, st, 0, S.sweep[0].ntasks_b, vs);
     }
     return;
   }
@@ -430,7 +456,8 @@ void enqueue_pcg_iteration(cudaStream_t s, const SolverImpl& S, T* r, T* sv, T* 
   const TypedArrays<T> A = arrays_of<T>(S);
   ACG_VL_SWITCH(S.vl_spmv, spmv_pq_vl, s, S, A, p, q, S.st, eps, ctl);
   const int vs = vstride<T>(S);
-  k_update<T><<<kVecBlocks, kVecThreads, 0, s>>>(S.n, x3, p, q, r, sv, y, S.st, S.partials.p, ctl, vs);
+  k_update<T><<<kVecBlocks, kVecThreads, 0, s>>>(S.n, x3, p, q, r, sv, y, S.st, S.partials.p, ctl, vs,
+                                                 S.sweep[0].nslots);
   enqueue_sweeps<T>(s, S, r, sv, y, S.st);
   k_ysum<T><<<kVecBlocks, kVecThreads, 0, s>>>(S.n, y, S.st, S.partials.p, ctl, vs);
   k_zdot<T><<<kVecBlocks, kVecThreads, 0, s>>>(S.n, y, r, p, S.st, S.partials.p, eps, 0, ctl, vs);
@@ -483,7 +510,7 @@ cudaGraphExec_t build_fp64_graph(SolverImpl& S) {
   begin_into(s, top, {});
   k_gather_in<<<kVecBlocks, kVecThreads, 0, s>>>(n, S.perm.p, S.b_ext.p, S.bm.p, S.st, S.partials.p);
   k_center<double><<<kVecBlocks, kVecThreads, 0, s>>>(n, S.bm.p, S.r64.p, S.x3_64.p, S.s64.p, S.y64.p, S.st,
-                                                      S.partials.p, ctl, S.vs64);
+                                                      S.partials.p, ctl, S.vs64, S.sweep[0].nslots);
   enqueue_sweeps<double>(s, S, S.r64.p, S.s64.p, S.y64.p, S.st);
   k_ysum<double><<<kVecBlocks, kVecThreads, 0, s>>>(n, S.y64.p, S.st, S.partials.p, ctl, S.vs64);
   k_zdot<double><<<kVecBlocks, kVecThreads, 0, s>>>(n, S.y64.p, S.r64.p, S.p64.p, S.st, S.partials.p, kEps64, 1, ctl,
@@ -527,7 +554,7 @@ cudaGraphExec_t build_mixed_graph(SolverImpl& S) {
   k_gather_in<<<kVecBlocks, kVecThreads, 0, s>>>(n, S.perm.p, S.b_ext.p, S.bm.p, S.st, S.partials.p);
   // r64 = bm, x64 (xf) = 0
   k_center<double><<<kVecBlocks, kVecThreads, 0, s>>>(n, S.bm.p, S.r64.p, S.xf.p, (double*)nullptr,
-                                                      (double*)nullptr, S.st, S.partials.p, octl, 1);
+                                                      (double*)nullptr, S.st, S.partials.p, octl, 1, n);
   std::vector<cudaGraphNode_t> leaves = capture_leaves(s);
   end_into(s);
 
@@ -539,7 +566,7 @@ cudaGraphExec_t build_mixed_graph(SolverImpl& S) {
 
   begin_into(s, obody, {});
   k_outer_prep<float><<<kVecBlocks, kVecThreads, 0, s>>>(n, S.r64.p, S.r32.p, S.x3_32.p, S.s32.p, S.y32.p, S.st,
-                                                         S.partials.p, ictl, S.vs32);
+                                                         S.partials.p, ictl, S.vs32, S.sweep[0].nslots);
   enqueue_sweeps<float>(s, S, S.r32.p, S.s32.p, S.y32.p, S.st);
   k_ysum<float><<<kVecBlocks, kVecThreads, 0, s>>>(n, S.y32.p, S.st, S.partials.p, ictl, S.vs32);
   k_zdot<float><<<kVecBlocks, kVecThreads, 0, s>>>(n, S.y32.p, S.r32.p, S.p32.p, S.st, S.partials.p, eps32, 2, ictl,
@@ -580,6 +607,16 @@ cudaGraphExec_t build_mixed_graph(SolverImpl& S) {
 // ============================================================================
 namespace acg {
 namespace {
+
+// What a level merge is worth (see SweepCost): entries worked through in the
+// time of one hand-over, and the entries of a row a warp has in flight.  The
+// batched sweeps move a row of kp values per entry.  FP64 one-vector forward /
+// backward sweep in us at 10000, 25000, 60000 entries: grid3(50) 87/95, 74/90,
+// 76/103 (one level per block 258/278); grid3(100) 420/476, 358/377, 361/408.
+// 64 FP32 columns at 5000, 10000, 20000: grid3(50) 203/229, 132/160, 150/181;
+// grid3(100) 812/851, 716/777, 778/842.
+constexpr SweepCost kVectorCost{25000.0, 128.0, 0.4};
+constexpr SweepCost kBatchCost{10000.0, 32.0, 0.5};
 
 template <typename T>
 std::vector<float> to_f32(const std::vector<T>& v) {
@@ -962,127 +999,134 @@ void build_solver(SolverImpl& S, int64_t n64, const int64_t* a_colptr, const int
       l = l1;
     }
   }
-  // ---- sync-free task tables: tasks in level order (backward: reverse level
-  // order); a vertex with more than sweep_heavy entries (default 16) is a
-  // task of its own on a whole warp, other vertices go four to a task within
-  // one level.
-  {
-    std::vector<int> outdeg(n, 0);
-    for (int v = 0; v < n; ++v) outdeg[v] = bptr[v + 1] - bptr[v];
-    auto emit_level = [](std::vector<SweepTask>& tasks, int vs, int ve, const std::vector<int>& deg,
-                         const std::vector<int>& ptr, int heavy_min) {
-      int run = -1, cnt = 0;
-      auto push = [&](int v, int c, int heavy) {
-        SweepTask t = {};
-        t.v = v;
-        t.cnt_heavy = (c << 1) | heavy;
-        for (int i = 0; i <= c; ++i) t.p[i] = ptr[v + i];
-        tasks.push_back(t);
-      };
-      auto flush = [&]() {
-        if (cnt) push(run, cnt, 0);
-        cnt = 0;
-      };
-      for (int v = vs; v < ve; ++v) {
-        if (deg[v] > heavy_min) {
-          flush();
-          push(v, 1, 1);
-          continue;
+  // ---- sweep plans and their task tables: a row with more than sweep_heavy
+  // entries (default 16; batched 8) is a task of its own on a whole warp, other
+  // rows go four to a task within one run
+  S.sweep_mode = (opts && opts->sweep_lanes == 1 && nseg == 1) ? 1 : 0;
+  const bool merge = S.sweep_mode == 0 && !(opts && opts->tail == 2) && nseg == 1;
+  S.two_plans = merge;
+  int phases = nlev;
+  for (int w = 0; w < (S.two_plans ? 2 : 1); ++w) {
+    DevSweep& P = S.sweep[w];
+    const SweepDag dag{n, nlev, &runs, &fptr, &fidx, &bptr, &bidx, &fc, &bc, S.dt_K ? S.dt_L0 : nlev};
+    const SweepPlan plan = build_sweep_plan(dag, w == 0 ? kVectorCost : kBatchCost, merge);
+    P.nslots = plan.nslots;
+    P.nnz_f = (int64_t)plan.fwd.idx.size();
+    P.nnz_b = (int64_t)plan.bwd.idx.size();
+    P.f_idx.upload(plan.fwd.idx, S.stream);
+    P.f_c64.upload(plan.fwd.coef, S.stream);
+    P.f_c32.upload(to_f32(plan.fwd.coef), S.stream);
+    P.b_idx.upload(plan.bwd.idx, S.stream);
+    P.b_c64.upload(plan.bwd.coef, S.stream);
+    P.b_c32.upload(to_f32(plan.bwd.coef), S.stream);
+    // tasks of a direction; after[i] = tasks up to the end of run i
+    auto emit = [](const SweepRows& R, int heavy_min, std::vector<int>& after) {
+      std::vector<SweepTask> tasks;
+      for (const SweepRun& r : R.runs) {
+        int first = 0, cnt = 0;
+        auto push = [&](int i, int c, int heavy) {
+          SweepTask t = {};
+          t.v = r.v0 + i;
+          t.info = (r.kind << 4) | (c << 1) | heavy;
+          t.delta = r.delta;
+          for (int q = 0; q <= c; ++q) t.p[q] = R.ptr[r.row + i + q];
+          tasks.push_back(t);
+        };
+        for (int i = 0; i < r.count; ++i) {
+          if (R.ptr[r.row + i + 1] - R.ptr[r.row + i] > heavy_min) {
+            if (cnt) push(first, cnt, 0);
+            cnt = 0;
+            push(i, 1, 1);
+            continue;
+          }
+          if (cnt == 0) first = i;
+          if (++cnt == 4) {
+            push(first, 4, 0);
+            cnt = 0;
+          }
         }
-        if (cnt == 0) run = v;
-        if (++cnt == 4) flush();
+        if (cnt) push(first, cnt, 0);
+        after.push_back((int)tasks.size());
       }
-      flush();
+      return tasks;
     };
-    std::vector<int> fdeg(n);
-    for (int v = 0; v < n; ++v) fdeg[v] = fptr[v + 1] - fptr[v];
+    std::vector<int> af, ab, afb, abb;
     const int sheavy = (opts && opts->sweep_heavy > 0) ? opts->sweep_heavy : 16;
-    std::vector<SweepTask> tf, tb;
-    std::vector<int2> lf(nlev), lb(nlev);  // {first task, count} per level
+    const int bheavy = (opts && opts->batch_bwd_heavy > 0) ? opts->batch_bwd_heavy : 8;
+    const int fheavy = (opts && opts->batch_fwd_heavy > 0) ? opts->batch_fwd_heavy : 8;
+    std::vector<SweepTask> tfb = emit(plan.fwd, fheavy, afb), tbb = emit(plan.bwd, bheavy, abb);
+    P.tfb_upto.assign(nlev, 0);
+    P.tbb_from.assign(nlev, 0);
     for (int l = 0; l < nlev; ++l) {
-      const int t0 = (int)tf.size();
-      for (const auto& r : runs[l]) emit_level(tf, r.first, r.second, fdeg, fptr, sheavy);
-      lf[l] = make_int2(t0, (int)tf.size() - t0);
+      if (plan.fwd.upto[l]) P.tfb_upto[l] = afb[plan.fwd.upto[l] - 1];
+      if (plan.bwd.upto[l]) P.tbb_from[l] = abb[plan.bwd.upto[l] - 1];
     }
-    const int blev = S.dt_K ? S.dt_L0 : nlev;  // levels the backward sweep walks
-    for (int l = nlev - 1; l >= blev; --l) lb[l] = make_int2((int)tb.size(), 0);
-    for (int l = blev - 1; l >= 0; --l) {
-      const int t0 = (int)tb.size();
-      for (const auto& r : runs[l]) emit_level(tb, r.first, r.second, outdeg, bptr, sheavy);
-      lb[l] = make_int2(t0, (int)tb.size() - t0);
+    // Testing only: blank one forward task record (it stores nothing), so
+    // the values of its vertices are never produced and the waits on them
+    // run out after spin_limit polls; the solve then reports
+    // ACG_ERR_TIMEOUT.  This is how the bounded waits are tested without
+    // faulting or hanging the GPU.
+    const int blank = opts ? opts->test_unproduced_task : 0;
+    auto unproduced = [&](std::vector<SweepTask>& t) {
+      if (blank <= 0) return;
+      if (blank > (int)t.size()) throw InputError("test_unproduced_task is beyond the forward task tables");
+      t[blank - 1].info = 0;
+    };
+    unproduced(tfb);
+    P.ntasks_fb = (int)tfb.size();
+    P.tasks_fb.upload(tfb, S.stream);
+    P.ntasks_bb = (int)tbb.size();
+    P.tasks_bb.upload(tbb, S.stream);
+    if (w == 0) {
+      std::vector<SweepTask> tf = emit(plan.fwd, sheavy, af), tb = emit(plan.bwd, sheavy, ab);
+      phases = merge ? 2 * plan.blocks : (S.dt_K ? S.dt_L0 : nlev);
+      // the tail: the longest run of final levels with at most 32 tasks in both
+      // tables whose values fit in shared memory (FP64 sizes, so both precisions fit)
+      if (!merge && nseg == 1 && opts->tail == 2) {
+        std::vector<int2> lf(nlev), lb(nlev);  // {first task, count} per level
+        for (int l = 0; l < nlev; ++l) {
+          const int f1 = af[plan.fwd.upto[l] - 1], f0 = l ? af[plan.fwd.upto[l - 1] - 1] : 0;
+          const int b1 = ab[plan.bwd.upto[l] - 1], b0 = l + 1 < nlev ? ab[plan.bwd.upto[l + 1] - 1] : 0;
+          lf[l] = make_int2(f0, f1 - f0);
+          lb[l] = make_int2(b0, b1 - b0);
+        }
+        int optin = 0;
+        ACG_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, S.device));
+        const size_t cap = optin > 8192 ? (size_t)optin - 4096 : 0;
+        int lt = nlev, nv = 0;
+        while (lt > 0) {
+          const int l = lt - 1;
+          const int wd = S.lvl_off[l + 1] - S.lvl_off[l];
+          if (lf[l].y > kTailWarps || lb[l].y > kTailWarps) break;
+          if (tail_smem_bytes<double>(nv + wd, nlev - l) > cap) break;
+          nv += wd;
+          lt = l;
+        }
+        if (nlev - lt >= 8) {
+          S.tail_nl = nlev - lt;
+          S.tail_v0 = S.lvl_off[lt];
+          S.tail_nv = n - S.tail_v0;
+          S.tail_tf0 = lf[lt].x;
+          S.tail_tb0 = lb[lt].x + lb[lt].y;
+          std::vector<int2> tlf(lf.begin() + lt, lf.end()), tlb(lb.begin() + lt, lb.end());
+          S.tail_lvl_f.upload(tlf, S.stream);
+          S.tail_lvl_b.upload(tlb, S.stream);
+          const int tb_bytes = (int)tail_smem_bytes<double>(S.tail_nv, S.tail_nl);
+          ACG_CUDA(cudaFuncSetAttribute(k_tail<double, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, tb_bytes));
+          ACG_CUDA(cudaFuncSetAttribute(k_tail<double, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, tb_bytes));
+          ACG_CUDA(cudaFuncSetAttribute(k_tail<float, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, tb_bytes));
+          ACG_CUDA(cudaFuncSetAttribute(k_tail<float, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, tb_bytes));
+        }
+      }
+      unproduced(tf);
+      P.ntasks_f = (int)tf.size();
+      P.tasks_f.upload(tf, S.stream);
+      P.ntasks_b = (int)tb.size();
+      P.tasks_b.upload(tb, S.stream);
     }
-    // the tail: the longest run of final levels with at most 32 tasks in both
-    // tables whose values fit in shared memory (FP64 sizes, so both precisions fit)
-    {
-      int optin = 0;
-      ACG_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, S.device));
-      const size_t cap = optin > 8192 ? (size_t)optin - 4096 : 0;
-      int lt = nlev, nv = 0;
-      while (lt > 0) {
-        const int l = lt - 1;
-        const int w = S.lvl_off[l + 1] - S.lvl_off[l];
-        if (lf[l].y > kTailWarps || lb[l].y > kTailWarps) break;
-        if (tail_smem_bytes<double>(nv + w, nlev - l) > cap) break;
-        nv += w;
-        lt = l;
-      }
-      if (nlev - lt >= 8 && nseg == 1 && opts && opts->tail == 2) {
-        S.tail_nl = nlev - lt;
-        S.tail_v0 = S.lvl_off[lt];
-        S.tail_nv = n - S.tail_v0;
-        S.tail_tf0 = lf[lt].x;
-        S.tail_tb0 = lb[lt].x + lb[lt].y;
-        std::vector<int2> tlf(lf.begin() + lt, lf.end()), tlb(lb.begin() + lt, lb.end());
-        S.tail_lvl_f.upload(tlf, S.stream);
-        S.tail_lvl_b.upload(tlb, S.stream);
-        const int tb_bytes = (int)tail_smem_bytes<double>(S.tail_nv, S.tail_nl);
-        ACG_CUDA(cudaFuncSetAttribute(k_tail<double, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, tb_bytes));
-        ACG_CUDA(cudaFuncSetAttribute(k_tail<double, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, tb_bytes));
-        ACG_CUDA(cudaFuncSetAttribute(k_tail<float, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, tb_bytes));
-        ACG_CUDA(cudaFuncSetAttribute(k_tail<float, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, tb_bytes));
-      } else {
-        S.tail_nl = 0;
-      }
-    }
-    // task tables of the batched sweeps: a vertex with more than bheavy
-    // (backward) or fheavy (forward) entries gets a whole warp
-    {
-      const int bheavy = (opts && opts->batch_bwd_heavy > 0) ? opts->batch_bwd_heavy : 8;
-      const int fheavy = (opts && opts->batch_fwd_heavy > 0) ? opts->batch_fwd_heavy : 8;
-      std::vector<SweepTask> tbb, tfb;
-      S.tbb_from.assign(nlev, 0);
-      S.tfb_upto.assign(nlev, 0);
-      for (int l = blev - 1; l >= 0; --l) {
-        for (const auto& r : runs[l]) emit_level(tbb, r.first, r.second, outdeg, bptr, bheavy);
-        S.tbb_from[l] = (int)tbb.size();
-      }
-      for (int l = 0; l < nlev; ++l) {
-        for (const auto& r : runs[l]) emit_level(tfb, r.first, r.second, fdeg, fptr, fheavy);
-        S.tfb_upto[l] = (int)tfb.size();
-      }
-      // Testing only: blank one forward task record (it stores nothing), so
-      // the values of its vertices are never produced and the waits on them
-      // run out after spin_limit polls; the solve then reports
-      // ACG_ERR_TIMEOUT.  This is how the bounded waits are tested without
-      // faulting or hanging the GPU.
-      const int blank = opts ? opts->test_unproduced_task : 0;
-      if (blank > 0) {
-        if (blank > (int)tf.size() || blank > (int)tfb.size())
-          throw InputError("test_unproduced_task is beyond the forward task tables");
-        tf[blank - 1].cnt_heavy = 0;
-        tfb[blank - 1].cnt_heavy = 0;
-      }
-      S.ntasks_bb = (int)tbb.size();
-      S.tasks_bb.upload(tbb, S.stream);
-      S.ntasks_fb = (int)tfb.size();
-      S.tasks_fb.upload(tfb, S.stream);
-    }
-    S.ntasks_f = (int)tf.size();
-    S.ntasks_b = (int)tb.size();
-    S.nnz_fsweep = fptr[n];
-    S.nnz_bsweep = bptr[S.dt_K ? S.dt_v0 : n];
-    S.tasks_f.upload(tf, S.stream);
-    S.tasks_b.upload(tb, S.stream);
+    ACG_CUDA(cudaStreamSynchronize(S.stream));  // the uploads read this iteration's arrays
+  }
+  {
     int sms = 0;
     ACG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, S.device));
     int occ[4] = {0, 0, 0, 0};
@@ -1093,20 +1137,18 @@ void build_solver(SolverImpl& S, int64_t n64, const int64_t* a_colptr, const int
     // Resident blocks (8 warps each) per SM: a deep, narrow DAG gains nothing
     // from more warps (they add polling traffic without shortening the chains),
     // a wide one is throughput-bound in its wide levels and gains from them.
-    // Automatic choice by the tasks per swept level (measured: the 2M
-    // path+matchings graph, ~150 per level, is fastest with 1; the 1M 3D grid,
-    // ~750, with 2; 256 graphs in one launch, thousands, with 4).
+    // Automatic choice by the tasks per hand-over (measured: the 150k-vertex
+    // path+matchings graph, ~1,000, is fastest with 2: 102 us forward, 117 with
+    // 3; the 1M 3D grid, ~4,000, with 3 or more: 395 us against 409 with 2).
     int cap = 1;
     if (opts && opts->sweep_blocks_per_sm > 0) {
       cap = opts->sweep_blocks_per_sm;
     } else {
-      const int swept = std::max(1, (S.dt_K ? S.dt_L0 : nlev));
-      const double per_level = (double)std::max(S.ntasks_f, S.ntasks_b) / swept;
+      const double per_level = (double)std::max(S.sweep[0].ntasks_f, S.sweep[0].ntasks_b) / std::max(1, phases);
       cap = per_level < 300.0 ? 1 : (per_level < 2000.0 ? 2 : 4);
     }
     S.sweep_blocks[0] = sms * std::max(1, std::min(cap, std::min(occ[0], occ[1])));
     S.sweep_blocks[1] = sms * std::max(1, std::min(cap, std::min(occ[2], occ[3])));
-    S.sweep_mode = (opts && opts->sweep_lanes == 1 && nseg == 1) ? 1 : 0;
     if (opts && opts->poll_mode > 0) S.poll_mode = opts->poll_mode - 1;
     if (opts && opts->spin_limit > 0) S.spin_limit = (unsigned)opts->spin_limit;
     if (opts && opts->min_inner_tol > 0) S.min_inner_tol = std::min(0.25, opts->min_inner_tol);
@@ -1129,14 +1171,16 @@ void build_solver(SolverImpl& S, int64_t n64, const int64_t* a_colptr, const int
   S.l_idx.upload(lidx, s);
   S.l_v64.upload(lv, s);
   S.l_v32.upload(to_f32(lv), s);
-  S.f_ptr.upload(fptr, s);
-  S.f_idx.upload(fidx, s);
-  S.f_c64.upload(fc, s);
-  S.f_c32.upload(to_f32(fc), s);
-  S.b_ptr.upload(bptr, s);
-  S.b_idx.upload(bidx, s);
-  S.b_c64.upload(bc, s);
-  S.b_c32.upload(to_f32(bc), s);
+  if (S.sweep_mode == 1) {  // the per-level engine finds a vertex's entries by its id
+    S.f_ptr.upload(fptr, s);
+    S.f_idx.upload(fidx, s);
+    S.f_c64.upload(fc, s);
+    S.f_c32.upload(to_f32(fc), s);
+    S.b_ptr.upload(bptr, s);
+    S.b_idx.upload(bidx, s);
+    S.b_c64.upload(bc, s);
+    S.b_c32.upload(to_f32(bc), s);
+  }
   S.g64.upload(gi, s);
   S.g32.upload(to_f32(gi), s);
   if (S.dt_K) {
@@ -1154,10 +1198,10 @@ void build_solver(SolverImpl& S, int64_t n64, const int64_t* a_colptr, const int
   S.vs64 = pad ? 32 / (int)sizeof(double) : 1;
   S.vs32 = pad ? 32 / (int)sizeof(float) : 1;
   for (DevBuf<double>* b : {&S.b_ext, &S.x_ext, &S.bm, &S.r64, &S.p64, &S.q64, &S.xf}) b->alloc(n);
-  for (DevBuf<double>* b : {&S.s64, &S.y64}) b->alloc((size_t)n * S.vs64);
+  for (DevBuf<double>* b : {&S.s64, &S.y64}) b->alloc((size_t)S.sweep[0].nslots * S.vs64);
   S.x3_64.alloc((size_t)3 * n);
   for (DevBuf<float>* b : {&S.r32, &S.p32, &S.q32}) b->alloc(n);
-  for (DevBuf<float>* b : {&S.s32, &S.y32}) b->alloc((size_t)n * S.vs32);
+  for (DevBuf<float>* b : {&S.s32, &S.y32}) b->alloc((size_t)S.sweep[0].nslots * S.vs32);
   S.x3_32.alloc((size_t)3 * n);
   S.partials.alloc((size_t)4 * kMaxPartialBlocks);
   ACG_CUDA(cudaMalloc(&S.st, sizeof(PcgState)));
@@ -1235,7 +1279,7 @@ void ldlsolve_impl(SolverImpl& S, T* rbuf, T* sbuf, T* ybuf) {
   k_gather_in<<<kVecBlocks, kVecThreads, 0, s>>>(n, S.perm.p, S.b_ext.p, S.bm.p, S.st, S.partials.p);
   k_cast_from64<T><<<kVecBlocks, kVecThreads, 0, s>>>(n, S.bm.p, rbuf);
   const int vs = vstride<T>(S);
-  k_fill_pending<T><<<kVecBlocks, kVecThreads, 0, s>>>(n, sbuf, ybuf, vs);
+  k_fill_pending<T><<<kVecBlocks, kVecThreads, 0, s>>>((size_t)S.sweep[0].nslots, sbuf, ybuf, vs);
   enqueue_sweeps<T>(s, S, rbuf, sbuf, ybuf, S.st);
   k_ysum<T><<<kVecBlocks, kVecThreads, 0, s>>>(n, ybuf, S.st, S.partials.p, none, vs);
   k_minus_mean<T><<<kVecBlocks, kVecThreads, 0, s>>>(n, ybuf, S.st, S.xf.p, vs);
@@ -1260,7 +1304,10 @@ constexpr size_t kNoAllocPartials = (size_t)4 * kMaxPartialBlocks * sizeof(doubl
 // a dense tail has at most min(kDenseMaxK, n / 4) vertices
 constexpr int kNoAllocDenseK = kDenseMaxK < kNoAllocMaxN / 4 ? kDenseMaxK : kNoAllocMaxN / 4;
 constexpr size_t kNoAllocDense = (size_t)dense_chunks(kNoAllocDenseK) * kNoAllocDenseK * sizeof(double);
-constexpr size_t kNoAllocState = 4 * kNoAllocVec + kNoAllocPartials + kNoAllocDense;
+// r as FP64 and in the sweeps' type, and the two sweep vectors with a work
+// slot per vertex at most
+constexpr size_t kNoAllocVectors = 6 * kNoAllocVec;
+constexpr size_t kNoAllocState = kNoAllocVectors + kNoAllocPartials + kNoAllocDense;
 constexpr size_t kNoAllocBytes = kNoAllocState + ((sizeof(PcgState) + 255) / 256) * 256;
 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kNoAllocBytes];
@@ -1288,17 +1335,17 @@ void ldlsolve_noalloc_impl(const SolverImpl& S, cudaStream_t s, const double* r_
   double* r64 = reinterpret_cast<double*>(base);
   T* rT = reinterpret_cast<T*>(base + kNoAllocVec);
   T* sv = reinterpret_cast<T*>(base + 2 * kNoAllocVec);
-  T* yv = reinterpret_cast<T*>(base + 3 * kNoAllocVec);
-  double* partials = reinterpret_cast<double*>(base + 4 * kNoAllocVec);
-  T* dense_part = reinterpret_cast<T*>(base + 4 * kNoAllocVec + kNoAllocPartials);
+  T* yv = reinterpret_cast<T*>(base + 4 * kNoAllocVec);
+  double* partials = reinterpret_cast<double*>(base + kNoAllocVectors);
+  T* dense_part = reinterpret_cast<T*>(base + kNoAllocVectors + kNoAllocPartials);
   PcgState* st = reinterpret_cast<PcgState*>(base + kNoAllocState);
   LoopCtl none{0, 0};
   // the state (done flag, sweep error flag, reduction tickets) must start at zero
   ACG_CUDA(cudaMemsetAsync(st, 0, sizeof(PcgState), s));
   k_gather_in<<<kVecBlocks, kVecThreads, 0, s>>>(n, S.perm.p, r_ext, r64, st, partials);
   k_cast_from64<T><<<kVecBlocks, kVecThreads, 0, s>>>(n, r64, rT);
-  // compact vectors (one value per vertex): the fixed array holds n values each
-  k_fill_pending<T><<<kVecBlocks, kVecThreads, 0, s>>>(n, sv, yv, 1);
+  // compact vectors (one value per slot): the fixed array holds 2n values each
+  k_fill_pending<T><<<kVecBlocks, kVecThreads, 0, s>>>((size_t)S.sweep[0].nslots, sv, yv, 1);
   enqueue_sweeps<T>(s, S, rT, sv, yv, st, dense_part, 1);
   k_ysum<T><<<kVecBlocks, kVecThreads, 0, s>>>(n, yv, st, partials, none, 1);
   k_minus_mean<T><<<kVecBlocks, kVecThreads, 0, s>>>(n, yv, st, r64, 1);
@@ -1359,8 +1406,9 @@ void time_kernels_t(SolverImpl& S, int reps, acg_kernel_times* out, T* r, T* sv,
     return (double)ms / reps;
   };
   const int vs = vstride<T>(S);
-  auto fill_s = [&]() { k_fill_pending<T><<<kVecBlocks, kVecThreads, 0, s>>>(S.n, sv, (T*)nullptr, vs); };
-  auto fill_y = [&]() { k_fill_pending<T><<<kVecBlocks, kVecThreads, 0, s>>>(S.n, y, (T*)nullptr, vs); };
+  const size_t ns = (size_t)S.sweep[0].nslots;
+  auto fill_s = [&]() { k_fill_pending<T><<<kVecBlocks, kVecThreads, 0, s>>>(ns, sv, (T*)nullptr, vs); };
+  auto fill_y = [&]() { k_fill_pending<T><<<kVecBlocks, kVecThreads, 0, s>>>(ns, y, (T*)nullptr, vs); };
   const double t_fill = time_graph(fill_s);
   out->spmv_ms = time_graph([&]() { ACG_VL_SWITCH(S.vl_spmv, spmv_plain_vl, s, S, A, p, S.xf.p); });
   out->forward_ms = time_graph([&]() {
@@ -1374,7 +1422,7 @@ void time_kernels_t(SolverImpl& S, int reps, acg_kernel_times* out, T* r, T* sv,
   out->iteration_ms = time_graph([&]() {
     // the kernels of one PCG iteration without the stop logic taking effect
     ACG_VL_SWITCH(S.vl_spmv, spmv_plain_vl, s, S, A, p, S.xf.p);
-    k_fill_pending<T><<<kVecBlocks, kVecThreads, 0, s>>>(S.n, sv, y, vs);
+    k_fill_pending<T><<<kVecBlocks, kVecThreads, 0, s>>>(ns, sv, y, vs);
     enqueue_sweeps<T>(s, S, r, sv, y, S.st);
     k_ysum<T><<<kVecBlocks, kVecThreads, 0, s>>>(S.n, y, S.st, S.partials.p, none, vs);
     k_ysum<T><<<kVecBlocks, kVecThreads, 0, s>>>(S.n, y, S.st, S.partials.p, none, vs);
@@ -1387,7 +1435,8 @@ void time_kernels_t(SolverImpl& S, int reps, acg_kernel_times* out, T* r, T* sv,
   // the backward sweep alone reads the tail values the dense product wrote in
   // the backward_ms runs above, so only the head is marked pending
   auto fill_yh = [&]() {
-    k_fill_pending<T><<<kVecBlocks, kVecThreads, 0, s>>>(S.dt_K ? S.dt_v0 : S.n, y, (T*)nullptr, vs);
+    k_fill_pending<T><<<kVecBlocks, kVecThreads, 0, s>>>((size_t)(S.dt_K ? S.dt_v0 : S.n), y, (T*)nullptr, vs);
+    k_fill_pending<T><<<kVecBlocks, kVecThreads, 0, s>>>(ns - S.n, y + (size_t)S.n * vs, (T*)nullptr, vs);
   };
   const double t_fill_h = time_graph(fill_yh);
   out->backward_sweep_ms = time_graph([&]() {
@@ -1403,8 +1452,8 @@ void time_kernels_t(SolverImpl& S, int reps, acg_kernel_times* out, T* r, T* sv,
   out->spmv_bytes = 4.0 * (nv + 1) + (double)S.nnz_l * (4.0 + vb) + nv * vb + nv * 8.0;
   // sweeps: (index, coefficient) per entry, one 32-byte task record per task,
   // aux (r or g) in, own forward value (backward), each input value once, output
-  out->forward_sweep_bytes = (double)S.nnz_fsweep * (4.0 + vb) + 32.0 * S.ntasks_f + nv * vb * 3.0;
-  out->backward_sweep_bytes = (double)S.nnz_bsweep * (4.0 + vb) + 32.0 * S.ntasks_b + nv * vb * 4.0;
+  out->forward_sweep_bytes = (double)S.sweep[0].nnz_f * (4.0 + vb) + 32.0 * S.sweep[0].ntasks_f + (nv + 2.0 * ns) * vb;
+  out->backward_sweep_bytes = (double)S.sweep[0].nnz_b * (4.0 + vb) + 32.0 * S.sweep[0].ntasks_b + 2.0 * (nv + ns) * vb;
   // dense tail: the K(K+1)/2 entries of M once per product
   const double kk = (double)S.dt_K;
   out->dense_bytes = 2.0 * kk * (kk + 1.0) / 2.0 * vb;
@@ -1456,7 +1505,7 @@ void with_cpl(int kp, F&& f) {
 
 template <typename T, int CPL, bool kForward>
 void enqueue_bsweep(cudaStream_t s, const SolverImpl& S, const T* aux, T* sfwd, T* out, T* mark, int ntasks = -1) {
-  const TypedArrays<T> A = arrays_of<T>(S);
+  const DevSweep& P = S.batch_sweep();
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(S.bsweep_blocks[plan_index<T>()][kp_index(CPL * kBatchLanes)]);
   cfg.blockDim = dim3(kSweepThreads);
@@ -1466,10 +1515,11 @@ void enqueue_bsweep(cudaStream_t s, const SolverImpl& S, const T* aux, T* sfwd, 
   at[0].val.cooperative = 1;
   cfg.attrs = at;
   cfg.numAttrs = 1;
-  if (ntasks < 0) ntasks = kForward ? S.ntasks_fb : S.ntasks_bb;
+  if (ntasks < 0) ntasks = kForward ? P.ntasks_fb : P.ntasks_bb;
   ACG_CUDA(cudaLaunchKernelEx(&cfg, kb_sweep<T, CPL, kForward>, ntasks,
-                              (const SweepTask*)(kForward ? S.tasks_fb.p : S.tasks_bb.p), kForward ? A.fi : A.bi,
-                              kForward ? A.fc : A.bc, aux, (const T*)sfwd, out, mark, S.bsh, S.spin_limit));
+                              (const SweepTask*)(kForward ? P.tasks_fb.p : P.tasks_bb.p),
+                              (const int*)(kForward ? P.f_idx.p : P.b_idx.p), P.coef<T>(kForward), aux,
+                              (const T*)sfwd, out, mark, S.bsh, S.spin_limit));
 }
 
 // Batched forward (s from r) and backward (y from s) sweeps, dense tail included.
@@ -1524,7 +1574,7 @@ cudaGraphExec_t build_batch_fp64_graph(SolverImpl& S, int slot) {
   kb_gather_in<<<kVecBlocks, kVecThreads, 0, s>>>(n, kp, S.iperm.p, S.bb_ext[slot].p, (long long)n, S.bbm.p, S.bst, S.bsh,
                                                   S.bpartials.p);
   kb_center<double><<<kVecBlocks, kVecThreads, 0, s>>>(n, kp, S.bbm.p, S.br64.p, x3, S.bs64.p, S.by64.p, S.bst,
-                                                       S.bsh, S.bpartials.p, ctl);
+                                                       S.bsh, S.bpartials.p, ctl, S.batch_sweep().nslots);
   enqueue_bsweeps<double, CPL>(s, S, S.br64.p, S.bs64.p, S.by64.p);
   kb_ysum<double><<<kBVecBlocks, kBVecThreads, 0, s>>>(n, kp, S.by64.p, S.bst, S.bsh, S.bpartials.p, ctl);
   kb_zdot<double><<<kBVecBlocks, kBVecThreads, 0, s>>>(n, kp, S.by64.p, S.br64.p, S.bp64.p, S.bst, S.bsh,
@@ -1564,7 +1614,7 @@ cudaGraphExec_t build_batch_mixed_graph(SolverImpl& S, int slot) {
   kb_gather_in<<<kVecBlocks, kVecThreads, 0, s>>>(n, kp, S.iperm.p, S.bb_ext[slot].p, (long long)n, S.bbm.p, S.bst, S.bsh,
                                                   S.bpartials.p);
   kb_center<double><<<kVecBlocks, kVecThreads, 0, s>>>(n, kp, S.bbm.p, S.br64.p, S.bxf.p, (double*)nullptr,
-                                                       (double*)nullptr, S.bst, S.bsh, S.bpartials.p, octl);
+                                                       (double*)nullptr, S.bst, S.bsh, S.bpartials.p, octl, n);
   std::vector<cudaGraphNode_t> leaves = capture_leaves(s);
   end_into(s);
   cudaGraph_t obody;
@@ -1574,7 +1624,8 @@ cudaGraphExec_t build_batch_mixed_graph(SolverImpl& S, int slot) {
   LoopCtl ictl{hi, 1};
   begin_into(s, obody, {});
   kb_outer_prep<float><<<kVecBlocks, kVecThreads, 0, s>>>(n, kp, S.br64.p, S.br32.p, S.bx3_32.p, S.bs32.p, S.by32.p,
-                                                          S.bst, S.bsh, S.bpartials.p, ictl);
+                                                          S.bst, S.bsh, S.bpartials.p, ictl,
+                                                          S.batch_sweep().nslots);
   enqueue_bsweeps<float, CPL>(s, S, S.br32.p, S.bs32.p, S.by32.p);
   kb_ysum<float><<<kBVecBlocks, kBVecThreads, 0, s>>>(n, kp, S.by32.p, S.bst, S.bsh, S.bpartials.p, ictl);
   kb_zdot<float><<<kBVecBlocks, kBVecThreads, 0, s>>>(n, kp, S.by32.p, S.br32.p, S.bp32.p, S.bst, S.bsh, S.bpartials.p,
@@ -1691,10 +1742,13 @@ void ensure_batch(SolverImpl& S, int kp) {
     S.bb_ext[1].alloc(N);
     S.bx_ext[1].alloc(N);
   }
-  for (DevBuf<double>* b : {&S.bb_ext[0], &S.bx_ext[0], &S.bbm, &S.br64, &S.bxf, &S.bs64, &S.by64, &S.bp64, &S.bq64})
+  for (DevBuf<double>* b : {&S.bb_ext[0], &S.bx_ext[0], &S.bbm, &S.br64, &S.bxf, &S.bp64, &S.bq64})
     b->alloc(N);
+  const size_t Ns = (size_t)S.batch_sweep().nslots * kp;
+  for (DevBuf<double>* b : {&S.bs64, &S.by64}) b->alloc(Ns);
+  for (DevBuf<float>* b : {&S.bs32, &S.by32}) b->alloc(Ns);
   S.bx3_64.alloc(3 * N);
-  for (DevBuf<float>* b : {&S.br32, &S.bs32, &S.by32, &S.bp32, &S.bq32}) b->alloc(N);
+  for (DevBuf<float>* b : {&S.br32, &S.bp32, &S.bq32}) b->alloc(N);
   S.bx3_32.alloc(3 * N);
   S.batch_kp = kp;
 }
@@ -1792,7 +1846,7 @@ int solve_batch(SolverImpl& S, const double* B, int64_t ldb, double* X, int64_t 
 
 GroupArgs group_args(const SolverImpl& S) {
   return GroupArgs{S.chunks.p, S.seg_first.p, S.seg_nchunk.p, S.seg_cnt.p, S.gpartials.p, S.gstates, S.gflags,
-                   S.gsh, S.nseg};
+                   S.gsh, S.nseg, S.n, S.sweep[0].nslots};
 }
 
 cudaGraphExec_t build_group_graph(SolverImpl& S) {
@@ -2047,8 +2101,10 @@ void time_batch_t(SolverImpl& S, int reps, acg_kernel_times* out, T* r, T* sv, T
   const TypedArrays<T> A = arrays_of<T>(S);
   const size_t N = (size_t)S.n * kp;
   auto time_graph = [&](auto&& body) -> double { return graph_ms(s, reps, body); };
-  auto fill_s = [&]() { k_fill_pending<T><<<kVecBlocks, kVecThreads, 0, s>>>((int)N, sv, (T*)nullptr); };
-  auto fill_y = [&]() { k_fill_pending<T><<<kVecBlocks, kVecThreads, 0, s>>>((int)N, y, (T*)nullptr); };
+  const DevSweep& P = S.batch_sweep();
+  const size_t Ns = (size_t)P.nslots * kp;
+  auto fill_s = [&]() { k_fill_pending<T><<<kVecBlocks, kVecThreads, 0, s>>>(Ns, sv, (T*)nullptr); };
+  auto fill_y = [&]() { k_fill_pending<T><<<kVecBlocks, kVecThreads, 0, s>>>(Ns, y, (T*)nullptr); };
   const double t_fill = time_graph(fill_s);
   out->spmv_ms = time_graph([&]() {
     kb_spmv<T, CPL, true><<<S.bspmv_blocks[plan_index<T>()][kp_index(kp)], kVecThreads, 0, s>>>(
@@ -2080,7 +2136,8 @@ void time_batch_t(SolverImpl& S, int reps, acg_kernel_times* out, T* r, T* sv, T
   // the backward sweep alone reads the tail rows the dense product wrote in
   // the backward_ms runs above, so only the head is marked pending
   auto fill_yh = [&]() {
-    k_fill_pending<T><<<kVecBlocks, kVecThreads, 0, s>>>((int)((size_t)(S.dt_K ? S.dt_v0 : S.n) * kp), y, (T*)nullptr);
+    k_fill_pending<T><<<kVecBlocks, kVecThreads, 0, s>>>((size_t)(S.dt_K ? S.dt_v0 : S.n) * kp, y, (T*)nullptr);
+    k_fill_pending<T><<<kVecBlocks, kVecThreads, 0, s>>>(Ns - N, y + N, (T*)nullptr);
   };
   const double t_fill_h = time_graph(fill_yh);
   out->backward_sweep_ms = time_graph([&]() {
@@ -2153,8 +2210,8 @@ void time_batch_t(SolverImpl& S, int reps, acg_kernel_times* out, T* r, T* sv, T
   out->forward_launches = 1 + dense_launches;
   const double vb = sizeof(T), nv = S.n;
   out->spmv_bytes = 4.0 * (nv + 1) + (double)S.nnz_l * (4.0 + vb) + 2.0 * nv * kp * vb;
-  out->forward_sweep_bytes = (double)S.nnz_fsweep * (4.0 + vb) + 32.0 * S.ntasks_fb + 3.0 * nv * kp * vb;
-  out->backward_sweep_bytes = (double)S.nnz_bsweep * (4.0 + vb) + 32.0 * S.ntasks_bb + nv * vb + 3.0 * nv * kp * vb;
+  out->forward_sweep_bytes = (double)P.nnz_f * (4.0 + vb) + 32.0 * P.ntasks_fb + (nv + 2.0 * P.nslots) * kp * vb;
+  out->backward_sweep_bytes = (double)P.nnz_b * (4.0 + vb) + 32.0 * P.ntasks_bb + nv * vb + (nv + 2.0 * P.nslots) * kp * vb;
   const double kk = (double)S.dt_K;
   out->dense_bytes = 2.0 * kk * (kk + 1.0) / 2.0 * vb;
   out->forward_bytes = out->forward_sweep_bytes + out->dense_bytes / 2.0;
@@ -2179,9 +2236,12 @@ void time_levels_t(SolverImpl& S, int reps, int npts, const int* levels, double*
   const size_t N = (size_t)S.n * kp;
   ACG_CUDA(cudaMemsetAsync(S.bsh, 0, sizeof(BatchShared), s));
   ACG_CUDA(cudaMemsetAsync(r, 0, sizeof(T) * N, s));
-  auto fill_s = [&]() { k_fill_pending<T><<<kVecBlocks, kVecThreads, 0, s>>>((int)N, sv, (T*)nullptr); };
+  const DevSweep& P = S.batch_sweep();
+  const size_t Ns = (size_t)P.nslots * kp;
+  auto fill_s = [&]() { k_fill_pending<T><<<kVecBlocks, kVecThreads, 0, s>>>(Ns, sv, (T*)nullptr); };
   auto fill_yh = [&]() {
-    k_fill_pending<T><<<kVecBlocks, kVecThreads, 0, s>>>((int)((size_t)(S.dt_K ? S.dt_v0 : S.n) * kp), y, (T*)nullptr);
+    k_fill_pending<T><<<kVecBlocks, kVecThreads, 0, s>>>((size_t)(S.dt_K ? S.dt_v0 : S.n) * kp, y, (T*)nullptr);
+    k_fill_pending<T><<<kVecBlocks, kVecThreads, 0, s>>>(Ns - N, y + N, (T*)nullptr);
   };
   auto restore_s = [&]() { ACG_CUDA(cudaMemcpyAsync(sv, saved, sizeof(T) * N, cudaMemcpyDeviceToDevice, s)); };
   // one whole forward pass (sweep and dense product) gives the backward runs
@@ -2197,11 +2257,11 @@ void time_levels_t(SolverImpl& S, int reps, int npts, const int* levels, double*
     restore_s();
     fill_yh();
   });
-  const int nl = (int)S.tfb_upto.size();
-  if (nl == 0 || (int)S.tbb_from.size() != nl) throw InputError("the solver has no batched sweep tables");
+  const int nl = (int)P.tfb_upto.size();
+  if (nl == 0 || (int)P.tbb_from.size() != nl) throw InputError("the solver has no batched sweep tables");
   for (int i = 0; i < npts; ++i) {
     const int L = std::min(std::max(levels[i], 0), nl - 1);
-    const int tf = S.tfb_upto[L], tb = S.tbb_from[L];
+    const int tf = P.tfb_upto[L], tb = P.tbb_from[L];
     fwd_tasks[i] = tf;
     bwd_tasks[i] = tb;
     // differences of two timings: a prefix shorter than the timing noise may
@@ -2683,7 +2743,7 @@ int acg_solver_stats(const acg_solver* h, acg_stats* out) {
   add(S.l_v64); add(S.f_c64); add(S.b_c64); add(S.g64); add(S.l_v32); add(S.f_c32); add(S.b_c32); add(S.g32);
   add(S.b_ext); add(S.x_ext); add(S.bm); add(S.r64); add(S.s64); add(S.y64); add(S.p64); add(S.q64); add(S.x3_64);
   add(S.xf); add(S.r32); add(S.s32); add(S.y32); add(S.p32); add(S.q32); add(S.x3_32); add(S.partials);
-  add(S.tasks_f); add(S.tasks_b);
+  bytes += S.sweep[0].bytes() + S.sweep[1].bytes();
   add(S.bb_ext[0]); add(S.bx_ext[0]); add(S.bb_ext[1]); add(S.bx_ext[1]); add(S.bbm); add(S.br64); add(S.bxf); add(S.bpartials); add(S.br32); add(S.bs32);
   add(S.by32); add(S.bp32); add(S.bq32); add(S.bx3_32); add(S.bs64); add(S.by64); add(S.bp64); add(S.bq64);
   add(S.bx3_64);
@@ -3090,15 +3150,15 @@ int acg_serve_open(acg_solver* h, int precision, int slots, int queue, acg_serve
       // solver's values) for ready inputs, and the columns admitted in the
       // first tick began their PCG from a wrong z.  The columns' other vectors
       // start at zero, so free slots carry finite values through the sweeps.
-      const size_t N = (size_t)S.n * srv->kp;
+      const size_t N = (size_t)S.n * srv->kp, Ns = (size_t)S.batch_sweep().nslots * srv->kp;
       for (acg::DevBuf<double>* b : {&S.bbm, &S.br64, &S.bxf, &S.bp64, &S.bq64})
         ACG_CUDA(cudaMemsetAsync(b->p, 0, sizeof(double) * N, S.stream));
       ACG_CUDA(cudaMemsetAsync(S.bx3_64.p, 0, sizeof(double) * 3 * N, S.stream));
       for (acg::DevBuf<float>* b : {&S.br32, &S.bp32, &S.bq32})
         ACG_CUDA(cudaMemsetAsync(b->p, 0, sizeof(float) * N, S.stream));
       ACG_CUDA(cudaMemsetAsync(S.bx3_32.p, 0, sizeof(float) * 3 * N, S.stream));
-      acg::k_fill_pending<double><<<acg::kVecBlocks, acg::kVecThreads, 0, S.stream>>>((int)N, S.bs64.p, S.by64.p);
-      acg::k_fill_pending<float><<<acg::kVecBlocks, acg::kVecThreads, 0, S.stream>>>((int)N, S.bs32.p, S.by32.p);
+      acg::k_fill_pending<double><<<acg::kVecBlocks, acg::kVecThreads, 0, S.stream>>>(Ns, S.bs64.p, S.by64.p);
+      acg::k_fill_pending<float><<<acg::kVecBlocks, acg::kVecThreads, 0, S.stream>>>(Ns, S.bs32.p, S.by32.p);
       ACG_CUDA(cudaGetLastError());
     }
     acg::with_cpl(srv->kp, [&](auto cpl) {
