@@ -308,7 +308,9 @@ int acg_ldlsolve(acg_solver* h, const double* r, double* y, int precision);
 /* y = lap(a) * x on the device (FP64 or FP32 values); host arrays. */
 int acg_lap_mul(acg_solver* h, const double* x, double* y, int precision);
 /* Time the solve's kernels: each captured `reps` times into a CUDA graph and
- * timed with CUDA events on the solver's stream (no reference counterpart). */
+ * timed with CUDA events on the solver's stream (no reference counterpart).
+ * One-vector solves run their whole PCG in one launch; the times here are of
+ * the same phases as separate launches. */
 int acg_time_kernels(acg_solver* h, int precision, int reps, acg_kernel_times* out);
 /* The same for the batched kernels with nrhs (<= 64) right-hand sides
  * (iteration_ms is not measured there). */

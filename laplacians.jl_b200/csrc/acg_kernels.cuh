@@ -67,6 +67,7 @@ struct PcgState {
   int entering;                // joined a running serving loop: this pass is its pre-loop step
   int pad1;
   double pq_dot;               // batched loop: p.q summed by the mat-vec
+  double elapsed;              // one-launch solves: seconds since t_start, as every block reads them
   unsigned int counter[16];    // last-block tickets of the reducing kernels
 };
 
@@ -497,14 +498,14 @@ __device__ __forceinline__ void load_entries(SweepEntries<T, U>& e, const SweepT
 // Single-vector mixed solve on the 1M grid: 39.5 -> 36.9 ms.  FP64 keeps the
 // waits one by one: with joint polls, 256 graphs in one FP64 launch (many
 // graphs, thousands of tasks per level) went from 146.7 to 156.3 ms.
-template <typename T, int U>
+template <typename T, int U, bool kJoint = sizeof(T) == 4>
 __device__ __forceinline__ void gather_entries(T& acc, const int (&id)[U], const T (&c)[U], const T* out, int vs,
                                                PcgState* st, int poll_mode, unsigned spin_limit) {
   T xv[U];
 #pragma unroll
   for (int j = 0; j < U; ++j) xv[j] = id[j] >= 0 ? ld_relaxed(&out[(size_t)id[j] * vs]) : T(0);
   unsigned pend = 0;
-  if constexpr (sizeof(T) == 4) {
+  if constexpr (kJoint) {
 #pragma unroll
     for (int j = 0; j < U; ++j)
       if (id[j] >= 0 && is_pending(xv[j])) pend |= 1u << j;
@@ -679,8 +680,27 @@ __global__ void k_fill_pending(size_t n, T* a, T* b, int vs = 1) {
   }
 }
 
-// Marks the work slots [n, nslots) of the one-vector sweep vectors pending
-// (the kernels that mark the n values of s and y).
+// What the kernels that mark the n values of s and y pending mark besides: the
+// work slots [n, nslots) of both, and for the one-launch solve (acg_persist.cuh)
+// its reduction slots and packed tail values.
+template <typename T>
+struct MarkArgs {
+  int nslots;
+  double* red;
+  int nred;
+  T* wt;
+  int nwt;
+};
+template <typename T>
+__device__ __forceinline__ void mark_work_slots(int n, int nslots, T* s, T* y, int vs);
+template <typename T>
+__device__ __forceinline__ void mark_all(int n, const MarkArgs<T>& m, T* s, T* y, int vs) {
+  mark_work_slots(n, m.nslots, s, y, vs);
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < m.nred; i += gridDim.x * blockDim.x)
+    m.red[i] = pending_value<double>();
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < m.nwt; i += gridDim.x * blockDim.x)
+    m.wt[i] = pending_value<T>();
+}
 template <typename T>
 __device__ __forceinline__ void mark_work_slots(int n, int nslots, T* s, T* y, int vs) {
   const T pv = pending_value<T>();

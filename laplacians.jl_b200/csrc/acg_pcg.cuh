@@ -116,12 +116,15 @@ __device__ __forceinline__ bool pcg_scalar_rho(PcgState* st, double rho) {
 
 // the rest of the iteration: the third L1 test (every 10th iteration, with
 // st->sum_abs_z of this iteration's z), maxtime and maxits (src/pcg.jl:406-432)
-__device__ __forceinline__ bool pcg_scalar_tail(PcgState* st, double eps) {
+// `el`: seconds since t_start.
+__device__ __forceinline__ bool pcg_scalar_tail(PcgState* st, double eps, double el) {
   if (st->itcnt % 10 == 0 && st->beta * st->sum_abs_p < eps * st->sum_abs_z) return mark_stop(st, kStagP);
-  const double el = (double)(globaltimer_ns() - st->t_start) * 1e-9;
   if (el > st->maxtime_s) return mark_stop(st, kMaxtime);
   if (st->itcnt >= st->maxits) return mark_stop(st, kMaxits);
   return false;
+}
+__device__ __forceinline__ bool pcg_scalar_tail(PcgState* st, double eps) {
+  return pcg_scalar_tail(st, eps, (double)(globaltimer_ns() - st->t_start) * 1e-9);
 }
 
 // The pre-loop step of a system that joined a running serving loop, taken in
@@ -273,10 +276,10 @@ __global__ void __launch_bounds__(kVecThreads) k_gather_in(int n, const int* __r
 template <typename T>
 __global__ void __launch_bounds__(kVecThreads) k_center(int n, double* __restrict__ bm, T* __restrict__ r, T* __restrict__ x0,
                                                         T* __restrict__ s_out, T* __restrict__ y_out, PcgState* st,
-                                                        double* partials, LoopCtl ctl, int vs, int nslots) {
+                                                        double* partials, LoopCtl ctl, int vs, MarkArgs<T> marks) {
   const double mu = st->mean;
   const T pend = pending_value<T>();
-  if (s_out) mark_work_slots(n, nslots, s_out, y_out, vs);
+  if (s_out) mark_all(n, marks, s_out, y_out, vs);
   double acc[2] = {0.0, 0.0};
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     const double v = bm[i] - mu;
@@ -365,10 +368,10 @@ template <typename T>
 __global__ void __launch_bounds__(kVecThreads) k_outer_prep(int n, const double* __restrict__ r64, T* __restrict__ rin,
                                                             T* __restrict__ x0, T* __restrict__ s_out, T* __restrict__ y_out,
                                                             PcgState* st, double* partials, LoopCtl inner_ctl, int vs,
-                                                           int nslots) {
+                                                           MarkArgs<T> marks) {
   const double inv = 1.0 / st->scale;
   const T pend = pending_value<T>();
-  mark_work_slots(n, nslots, s_out, y_out, vs);
+  mark_all(n, marks, s_out, y_out, vs);
   double acc[2] = {0.0, 0.0};
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     const T v = (T)(r64[i] * inv);

@@ -23,6 +23,7 @@
 #include "acg_batch.cuh"
 #include "acg_dense.cuh"
 #include "acg_group.cuh"
+#include "acg_persist.cuh"
 #include "acg_serve.cuh"
 
 namespace acg {
@@ -159,6 +160,13 @@ struct SolverImpl {
   PcgState* h_st = nullptr;  // pinned host mirror
 
   cudaGraphExec_t exec[2] = {nullptr, nullptr};
+  // one-vector solves in one launch (acg_persist.cuh): per value type the grid
+  // and W = M^T diag(g) M of the dense tail, or of the whole graph (w_K = n)
+  bool persist = false;
+  int persist_blocks[2] = {0, 0};
+  int w_K = 0, w_v0 = 0;
+  DevBuf<double> W64, r64b, p64b, wt64, red;
+  DevBuf<float> W32, r32b, p32b, wt32;
   std::mutex mu;
   unsigned char* noalloc_scratch = nullptr;  // device address of the fixed scratch array
 
@@ -464,6 +472,96 @@ void enqueue_pcg_iteration(cudaStream_t s, const SolverImpl& S, T* r, T* sv, T* 
   k_pupdate<T><<<kVecBlocks, kVecThreads, 0, s>>>(S.n, y, p, S.st, vs);
 }
 
+// ---- one-launch solves ---------------------------------------------------------
+
+template <typename T>
+MarkArgs<T> mark_args(const SolverImpl& S) {
+  MarkArgs<T> m = {S.sweep[0].nslots, nullptr, 0, nullptr, 0};
+  if (S.persist) {
+    m.red = S.red.p;
+    m.nred = persist_slots(S.persist_blocks[plan_index<T>()]);
+    m.nwt = S.w_K;
+    if constexpr (sizeof(T) == 8) m.wt = S.wt64.p;
+    else m.wt = S.wt32.p;
+  }
+  return m;
+}
+
+template <typename T>
+size_t persist_smem(int K) {
+  return (size_t)w_stride(K) * sizeof(T);
+}
+
+// The whole PCG of one right-hand side (r, x buffer 0 and the state set up by
+// k_center or k_outer_prep) as one cooperative launch.
+template <typename T>
+void enqueue_persist(cudaStream_t s, const SolverImpl& S, double eps, int init) {
+  PersistArgs<T> P = {};
+  const DevSweep& D = S.sweep[0];
+  const TypedArrays<T> A = arrays_of<T>(S);
+  P.n = S.n;
+  P.nslots = D.nslots;
+  P.vs = vstride<T>(S);
+  // four entries a lane in flight: half the lanes of the plain mat-vec cover a row
+  P.vl = std::max(2, S.vl_spmv / 2);
+  P.lp = A.lp;
+  P.li = A.li;
+  P.lv = A.lv;
+  P.ntf = D.ntasks_f;
+  P.ntb = D.ntasks_b;
+  P.tf = D.tasks_f.p;
+  P.tb = D.tasks_b.p;
+  P.fi = D.f_idx.p;
+  P.bi = D.b_idx.p;
+  P.fc = D.coef<T>(true);
+  P.bc = D.coef<T>(false);
+  P.g = A.g;
+  P.K = S.w_K;
+  P.v0 = S.w_K ? S.w_v0 : S.n;
+  if constexpr (sizeof(T) == 8) {
+    P.W = S.W64.p;
+    P.r0 = S.r64.p; P.r1 = S.r64b.p; P.p0 = S.p64.p; P.p1 = S.p64b.p;
+    P.q = S.q64.p; P.x3 = S.x3_64.p; P.s = S.s64.p; P.y = S.y64.p; P.wt = S.wt64.p;
+  } else {
+    P.W = S.W32.p;
+    P.r0 = S.r32.p; P.r1 = S.r32b.p; P.p0 = S.p32.p; P.p1 = S.p32b.p;
+    P.q = S.q32.p; P.x3 = S.x3_32.p; P.s = S.s32.p; P.y = S.y32.p; P.wt = S.wt32.p;
+  }
+  P.red = S.red.p;
+  P.st = S.st;
+  P.eps = eps;
+  P.init = init;
+  P.poll_mode = S.poll_mode;
+  P.spin_limit = S.spin_limit;
+  // a block idle through a long sweep polls a reduction all the while; a wait
+  // that gives up elsewhere ends it early
+  P.red_limit = std::max(S.spin_limit, kSpinLimit);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(S.persist_blocks[plan_index<T>()]);
+  cfg.blockDim = dim3(kPersistThreads);
+  cfg.dynamicSmemBytes = persist_smem<T>(S.w_K);
+  cfg.stream = s;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeCooperative;
+  at[0].val.cooperative = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  if (S.w_K == S.n) ACG_CUDA(cudaLaunchKernelEx(&cfg, k_pcg<T, true>, P));
+  else ACG_CUDA(cudaLaunchKernelEx(&cfg, k_pcg<T, false>, P));
+}
+
+// Resident blocks of k_pcg: at most `want` per SM.
+template <typename T>
+int persist_grid(int sms, int want, int K, bool whole) {
+  int occ = 0;
+  const int smem = (int)persist_smem<T>(K);
+  auto kern = whole ? k_pcg<T, true> : k_pcg<T, false>;
+  ACG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)persist_smem<T>(kDenseMaxK)));
+  ACG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, kPersistThreads, smem));
+  return sms * std::max(1, std::min(want, occ));
+}
+
 // ---- graph construction -----------------------------------------------------
 
 // Current leaf nodes of a capture in progress.
@@ -497,20 +595,49 @@ void end_into(cudaStream_t s) {
   ACG_CUDA(cudaStreamEndCapture(s, &g));
 }
 
+// Ends the capture in progress; its leaf nodes.
+std::vector<cudaGraphNode_t> capture_end(cudaStream_t s) {
+  std::vector<cudaGraphNode_t> leaves = capture_leaves(s);
+  end_into(s);
+  return leaves;
+}
+
+// The end of an FP64 solve after the nodes `deps`: best x, its true residual,
+// the caller's vertex order.
+cudaGraphExec_t finish_fp64_graph(SolverImpl& S, cudaGraph_t top, const std::vector<cudaGraphNode_t>& deps) {
+  cudaStream_t s = S.stream;
+  begin_into(s, top, deps);
+  k_take_best<double><<<kVecBlocks, kVecThreads, 0, s>>>(S.n, S.x3_64.p, S.xf.p, S.st);
+  {
+    using T = double;
+    ACG_VL_SWITCH(S.vl_spmv, true_res_vl, s, S, S.xf.p, S.bm.p, nullptr, S.st);
+  }
+  k_scatter_out<<<kVecBlocks, kVecThreads, 0, s>>>(S.n, S.perm.p, S.xf.p, S.x_ext.p);
+  end_into(s);
+  cudaGraphExec_t exec;
+  ACG_CUDA(cudaGraphInstantiate(&exec, top, 0));
+  cudaGraphDestroy(top);
+  return exec;
+}
+
 // Plain FP64 PCG, the reference algorithm end to end.
 cudaGraphExec_t build_fp64_graph(SolverImpl& S) {
   cudaStream_t s = S.stream;
   const int n = S.n;
   cudaGraph_t top;
   ACG_CUDA(cudaGraphCreate(&top, 0));
-  cudaGraphConditionalHandle h;
-  ACG_CUDA(cudaGraphConditionalHandleCreate(&h, top, 1u, cudaGraphCondAssignDefault));
-  LoopCtl ctl{h, 1};
+  cudaGraphConditionalHandle h{};
+  if (!S.persist) ACG_CUDA(cudaGraphConditionalHandleCreate(&h, top, 1u, cudaGraphCondAssignDefault));
+  LoopCtl ctl{h, S.persist ? 0 : 1};
 
   begin_into(s, top, {});
   k_gather_in<<<kVecBlocks, kVecThreads, 0, s>>>(n, S.perm.p, S.b_ext.p, S.bm.p, S.st, S.partials.p);
   k_center<double><<<kVecBlocks, kVecThreads, 0, s>>>(n, S.bm.p, S.r64.p, S.x3_64.p, S.s64.p, S.y64.p, S.st,
-                                                      S.partials.p, ctl, S.vs64, S.sweep[0].nslots);
+                                                      S.partials.p, ctl, S.vs64, mark_args<double>(S));
+  if (S.persist) {
+    enqueue_persist<double>(s, S, kEps64, 1);
+    return finish_fp64_graph(S, top, capture_end(s));
+  }
   enqueue_sweeps<double>(s, S, S.r64.p, S.s64.p, S.y64.p, S.st);
   k_ysum<double><<<kVecBlocks, kVecThreads, 0, s>>>(n, S.y64.p, S.st, S.partials.p, ctl, S.vs64);
   k_zdot<double><<<kVecBlocks, kVecThreads, 0, s>>>(n, S.y64.p, S.r64.p, S.p64.p, S.st, S.partials.p, kEps64, 1, ctl,
@@ -523,14 +650,25 @@ cudaGraphExec_t build_fp64_graph(SolverImpl& S) {
   begin_into(s, body, {});
   enqueue_pcg_iteration<double>(s, S, S.r64.p, S.s64.p, S.y64.p, S.p64.p, S.q64.p, S.x3_64.p, kEps64, ctl);
   end_into(s);
+  return finish_fp64_graph(S, top, {wnode});
+}
 
-  begin_into(s, top, {wnode});
-  k_take_best<double><<<kVecBlocks, kVecThreads, 0, s>>>(n, S.x3_64.p, S.xf.p, S.st);
+// The end of a refinement step after the inner solve's nodes `deps` (in the
+// loop body obody), and of the solve after the loop node.
+cudaGraphExec_t finish_mixed_graph(SolverImpl& S, cudaGraph_t top, cudaGraph_t obody, cudaGraphNode_t onode,
+                                   LoopCtl octl, const std::vector<cudaGraphNode_t>& deps) {
+  cudaStream_t s = S.stream;
+  begin_into(s, obody, deps);
+  k_outer_correct<float><<<kVecBlocks, kVecThreads, 0, s>>>(S.n, S.x3_32.p, S.xf.p, S.st);
   {
     using T = double;
-    ACG_VL_SWITCH(S.vl_spmv, true_res_vl, s, S, S.xf.p, S.bm.p, nullptr, S.st);
+    ACG_VL_SWITCH(S.vl_spmv, true_res_vl, s, S, S.xf.p, S.bm.p, S.r64.p, S.st);
   }
-  k_scatter_out<<<kVecBlocks, kVecThreads, 0, s>>>(n, S.perm.p, S.xf.p, S.x_ext.p);
+  k_outer_decide<<<1, 32, 0, s>>>(S.st, octl);
+  end_into(s);
+
+  begin_into(s, top, {onode});
+  k_scatter_out<<<kVecBlocks, kVecThreads, 0, s>>>(S.n, S.perm.p, S.xf.p, S.x_ext.p);
   end_into(s);
 
   cudaGraphExec_t exec;
@@ -554,19 +692,23 @@ cudaGraphExec_t build_mixed_graph(SolverImpl& S) {
   k_gather_in<<<kVecBlocks, kVecThreads, 0, s>>>(n, S.perm.p, S.b_ext.p, S.bm.p, S.st, S.partials.p);
   // r64 = bm, x64 (xf) = 0
   k_center<double><<<kVecBlocks, kVecThreads, 0, s>>>(n, S.bm.p, S.r64.p, S.xf.p, (double*)nullptr,
-                                                      (double*)nullptr, S.st, S.partials.p, octl, 1, n);
+                                                      (double*)nullptr, S.st, S.partials.p, octl, 1, MarkArgs<double>{});
   std::vector<cudaGraphNode_t> leaves = capture_leaves(s);
   end_into(s);
 
   cudaGraph_t obody;
   cudaGraphNode_t onode = add_while(top, leaves, ho, &obody);
-  cudaGraphConditionalHandle hi;
-  ACG_CUDA(cudaGraphConditionalHandleCreate(&hi, obody, 1u, cudaGraphCondAssignDefault));
-  LoopCtl ictl{hi, 1};
+  cudaGraphConditionalHandle hi{};
+  if (!S.persist) ACG_CUDA(cudaGraphConditionalHandleCreate(&hi, obody, 1u, cudaGraphCondAssignDefault));
+  LoopCtl ictl{hi, S.persist ? 0 : 1};
 
   begin_into(s, obody, {});
   k_outer_prep<float><<<kVecBlocks, kVecThreads, 0, s>>>(n, S.r64.p, S.r32.p, S.x3_32.p, S.s32.p, S.y32.p, S.st,
-                                                         S.partials.p, ictl, S.vs32, S.sweep[0].nslots);
+                                                         S.partials.p, ictl, S.vs32, mark_args<float>(S));
+  if (S.persist) {
+    enqueue_persist<float>(s, S, eps32, 2);
+    return finish_mixed_graph(S, top, obody, onode, octl, capture_end(s));
+  }
   enqueue_sweeps<float>(s, S, S.r32.p, S.s32.p, S.y32.p, S.st);
   k_ysum<float><<<kVecBlocks, kVecThreads, 0, s>>>(n, S.y32.p, S.st, S.partials.p, ictl, S.vs32);
   k_zdot<float><<<kVecBlocks, kVecThreads, 0, s>>>(n, S.y32.p, S.r32.p, S.p32.p, S.st, S.partials.p, eps32, 2, ictl,
@@ -580,23 +722,7 @@ cudaGraphExec_t build_mixed_graph(SolverImpl& S) {
   enqueue_pcg_iteration<float>(s, S, S.r32.p, S.s32.p, S.y32.p, S.p32.p, S.q32.p, S.x3_32.p, eps32, ictl);
   end_into(s);
 
-  begin_into(s, obody, {inode});
-  k_outer_correct<float><<<kVecBlocks, kVecThreads, 0, s>>>(n, S.x3_32.p, S.xf.p, S.st);
-  {
-    using T = double;
-    ACG_VL_SWITCH(S.vl_spmv, true_res_vl, s, S, S.xf.p, S.bm.p, S.r64.p, S.st);
-  }
-  k_outer_decide<<<1, 32, 0, s>>>(S.st, octl);
-  end_into(s);
-
-  begin_into(s, top, {onode});
-  k_scatter_out<<<kVecBlocks, kVecThreads, 0, s>>>(n, S.perm.p, S.xf.p, S.x_ext.p);
-  end_into(s);
-
-  cudaGraphExec_t exec;
-  ACG_CUDA(cudaGraphInstantiate(&exec, top, 0));
-  cudaGraphDestroy(top);
-  return exec;
+  return finish_mixed_graph(S, top, obody, onode, octl, {inode});
 }
 
 }  // namespace
@@ -691,6 +817,39 @@ void validate_inputs(int64_t n64, const int64_t* a_colptr, const int64_t* a_rowv
   }
   for (int64_t v = 0; v < n; ++v)
     if (!(d[v] >= 0.0) || std::isinf(d[v])) throw InputError("ldli.d must be finite and non-negative");
+}
+
+// M = (I - C)^{-1} of the vertices [v0, v0 + K) (closed under successors), row
+// by row: M[i,:] = e_i + sum over inputs u of i in the range of coef * M[u,:]
+// (inputs precede i in internal order).  Threads own interleaved blocks of 64
+// columns and walk all rows, so no thread waits for another and each entry is
+// summed in one fixed order.
+std::vector<double> triangular_inverse(const std::vector<int>& fptr, const std::vector<int>& fidx,
+                                       const std::vector<double>& fc, int v0, int K) {
+  std::vector<double> m((size_t)K * K, 0.0);
+  const int nthreads = std::max(1, std::min(K / 64, std::min(32, (int)std::thread::hardware_concurrency())));
+  auto work = [&](int tid) {
+    for (int i = 0; i < K; ++i) {
+      double* row = &m[(size_t)i * K];
+      for (int cb = tid * 64; cb <= i; cb += nthreads * 64) {
+        const int ce = std::min(cb + 64, i + 1);
+        if (i >= cb && i < ce) row[i] = 1.0;
+        for (int k = fptr[v0 + i]; k < fptr[v0 + i + 1]; ++k) {
+          const int u = fidx[k] - v0;
+          if (u < 0) continue;
+          const double c = fc[k];
+          const double* mu = &m[(size_t)u * K];
+          const int e2 = std::min(ce, u + 1);
+          for (int j = cb; j < e2; ++j) row[j] += c * mu[j];
+        }
+      }
+    }
+  };
+  std::vector<std::thread> pool;
+  for (int t = 1; t < nthreads; ++t) pool.emplace_back(work, t);
+  work(0);
+  for (auto& t : pool) t.join();
+  return m;
 }
 
 // Builds the device solver for one graph, or for the block-diagonal union of
@@ -881,36 +1040,17 @@ void build_solver(SolverImpl& S, int64_t n64, const int64_t* a_colptr, const int
       S.dt_K = n - S.dt_v0;
     }
   }
+  // One-vector solves run as one launch, except for the engines with their own
+  // launches per level and for groups.  Small graphs have W for every vertex.
+  S.persist = nseg == 1 && !(opts && (opts->sweep_lanes == 1 || opts->tail == 2));
+  const bool w_whole = S.persist && n <= kDenseWhole && !(opts && opts->dense_tail != 0) &&
+                       !(opts && opts->test_unproduced_task > 0);
+  std::vector<double> whole_m;
+  if (w_whole) whole_m = triangular_inverse(fptr, fidx, fc, 0, n);
   std::vector<double> dense_m;
   if (S.dt_K) {
     const int K = S.dt_K, v0 = S.dt_v0;
-    // M = (I - C_TT)^{-1}, row by row: M[i,:] = e_i + sum over tail inputs u of
-    // i of coef * M[u,:] (inputs precede i in internal order).  Threads own
-    // interleaved blocks of 64 columns and walk all rows, so no thread waits
-    // for another and each entry is summed in one fixed order.
-    dense_m.assign((size_t)K * K, 0.0);
-    const int nthreads = std::max(1, std::min(32, (int)std::thread::hardware_concurrency()));
-    auto work = [&](int tid) {
-      for (int i = 0; i < K; ++i) {
-        double* row = &dense_m[(size_t)i * K];
-        for (int cb = tid * 64; cb <= i; cb += nthreads * 64) {
-          const int ce = std::min(cb + 64, i + 1);
-          if (i >= cb && i < ce) row[i] = 1.0;
-          for (int k = fptr[v0 + i]; k < fptr[v0 + i + 1]; ++k) {
-            const int u = fidx[k] - v0;
-            if (u < 0) continue;
-            const double c = fc[k];
-            const double* mu = &dense_m[(size_t)u * K];
-            const int e2 = std::min(ce, u + 1);
-            for (int j = cb; j < e2; ++j) row[j] += c * mu[j];
-          }
-        }
-      }
-    };
-    std::vector<std::thread> pool;
-    for (int t = 1; t < nthreads; ++t) pool.emplace_back(work, t);
-    work(0);
-    for (auto& t : pool) t.join();
+    dense_m = triangular_inverse(fptr, fidx, fc, v0, K);
     // the sweep keeps only the head inputs of tail vertices (a prefix: entries
     // are in increasing internal order)
     std::vector<int> nptr(n + 1, 0);
@@ -1204,6 +1344,34 @@ void build_solver(SolverImpl& S, int64_t n64, const int64_t* a_colptr, const int
   for (DevBuf<float>* b : {&S.s32, &S.y32}) b->alloc((size_t)S.sweep[0].nslots * S.vs32);
   S.x3_32.alloc((size_t)3 * n);
   S.partials.alloc((size_t)4 * kMaxPartialBlocks);
+  if (S.persist) {
+    S.w_K = w_whole ? n : S.dt_K;
+    S.w_v0 = w_whole ? 0 : S.dt_v0;
+    if (S.w_K) {
+      const int K = S.w_K, ldw = w_stride(K);
+      DevBuf<double> m;
+      if (w_whole) m.upload(whole_m, s);
+      S.W64.alloc((size_t)K * ldw);
+      S.W32.alloc((size_t)K * ldw);
+      k_form_w<<<dim3(ldw / kWTile, (K + kWTile - 1) / kWTile), 256, 0, s>>>(
+          K, ldw, w_whole ? m.p : S.dt_M64.p, S.g64.p + S.w_v0, S.W64.p, S.W32.p);
+      ACG_CUDA(cudaGetLastError());
+      ACG_CUDA(cudaStreamSynchronize(s));
+      m.free();
+    }
+    int sms = 0;
+    ACG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, S.device));
+    const int want = S.w_K == n ? 1 : std::max(S.sweep_blocks[0], S.sweep_blocks[1]) / sms;
+    S.persist_blocks[0] = persist_grid<double>(sms, want, S.w_K, S.w_K == n);
+    S.persist_blocks[1] = persist_grid<float>(sms, want, S.w_K, S.w_K == n);
+    S.red.alloc(persist_slots(std::max(S.persist_blocks[0], S.persist_blocks[1])));
+    if (w_whole) {
+      for (DevBuf<double>* b : {&S.r64b, &S.p64b}) b->alloc(n);
+      for (DevBuf<float>* b : {&S.r32b, &S.p32b}) b->alloc(n);
+    }
+    S.wt64.alloc(S.w_K);
+    S.wt32.alloc(S.w_K);
+  }
   ACG_CUDA(cudaMalloc(&S.st, sizeof(PcgState)));
   ACG_CUDA(cudaMemsetAsync(S.st, 0, sizeof(PcgState), s));
   ACG_CUDA(cudaMallocHost(&S.h_st, sizeof(PcgState)));
@@ -2744,6 +2912,7 @@ int acg_solver_stats(const acg_solver* h, acg_stats* out) {
   add(S.b_ext); add(S.x_ext); add(S.bm); add(S.r64); add(S.s64); add(S.y64); add(S.p64); add(S.q64); add(S.x3_64);
   add(S.xf); add(S.r32); add(S.s32); add(S.y32); add(S.p32); add(S.q32); add(S.x3_32); add(S.partials);
   bytes += S.sweep[0].bytes() + S.sweep[1].bytes();
+  add(S.W64); add(S.W32); add(S.r64b); add(S.p64b); add(S.r32b); add(S.p32b); add(S.wt64); add(S.wt32); add(S.red);
   add(S.bb_ext[0]); add(S.bx_ext[0]); add(S.bb_ext[1]); add(S.bx_ext[1]); add(S.bbm); add(S.br64); add(S.bxf); add(S.bpartials); add(S.br32); add(S.bs32);
   add(S.by32); add(S.bp32); add(S.bq32); add(S.bx3_32); add(S.bs64); add(S.by64); add(S.bp64); add(S.bq64);
   add(S.bx3_64);
