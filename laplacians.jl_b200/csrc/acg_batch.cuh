@@ -696,14 +696,12 @@ struct Vec16<double> {
 // kernels that can set a graph's conditional handle.
 template <bool kLoop = true>
 __device__ __forceinline__ void batch_check_all(PcgState* st, BatchShared* bs, int kp, const LoopCtl& ctl) {
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    bool all = true;
-    for (int c = 0; c < kp; ++c) all &= (st[c].done != 0);
-    if (all) {
-      bs->all_done = 1;
-      if constexpr (kLoop) clear_loop(ctl);
-    }
+  // thread c reads its own column's flag (one thread reading them in turn paid
+  // a round trip per few columns at the end of every kernel of an iteration)
+  const int all = __syncthreads_and((int)threadIdx.x >= kp || st[threadIdx.x].done != 0);
+  if (threadIdx.x == 0 && all) {
+    bs->all_done = 1;
+    if constexpr (kLoop) clear_loop(ctl);
   }
 }
 

@@ -77,28 +77,45 @@ __global__ void __launch_bounds__(kDenseThreads) kd_partial(int K, const T* __re
   for (int a = 0; a < RT; ++a)
 #pragma unroll
     for (int b = 0; b < CT; ++b) acc[a][b] = T(0);
-  const int jend = min(K, kc * kDenseChunk + kDenseChunk);
-  for (int j0 = kc * kDenseChunk; j0 < jend; j0 += SUB) {
-    for (int e = tid; e < kDenseRows * SUB; e += kDenseThreads) {
+  // The next stage's tiles are on their way to registers while this stage is
+  // computed: with few columns a stage computes for less than a load takes.
+  constexpr int NA = kDenseRows * SUB / kDenseThreads, NB = SUB * kp / kDenseThreads;
+  T ra[NA], rb[NB];
+  auto load = [&](int j0) {
+#pragma unroll
+    for (int q = 0; q < NA; ++q) {
+      const int e = tid + q * kDenseThreads;
       // forward reads rows of M along j, backward reads rows of M along i:
       // both coalesced, both conflict-free in shared memory
-      const int rr = kFwd ? e / SUB : e % kDenseRows;
-      const int jj = kFwd ? e % SUB : e / kDenseRows;
-      const int ii = i0 + rr, j = j0 + jj;
-      T a = T(0);
-      if (ii < K && j < K && (kFwd ? j <= ii : j >= ii)) a = kFwd ? M[(size_t)ii * K + j] : M[(size_t)j * K + ii];
-      As[rr][jj] = a;
+      const int ii = i0 + (kFwd ? e / SUB : e % kDenseRows), j = j0 + (kFwd ? e % SUB : e / kDenseRows);
+      ra[q] = T(0);
+      if (ii < K && j < K && (kFwd ? j <= ii : j >= ii)) ra[q] = kFwd ? M[(size_t)ii * K + j] : M[(size_t)j * K + ii];
     }
-    for (int e = tid; e < SUB * kp; e += kDenseThreads) {
-      const int jj = e / kp, c = e % kp, j = j0 + jj;
-      T b = T(0);
+#pragma unroll
+    for (int q = 0; q < NB; ++q) {
+      const int e = tid + q * kDenseThreads, j = j0 + e / kp;
+      rb[q] = T(0);
       if (j < K) {
-        b = src[(size_t)j * kp + c];
-        if (!kFwd) b *= g[j];
+        rb[q] = src[(size_t)j * kp + e % kp];
+        if (!kFwd) rb[q] *= g[j];
       }
-      Bs[jj][c] = b;
+    }
+  };
+  const int jend = min(K, kc * kDenseChunk + kDenseChunk);
+  load(kc * kDenseChunk);
+  for (int j0 = kc * kDenseChunk; j0 < jend; j0 += SUB) {
+#pragma unroll
+    for (int q = 0; q < NA; ++q) {
+      const int e = tid + q * kDenseThreads;
+      As[kFwd ? e / SUB : e % kDenseRows][kFwd ? e % SUB : e / kDenseRows] = ra[q];
+    }
+#pragma unroll
+    for (int q = 0; q < NB; ++q) {
+      const int e = tid + q * kDenseThreads;
+      Bs[e / kp][e % kp] = rb[q];
     }
     __syncthreads();
+    if (j0 + SUB < jend) load(j0 + SUB);
 #pragma unroll 4
     for (int jj = 0; jj < SUB; ++jj) {
       T a[RT], b[CT];
@@ -195,8 +212,14 @@ __global__ void __launch_bounds__(kVecThreads) kd_reduce(int K, int kp, const T*
   for (size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x; e < N; e += (size_t)gridDim.x * blockDim.x) {
     const int rt = (int)(e / kp) / kDenseRows;
     T sum = T(0);
-    for (int kc = 0; kc < nch; ++kc)
-      if (dense_active(kFwd, rt, kc)) sum += part[(size_t)kc * N + e];
+    for (int k0 = 0; k0 < nch; k0 += 8) {
+      T v[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u)
+        v[u] = k0 + u < nch && dense_active(kFwd, rt, k0 + u) ? part[(size_t)(k0 + u) * N + e] : T(0);
+#pragma unroll
+      for (int u = 0; u < 8; ++u) sum += v[u];
+    }
     dst[(e / kp) * rs + e % kp] = sum;
   }
 }

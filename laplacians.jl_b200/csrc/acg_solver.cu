@@ -1710,15 +1710,34 @@ void enqueue_bsweeps(cudaStream_t s, const SolverImpl& S, const T* r, T* sv, T* 
   enqueue_bbackward<T, CPL>(s, S, sv, y);
 }
 
+// Grids of the loop body: at most one resident wave, and no more blocks than
+// give a thread two vectors (the mat-vec: a group of lanes one row), since the
+// reductions pay for every block (8 FP64 columns of 2,627 vertices: 104 -> 87 us
+// an iteration, with the columns' flags read in parallel and the dense
+// product's next tiles on their way).
+template <typename T>
+void bvec_grids(const SolverImpl& S, int kp, int (&vg)[4]) {
+  const long long per = 2ll * kVecThreads * Vec16<T>::W;
+  const long long want = ((long long)S.n * kp + per - 1) / per;
+  for (int q = 0; q < 4; ++q)
+    vg[q] = (int)std::max(1ll, std::min<long long>(S.bvec_blocks[plan_index<T>()][q], want));
+}
+template <typename T>
+int bspmv_grid(const SolverImpl& S, int kp) {
+  const int rows = kVecThreads / kBatchLanes;
+  return std::min(S.bspmv_blocks[plan_index<T>()][kp_index(kp)], (S.n + rows - 1) / rows);
+}
+
 template <typename T, int CPL>
 void enqueue_biteration(cudaStream_t s, const SolverImpl& S, T* r, T* sv, T* y, T* p, T* q, T* x3, double eps,
                         LoopCtl ctl) {
   constexpr int kp = CPL * kBatchLanes;
   const TypedArrays<T> A = arrays_of<T>(S);
   const int n = S.n;
-  kb_spmv<T, CPL, true><<<S.bspmv_blocks[plan_index<T>()][kp_index(kp)], kVecThreads, 0, s>>>(
-      n, A.lp, A.li, A.lv, p, q, S.bsh, S.bst, S.bpartials.p);
-  const int* vg = S.bvec_blocks[plan_index<T>()];
+  kb_spmv<T, CPL, true><<<bspmv_grid<T>(S, kp), kVecThreads, 0, s>>>(n, A.lp, A.li, A.lv, p, q, S.bsh, S.bst,
+                                                                    S.bpartials.p);
+  int vg[4];
+  bvec_grids<T>(S, kp, vg);
   kb_pq<T><<<vg[0], kVecThreads, 0, s>>>(n, kp, p, q, S.bst, S.bsh, S.bpartials.p, eps, ctl);
   kb_update<T><<<vg[1], kVecThreads, 0, s>>>(n, kp, x3, p, q, r, S.bst, S.bsh, S.bpartials.p, ctl);
   enqueue_bsweeps<T, CPL>(s, S, r, sv, y);
@@ -2275,8 +2294,8 @@ void time_batch_t(SolverImpl& S, int reps, acg_kernel_times* out, T* r, T* sv, T
   auto fill_y = [&]() { k_fill_pending<T><<<kVecBlocks, kVecThreads, 0, s>>>(Ns, y, (T*)nullptr); };
   const double t_fill = time_graph(fill_s);
   out->spmv_ms = time_graph([&]() {
-    kb_spmv<T, CPL, true><<<S.bspmv_blocks[plan_index<T>()][kp_index(kp)], kVecThreads, 0, s>>>(
-        S.n, A.lp, A.li, A.lv, p, q, S.bsh, S.bst, S.bpartials.p);
+    kb_spmv<T, CPL, true><<<bspmv_grid<T>(S, kp), kVecThreads, 0, s>>>(S.n, A.lp, A.li, A.lv, p, q, S.bsh, S.bst,
+                                                                      S.bpartials.p);
   });
   out->forward_ms = time_graph([&]() {
     fill_s();
@@ -2329,7 +2348,8 @@ void time_batch_t(SolverImpl& S, int reps, acg_kernel_times* out, T* r, T* sv, T
     auto reset = [&]() { kb_timing_state<<<1, 64, 0, s>>>(S.bst, S.bsh, kp); };
     // the copies without the loop-condition call (the same passes; a profiler
     // measures these, not the loop's own kernels)
-    const int* vg = S.bvec_blocks[plan_index<T>()];
+    int vg[4];
+    bvec_grids<T>(S, kp, vg);
     const double t_reset = time_graph(reset);
     out->pq_ms = time_graph([&]() {
       reset();
