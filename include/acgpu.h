@@ -372,7 +372,7 @@ int acg_serve_close(acg_server* s);
  * y_dev = LDLsolver(ldli, r_dev), as acg_ldlsolve computes it, for vectors
  * already in device memory, without allocating: every piece of scratch comes
  * from one fixed device array inside the library (ACG_NOALLOC_MAX_N vertices
- * at most, about 8.5 MB, reserved on each GPU that loads the library until
+ * at most, about 10.6 MB, reserved on each GPU that loads the library until
  * the process exits).  Meant for callers that must not allocate while they
  * solve: a serving loop whose device memory is a fixed pool sized at start-up,
  * a host runtime whose own allocator owns the GPU's memory, or a caller that

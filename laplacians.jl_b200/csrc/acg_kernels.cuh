@@ -442,7 +442,9 @@ struct SweepEntries {
   __device__ __forceinline__ bool active(int lane) const {
     return ((info & 1) ? 0 : (lane >> 3)) < ((info >> 1) & 7);
   }
-  __device__ __forceinline__ int slot() const { return kind() == kRowWork ? v + delta : v; }
+  __device__ __forceinline__ bool term() const { return kind() < kRowFinal; }  // the row adds its vertex's own term
+  __device__ __forceinline__ bool value() const { return (kind() & 1) == 0; }  // the row is its vertex's value
+  __device__ __forceinline__ int slot() const { return value() ? v : v + delta; }
 };
 
 __device__ __forceinline__ SweepTask load_task(const SweepTask* __restrict__ tasks, int t, int ntasks) {
@@ -480,7 +482,7 @@ __device__ __forceinline__ void load_entries(SweepEntries<T, U>& e, const SweepT
   if (!active) k0 = k1 = 0;
   e.k0 = k0 + gl;
   e.k1 = k1;
-  const bool term = kLoadAux && active && e.kind() != kRowFinal;
+  const bool term = kLoadAux && active && e.term();
   e.a = term ? __ldg(&aux[e.v]) : T(0);
   e.own = (!kForward && term) ? __ldg(&sfwd[(size_t)e.v * vs]) : T(0);
 #pragma unroll

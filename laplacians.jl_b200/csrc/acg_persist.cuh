@@ -220,13 +220,13 @@ __device__ __forceinline__ void persist_sweep(const PersistArgs<T>& P, const T* 
   auto fetch = [&](SweepEntries<T, U>& e, T& a, T& b, const SweepTask& rec) {
     load_entries<T, true, false, U>(e, rec, lane, idx, coef, coef, coef);
     const bool lead = e.active(lane) && (lane & (e.gw() - 1)) == 0;
-    const bool term = lead && e.kind() != kRowFinal;
+    const bool term = lead && e.term();
     if constexpr (kForward) {
       a = term ? r[e.v] : T(0);
       b = T(0);
     } else {
       a = term ? __ldg(&P.g[e.v]) : T(0);
-      b = lead && e.kind() != kRowWork ? r[e.v] : T(0);
+      b = lead && e.value() ? r[e.v] : T(0);
     }
   };
   fetch(e0, a0, b0, load_task(tasks, t, ntasks));
@@ -238,7 +238,7 @@ __device__ __forceinline__ void persist_sweep(const PersistArgs<T>& P, const T* 
     const int gw = e0.gw();
     const bool lead = e0.active(lane) && (lane & (gw - 1)) == 0;
     T own = T(0);
-    if (!kForward && lead && e0.kind() != kRowFinal) own = ld_relaxed(&P.s[(size_t)e0.v * vs]);
+    if (!kForward && lead && e0.term()) own = ld_relaxed(&P.s[(size_t)e0.v * vs]);
     T acc = T(0);
     gather_entries<T, U, true>(acc, e0.id, e0.c, out, (int)vs, P.st, P.poll_mode, P.spin_limit);
     for (int k = e0.k0 + U * gw; k < e0.k1; k += 4 * gw) {
@@ -257,9 +257,9 @@ __device__ __forceinline__ void persist_sweep(const PersistArgs<T>& P, const T* 
     acc = group_sum_w(acc, gw);
     if (lead) {
       const T res = kForward ? a0 + acc : a0 * own + acc;
-      if (kForward && e0.v >= P.v0) st_relaxed(&P.wt[e0.v - P.v0], res);
+      if (kForward && e0.value() && e0.v >= P.v0) st_relaxed(&P.wt[e0.v - P.v0], res);
       else st_relaxed(&out[(size_t)e0.slot() * vs], res);
-      if (!kForward && e0.kind() != kRowWork) {
+      if (!kForward && e0.value()) {
         ysum += (double)res;
         yr += (double)res * (double)b0;
       }

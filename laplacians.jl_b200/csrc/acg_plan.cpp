@@ -95,7 +95,8 @@ void partition(Shared& s, int la, int lb, std::vector<Block>& out) {
         const double ends = 0.5 * (double)(first + last);
         const double work = all - inner;
         const double fin = (double)b.idx.size() - ends + kRowCost * ((double)b.vert.size() - ends);
-        const double rounds = std::floor((double)(longest - 1) / s.cost->row_entries);
+        const double rounds = s.cost->split ? (longest > s.cost->split ? 1.0 : 0.0)
+                                            : std::floor((double)(longest - 1) / s.cost->row_entries);
         // a level costs a hand-over and its entries; the block two hand-overs
         const double gain = (len - 2) - (work + fin - all) / A - s.cost->row_round * rounds;
         if (gain > best) {
@@ -143,6 +144,55 @@ std::vector<std::pair<int, int>> ranges(const SweepDag& d, int l0, int l1) {
   }
   out.resize(w);
   return out;
+}
+
+// Cuts the rows of R longer than `split` into parts of `part` entries with
+// slots from `base` on; returns the parts.
+int split_rows(SweepRows& R, int split, int part, int base) {
+  SweepRows out;
+  out.ptr.push_back(0);
+  out.idx.reserve(R.idx.size());
+  out.coef.reserve(R.coef.size());
+  std::vector<int> after(R.runs.size() + 1, 0);  // runs of out up to the end of run i
+  int parts = 0;
+  for (size_t i = 0; i < R.runs.size(); ++i) {
+    SweepRun run = R.runs[i];
+    const int first = parts;
+    for (int q = 0; q < run.count; ++q) {
+      const int k0 = R.ptr[run.row + q], k1 = R.ptr[run.row + q + 1];
+      if (k1 - k0 <= split) continue;
+      for (int k = k0; k < k1; k += part, ++parts) {
+        const int e = std::min(k1, k + part);
+        out.idx.insert(out.idx.end(), R.idx.begin() + k, R.idx.begin() + e);
+        out.coef.insert(out.coef.end(), R.coef.begin() + k, R.coef.begin() + e);
+        out.ptr.push_back((int)out.idx.size());
+      }
+    }
+    if (parts > first)  // v0 counts from 0: a part has no vertex
+      out.runs.push_back(SweepRun{0, parts - first, kRowPart, base + first, (int)out.ptr.size() - 1 - (parts - first)});
+    int next = first;
+    const int row = run.row;
+    run.row = (int)out.ptr.size() - 1;
+    for (int q = 0; q < run.count; ++q) {
+      const int k0 = R.ptr[row + q], k1 = R.ptr[row + q + 1];
+      if (k1 - k0 <= split) {
+        out.idx.insert(out.idx.end(), R.idx.begin() + k0, R.idx.begin() + k1);
+        out.coef.insert(out.coef.end(), R.coef.begin() + k0, R.coef.begin() + k1);
+      } else {
+        for (int k = k0; k < k1; k += part, ++next) {
+          out.idx.push_back(base + next);
+          out.coef.push_back(1.0);
+        }
+      }
+      out.ptr.push_back((int)out.idx.size());
+    }
+    out.runs.push_back(run);
+    after[i + 1] = (int)out.runs.size();
+  }
+  out.upto.resize(R.upto.size());
+  for (size_t l = 0; l < R.upto.size(); ++l) out.upto[l] = after[R.upto[l]];
+  R = std::move(out);
+  return parts;
 }
 
 }  // namespace
@@ -329,6 +379,11 @@ SweepPlan build_sweep_plan(const SweepDag& d, const SweepCost& cost, bool merge)
       }
     }
     for (int l = b.l0; l < top; ++l) B.upto[l] = (int)B.runs.size();
+  }
+  if (merge && cost.split) {  // s and y are vectors of their own: the same slots serve both
+    const int base = plan.nslots;
+    const int pf = split_rows(F, cost.split, cost.part, base), pb = split_rows(B, cost.split, cost.part, base);
+    plan.nslots += std::max(pf, pb);
   }
   return plan;
 }

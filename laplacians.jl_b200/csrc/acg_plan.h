@@ -20,7 +20,11 @@
 //   kRowPlain  out[v] = aux(v) + sum          (a block's first level)
 //   kRowWork   out[v + delta] = aux(v) + sum  (the other levels' w or w')
 //   kRowFinal  out[v] = sum                   (the same vertices' M_B row)
-// A row's sum runs over entries (slot, coefficient).
+//   kRowPart   out[v + delta] = sum           (a part of a long row)
+// A row's sum runs over entries (slot, coefficient).  A long row would keep one
+// warp through many value round trips while its block's other rows are done, so
+// the one-vector plan cuts it into parts with slots of their own (behind the
+// work slots), whose sums the row adds.
 #pragma once
 #include <cstdint>
 #include <utility>
@@ -28,7 +32,7 @@
 
 namespace acg {
 
-enum SweepRowKind { kRowPlain = 0, kRowWork = 1, kRowFinal = 2 };
+enum SweepRowKind { kRowPlain = 0, kRowWork = 1, kRowFinal = 2, kRowPart = 3 };
 
 // A run of rows of one kind over consecutive vertices [v0, v0 + count).
 struct SweepRun {
@@ -45,7 +49,7 @@ struct SweepRows {
 };
 
 struct SweepPlan {
-  int nslots = 0;  // n + work slots
+  int nslots = 0;  // n + work slots + part slots
   int blocks = 0;
   SweepRows fwd, bwd;
 };
@@ -55,6 +59,8 @@ struct SweepCost {
   double entries_per_hop;  // entries all warps work through in the time of one hand-over
   double row_entries;      // entries of one row walked before it costs another load round trip
   double row_round;        // that round trip
+  int split = 0;           // rows longer than this are cut (one more hand-over); 0: none are
+  int part = 0;            // entries of a part
 };
 
 // The DAG in internal vertex order (per graph: level by level): in-edges and

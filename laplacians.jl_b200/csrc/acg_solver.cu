@@ -735,14 +735,17 @@ namespace acg {
 namespace {
 
 // What a level merge is worth (see SweepCost): entries worked through in the
-// time of one hand-over, and the entries of a row a warp has in flight.  The
-// batched sweeps move a row of kp values per entry.  FP64 one-vector forward /
-// backward sweep in us at 10000, 25000, 60000 entries: grid3(50) 87/95, 74/90,
-// 76/103 (one level per block 258/278); grid3(100) 420/476, 358/377, 361/408.
-// 64 FP32 columns at 5000, 10000, 20000: grid3(50) 203/229, 132/160, 150/181;
-// grid3(100) 812/851, 716/777, 778/842.
-constexpr SweepCost kVectorCost{25000.0, 128.0, 0.4};
-constexpr SweepCost kBatchCost{10000.0, 32.0, 0.5};
+// time of one hand-over, the entries of a row a warp has in flight, and where a
+// row is cut.  The batched sweeps move a row of kp values per entry; their
+// rows stay whole.  FP64 one-vector forward / backward sweep in us at 10000,
+// 25000, 60000 entries (rows whole): grid3(50) 87/95, 74/90, 76/103 (one level
+// per block 258/278); grid3(100) 420/476, 358/377, 361/408.  64 FP32 columns
+// at 5000, 10000, 20000: grid3(50) 203/229, 132/160, 150/181; grid3(100)
+// 812/851, 716/777, 778/842.  us per FP64 iteration with whole rows, rows cut
+// above 256 into parts of 128, above 256 and above 160 into parts of 64: matchings
+// of 150,000 vertices 321, 238, 230, 215; grid3(50) 208, 184, 179, 173.
+constexpr SweepCost kVectorCost{25000.0, 128.0, 0.4, 160, 64};
+constexpr SweepCost kBatchCost{10000.0, 32.0, 0.5, 0, 0};
 
 template <typename T>
 std::vector<float> to_f32(const std::vector<T>& v) {
@@ -1149,7 +1152,12 @@ void build_solver(SolverImpl& S, int64_t n64, const int64_t* a_colptr, const int
   for (int w = 0; w < (S.two_plans ? 2 : 1); ++w) {
     DevSweep& P = S.sweep[w];
     const SweepDag dag{n, nlev, &runs, &fptr, &fidx, &bptr, &bidx, &fc, &bc, S.dt_K ? S.dt_L0 : nlev};
-    const SweepPlan plan = build_sweep_plan(dag, w == 0 ? kVectorCost : kBatchCost, merge);
+    SweepCost cost = w == 0 ? kVectorCost : kBatchCost;
+    SweepPlan plan = build_sweep_plan(dag, cost, merge);
+    if (w == 0 && n <= ACG_NOALLOC_MAX_N && plan.nslots > 3 * ACG_NOALLOC_MAX_N) {
+      cost.split = 0;  // the fixed scratch of acg_ldlsolve_noalloc holds two slots a vertex and more
+      plan = build_sweep_plan(dag, cost, merge);
+    }
     P.nslots = plan.nslots;
     P.nnz_f = (int64_t)plan.fwd.idx.size();
     P.nnz_b = (int64_t)plan.bwd.idx.size();
@@ -1472,9 +1480,10 @@ constexpr size_t kNoAllocPartials = (size_t)4 * kMaxPartialBlocks * sizeof(doubl
 // a dense tail has at most min(kDenseMaxK, n / 4) vertices
 constexpr int kNoAllocDenseK = kDenseMaxK < kNoAllocMaxN / 4 ? kDenseMaxK : kNoAllocMaxN / 4;
 constexpr size_t kNoAllocDense = (size_t)dense_chunks(kNoAllocDenseK) * kNoAllocDenseK * sizeof(double);
-// r as FP64 and in the sweeps' type, and the two sweep vectors with a work
-// slot per vertex at most
-constexpr size_t kNoAllocVectors = 6 * kNoAllocVec;
+// r as FP64 and in the sweeps' type, and the two sweep vectors with up to
+// three slots per vertex (values, work values and parts of long rows)
+constexpr size_t kNoAllocSlots = 3 * (size_t)kNoAllocMaxN;
+constexpr size_t kNoAllocVectors = 8 * kNoAllocVec;
 constexpr size_t kNoAllocState = kNoAllocVectors + kNoAllocPartials + kNoAllocDense;
 constexpr size_t kNoAllocBytes = kNoAllocState + ((sizeof(PcgState) + 255) / 256) * 256;
 
@@ -1503,7 +1512,7 @@ void ldlsolve_noalloc_impl(const SolverImpl& S, cudaStream_t s, const double* r_
   double* r64 = reinterpret_cast<double*>(base);
   T* rT = reinterpret_cast<T*>(base + kNoAllocVec);
   T* sv = reinterpret_cast<T*>(base + 2 * kNoAllocVec);
-  T* yv = reinterpret_cast<T*>(base + 4 * kNoAllocVec);
+  T* yv = reinterpret_cast<T*>(base + 5 * kNoAllocVec);
   double* partials = reinterpret_cast<double*>(base + kNoAllocVectors);
   T* dense_part = reinterpret_cast<T*>(base + kNoAllocVectors + kNoAllocPartials);
   PcgState* st = reinterpret_cast<PcgState*>(base + kNoAllocState);
@@ -1512,7 +1521,7 @@ void ldlsolve_noalloc_impl(const SolverImpl& S, cudaStream_t s, const double* r_
   ACG_CUDA(cudaMemsetAsync(st, 0, sizeof(PcgState), s));
   k_gather_in<<<kVecBlocks, kVecThreads, 0, s>>>(n, S.perm.p, r_ext, r64, st, partials);
   k_cast_from64<T><<<kVecBlocks, kVecThreads, 0, s>>>(n, r64, rT);
-  // compact vectors (one value per slot): the fixed array holds 2n values each
+  // compact vectors (one value per slot): the fixed array holds kNoAllocSlots each
   k_fill_pending<T><<<kVecBlocks, kVecThreads, 0, s>>>((size_t)S.sweep[0].nslots, sv, yv, 1);
   enqueue_sweeps<T>(s, S, rT, sv, yv, st, dense_part, 1);
   k_ysum<T><<<kVecBlocks, kVecThreads, 0, s>>>(n, yv, st, partials, none, 1);
