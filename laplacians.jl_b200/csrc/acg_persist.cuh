@@ -544,6 +544,54 @@ __global__ void __launch_bounds__(kPersistThreads, 2) k_pcg(const __grid_constan
   }
 }
 
+// ---- one preconditioner application (LDLsolver, src/approxChol.jl:1347-1366) ----
+//
+// Two launches instead of a dozen: k_apply_begin takes r in solver order and
+// arms the vectors, k_apply runs both sweeps, the tail and the mean removal.
+// (One right-hand side of grid3(50), FP64: 277 -> 242 us a call.)
+template <typename T>
+__global__ void __launch_bounds__(kVecThreads) k_apply_begin(PersistArgs<T> P, const int* __restrict__ perm,
+                                                             const double* __restrict__ rext, int nred) {
+  const int gtid = blockIdx.x * blockDim.x + threadIdx.x, gsize = gridDim.x * blockDim.x;
+  for (int i = gtid; i < P.n; i += gsize) P.r0[i] = (T)rext[perm[i]];
+  for (int i = gtid; i < P.nslots; i += gsize) {
+    P.s[(size_t)i * P.vs] = pending_value<T>();
+    P.y[(size_t)i * P.vs] = pending_value<T>();
+  }
+  for (int i = gtid; i < P.K; i += gsize) P.wt[i] = pending_value<T>();
+  for (int i = gtid; i < nred; i += gsize) P.red[i] = pending_value<double>();
+  if (gtid == 0) *P.st = PcgState{};
+}
+
+template <typename T, bool kWhole>
+__global__ void __launch_bounds__(kPersistThreads, 2) k_apply(const __grid_constant__ PersistArgs<T> P,
+                                                              const int* __restrict__ perm, double* __restrict__ yext) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  T* w = reinterpret_cast<T*>(smem_raw);
+  __shared__ double red_sm[kRedValues * kPersistThreads / 32];
+  const int tid = threadIdx.x, lane = tid & 31;
+  const int gtid = blockIdx.x * blockDim.x + tid, gsize = gridDim.x * blockDim.x;
+  const int K = P.K, ldw = w_stride(K);
+  const size_t vs = P.vs;
+  double ysum[1] = {0.0}, unused = 0.0;
+  if constexpr (!kWhole) persist_sweep<T, true>(P, P.r0, ysum[0], unused);
+  for (int j = tid; j < ldw; j += blockDim.x)
+    w[j] = j < K ? (kWhole ? P.r0[j] : wait_inline(&P.wt[j], P.st, P.spin_limit)) : T(0);
+  __syncthreads();
+  for (int i = gtid >> 5; i < K; i += gsize >> 5) {
+    const T res = w_row<T>(P.W + (size_t)i * ldw, w, ldw, lane);
+    if (lane == 0) {
+      st_relaxed(&P.y[(size_t)(P.v0 + i) * vs], res);
+      ysum[0] += (double)res;
+    }
+  }
+  if constexpr (!kWhole) persist_sweep<T, false>(P, P.r0, ysum[0], unused);
+  red_publish<1>(P.red, 0, ysum, red_sm);
+  red_collect<1>(P.red, 0, 1, red_sm, P.st, P.red_limit);
+  const double mean = red_sm[0] / (double)P.n;
+  for (int i = gtid; i < P.n; i += gsize) yext[perm[i]] = (double)P.y[(size_t)i * vs] - mean;
+}
+
 // W = M^T diag(g) M for the dense tail (or the whole graph): M is K x K
 // row-major lower triangular, W's rows are padded with zeros to ldw columns.
 // 64 x 64 tiles, 4 x 4 entries a thread, FP64.  Run once per solver.

@@ -492,10 +492,8 @@ size_t persist_smem(int K) {
   return (size_t)w_stride(K) * sizeof(T);
 }
 
-// The whole PCG of one right-hand side (r, x buffer 0 and the state set up by
-// k_center or k_outer_prep) as one cooperative launch.
 template <typename T>
-void enqueue_persist(cudaStream_t s, const SolverImpl& S, double eps, int init) {
+PersistArgs<T> persist_args(const SolverImpl& S) {
   PersistArgs<T> P = {};
   const DevSweep& D = S.sweep[0];
   const TypedArrays<T> A = arrays_of<T>(S);
@@ -529,13 +527,17 @@ void enqueue_persist(cudaStream_t s, const SolverImpl& S, double eps, int init) 
   }
   P.red = S.red.p;
   P.st = S.st;
-  P.eps = eps;
-  P.init = init;
   P.poll_mode = S.poll_mode;
   P.spin_limit = S.spin_limit;
   // a block idle through a long sweep polls a reduction all the while; a wait
   // that gives up elsewhere ends it early
   P.red_limit = std::max(S.spin_limit, kSpinLimit);
+  return P;
+}
+
+// A cooperative launch of the solver's persistent grid.
+template <typename T, typename... KArgs, typename... Args>
+void launch_persist(cudaStream_t s, const SolverImpl& S, void (*kern)(KArgs...), Args... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(S.persist_blocks[plan_index<T>()]);
   cfg.blockDim = dim3(kPersistThreads);
@@ -546,20 +548,42 @@ void enqueue_persist(cudaStream_t s, const SolverImpl& S, double eps, int init) 
   at[0].val.cooperative = 1;
   cfg.attrs = at;
   cfg.numAttrs = 1;
-  if (S.w_K == S.n) ACG_CUDA(cudaLaunchKernelEx(&cfg, k_pcg<T, true>, P));
-  else ACG_CUDA(cudaLaunchKernelEx(&cfg, k_pcg<T, false>, P));
+  ACG_CUDA(cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...));
 }
 
-// Resident blocks of k_pcg: at most `want` per SM.
+// The whole PCG of one right-hand side (r, x buffer 0 and the state set up by
+// k_center or k_outer_prep) as one cooperative launch.
+template <typename T>
+void enqueue_persist(cudaStream_t s, const SolverImpl& S, double eps, int init) {
+  PersistArgs<T> P = persist_args<T>(S);
+  P.eps = eps;
+  P.init = init;
+  launch_persist<T>(s, S, S.w_K == S.n ? k_pcg<T, true> : k_pcg<T, false>, P);
+}
+
+// One preconditioner application in the caller's vertex order.
+template <typename T>
+void enqueue_apply(cudaStream_t s, const SolverImpl& S, const PersistArgs<T>& P, const double* rext, double* yext) {
+  k_apply_begin<T><<<kVecBlocks, kVecThreads, 0, s>>>(P, S.perm.p, rext,
+                                                      persist_slots(S.persist_blocks[plan_index<T>()]));
+  ACG_CUDA(cudaGetLastError());
+  launch_persist<T>(s, S, S.w_K == S.n ? k_apply<T, true> : k_apply<T, false>, P, (const int*)S.perm.p, yext);
+}
+
+// Resident blocks of the persistent kernels: at most `want` per SM.
 template <typename T>
 int persist_grid(int sms, int want, int K, bool whole) {
-  int occ = 0;
   const int smem = (int)persist_smem<T>(K);
-  auto kern = whole ? k_pcg<T, true> : k_pcg<T, false>;
-  ACG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)persist_smem<T>(kDenseMaxK)));
-  ACG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, kPersistThreads, smem));
-  return sms * std::max(1, std::min(want, occ));
+  auto fit = [&](auto kern) {
+    int occ = 0;
+    ACG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)persist_smem<T>(kDenseMaxK)));
+    ACG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, kPersistThreads, smem));
+    want = std::min(want, occ);
+  };
+  fit(whole ? k_pcg<T, true> : k_pcg<T, false>);
+  fit(whole ? k_apply<T, true> : k_apply<T, false>);
+  return sms * std::max(1, want);
 }
 
 // ---- graph construction -----------------------------------------------------
@@ -1450,6 +1474,10 @@ template <typename T>
 void ldlsolve_impl(SolverImpl& S, T* rbuf, T* sbuf, T* ybuf) {
   cudaStream_t s = S.stream;
   const int n = S.n;
+  if (S.persist) {
+    enqueue_apply<T>(s, S, persist_args<T>(S), S.b_ext.p, S.x_ext.p);
+    return;
+  }
   reset_state_for_direct_use(S);
   LoopCtl none{0, 0};
   k_gather_in<<<kVecBlocks, kVecThreads, 0, s>>>(n, S.perm.p, S.b_ext.p, S.bm.p, S.st, S.partials.p);
@@ -1476,7 +1504,8 @@ void ldlsolve_impl(SolverImpl& S, T* rbuf, T* sbuf, T* ybuf) {
 // as the process lives.
 constexpr int kNoAllocMaxN = ACG_NOALLOC_MAX_N;
 constexpr size_t kNoAllocVec = (size_t)kNoAllocMaxN * sizeof(double);
-constexpr size_t kNoAllocPartials = (size_t)4 * kMaxPartialBlocks * sizeof(double);
+constexpr size_t kNoAllocPartials = (size_t)4 * kMaxPartialBlocks * sizeof(double) * 4;
+static_assert(kNoAllocPartials >= sizeof(double) * persist_slots(592), "reduction slots of four blocks per SM");
 // a dense tail has at most min(kDenseMaxK, n / 4) vertices
 constexpr int kNoAllocDenseK = kDenseMaxK < kNoAllocMaxN / 4 ? kDenseMaxK : kNoAllocMaxN / 4;
 constexpr size_t kNoAllocDense = (size_t)dense_chunks(kNoAllocDenseK) * kNoAllocDenseK * sizeof(double);
@@ -1516,6 +1545,20 @@ void ldlsolve_noalloc_impl(const SolverImpl& S, cudaStream_t s, const double* r_
   double* partials = reinterpret_cast<double*>(base + kNoAllocVectors);
   T* dense_part = reinterpret_cast<T*>(base + kNoAllocVectors + kNoAllocPartials);
   PcgState* st = reinterpret_cast<PcgState*>(base + kNoAllocState);
+  if (S.persist) {
+    // the same launches as acg_ldlsolve with the scratch in place of the
+    // solver's vectors, one value per slot
+    PersistArgs<T> P = persist_args<T>(S);
+    P.vs = 1;
+    P.r0 = rT;
+    P.s = sv;
+    P.y = yv;
+    P.wt = dense_part;
+    P.red = partials;
+    P.st = st;
+    enqueue_apply<T>(s, S, P, r_ext, y_ext);
+    return;
+  }
   LoopCtl none{0, 0};
   // the state (done flag, sweep error flag, reduction tickets) must start at zero
   ACG_CUDA(cudaMemsetAsync(st, 0, sizeof(PcgState), s));
