@@ -22,6 +22,7 @@
 #include "acg_plan.h"
 #include "acg_batch.cuh"
 #include "acg_dense.cuh"
+#include "acg_gblock.cuh"
 #include "acg_group.cuh"
 #include "acg_persist.cuh"
 #include "acg_serve.cuh"
@@ -181,6 +182,12 @@ struct SolverImpl {
   GroupShared* gsh = nullptr;
   PcgState* h_gstates = nullptr;
   cudaGraphExec_t gexec = nullptr, gexec_mixed = nullptr;
+  // one block per graph (acg_gblock.cuh)
+  bool gblock[2] = {false, false};  // FP64, FP32
+  size_t gblock_smem = 0;
+  DevBuf<GBGraph> gb_graphs;
+  DevBuf<SweepTask> gb_tf, gb_tb;
+  DevBuf<int> gb_of, gb_ob;
 
   // batched solves: kp right-hand sides per launch (vertex-major n x kp blocks)
   int batch_kp = 0;  // capacity of the batch buffers
@@ -771,6 +778,17 @@ namespace {
 constexpr SweepCost kVectorCost{25000.0, 128.0, 0.4, 160, 64};
 constexpr SweepCost kBatchCost{10000.0, 32.0, 0.5, 0, 0};
 
+// Groups: us per iteration of a graph's block (by depth and vertices, and by
+// vertices where p does not fit shared memory), and of the launches all graphs
+// share (by the union's depth and vertices).  Blocks / launches, measured, FP64
+// and FP32, for 24 graphs of up to 1,579 vertices: 128 / 238, 109 / 215; 24 of up
+// to 6,268: 254 / 356, 206 / 336; 300 of up to 7,995: 502 / 816, 335 / 723; 24 of
+// up to 13,910: 544 / 458, 315 / 409; 60 of up to 39,326: 2,088 / 845, 753 / 815.
+struct GroupCost {
+  double block, level, vertex, far_vertex, all_level, all_vertex;
+};
+constexpr GroupCost kGroupCost[2] = {{20.0, 0.5, 0.024, 0.04, 2.0, 0.0003}, {20.0, 0.4, 0.015, 0.03, 1.8, 0.0003}};
+
 template <typename T>
 std::vector<float> to_f32(const std::vector<T>& v) {
   std::vector<float> o(v.size());
@@ -877,6 +895,89 @@ std::vector<double> triangular_inverse(const std::vector<int>& fptr, const std::
   work(0);
   for (auto& t : pool) t.join();
   return m;
+}
+
+// Decides whether the group's graphs run one block each (acg_gblock.cuh), and
+// cuts the union's task tables by graph and warp.  af / ab: tasks up to the end
+// of each run of the plan (a run is one level of one graph).
+void build_gblock(SolverImpl& S, const SweepPlan& plan, const std::vector<std::vector<std::pair<int, int>>>& level_runs,
+                  const std::vector<int>& af, const std::vector<int>& ab, const std::vector<SweepTask>& tf,
+                  const std::vector<SweepTask>& tb) {
+  const int nseg = S.nseg;
+  std::vector<int> depth(nseg, 0), seg_of(S.n);
+  int most = 0;
+  for (int g = 0; g < nseg; ++g) {
+    most = std::max(most, S.seg_off[g + 1] - S.seg_off[g]);
+    for (int v = S.seg_off[g]; v < S.seg_off[g + 1]; ++v) seg_of[v] = g;
+  }
+  if (most > kGBMaxChunks * kChunk) return;
+  for (size_t l = 0; l < level_runs.size(); ++l)
+    for (const auto& r : level_runs[l]) depth[seg_of[r.first]] = (int)l + 1;
+  int sms = 0, optin = 0;
+  ACG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, S.device));
+  ACG_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, S.device));
+  size_t fixed = 0;
+  cudaFuncAttributes fa;
+  ACG_CUDA(cudaFuncGetAttributes(&fa, k_group_pcg<double>));
+  fixed = std::max(fixed, fa.sharedSizeBytes);
+  ACG_CUDA(cudaFuncGetAttributes(&fa, k_group_pcg<float>));
+  fixed = std::max(fixed, fa.sharedSizeBytes);
+  const size_t cap = (size_t)optin - fixed - 1024;
+  for (int w = 0; w < 2; ++w) {
+    const GroupCost& c = kGroupCost[w];
+    const int fit = (int)(cap / (2 * (w == 0 ? sizeof(double) : sizeof(float))));
+    double longest = 0.0, total = 0.0;
+    for (int g = 0; g < nseg; ++g) {
+      const int n = S.seg_off[g + 1] - S.seg_off[g];
+      const double t = c.block + c.level * depth[g] + (n <= fit ? c.vertex : c.far_vertex) * n;
+      longest = std::max(longest, t);
+      total += t;
+    }
+    // the slowest block, or several rounds of blocks with a half-empty last one
+    const double blocks = nseg <= sms ? longest : std::max(longest, total / sms + 0.5 * longest);
+    S.gblock[w] = blocks < c.all_level * (double)level_runs.size() + c.all_vertex * (double)S.n;
+  }
+  if (!S.gblock[0] && !S.gblock[1]) return;
+  auto cut = [&](const SweepRows& R, const std::vector<int>& after, const std::vector<SweepTask>& all,
+                 std::vector<SweepTask>& out, std::vector<int>& off) {
+    std::vector<std::vector<SweepTask>> lists((size_t)nseg * kGBWarpsAll);
+    std::vector<int> next(nseg, 0), step(nseg, 0);
+    for (size_t i = 0; i < R.runs.size(); ++i) {  // a graph's runs come level by level
+      const int g = seg_of[R.runs[i].v0];
+      for (int t = i ? after[i - 1] : 0; t < after[i]; ++t) {
+        SweepTask task = all[t];
+        task.delta = step[g];
+        lists[(size_t)g * kGBWarpsAll + next[g]++ % kGBWarpsAll].push_back(task);
+      }
+      ++step[g];
+    }
+    off.reserve(lists.size() + nseg);
+    for (int g = 0; g < nseg; ++g) {
+      for (int w = 0; w < kGBWarpsAll; ++w) {
+        off.push_back((int)out.size());
+        const auto& list = lists[(size_t)g * kGBWarpsAll + w];
+        out.insert(out.end(), list.begin(), list.end());
+      }
+      off.push_back((int)out.size());
+    }
+  };
+  std::vector<SweepTask> gf, gb;
+  std::vector<int> of, ob;
+  cut(plan.fwd, af, tf, gf, of);
+  cut(plan.bwd, ab, tb, gb, ob);
+  std::vector<GBGraph> graphs(nseg);
+  for (int g = 0; g < nseg; ++g)
+    graphs[g] = {S.seg_off[g], S.seg_off[g + 1] - S.seg_off[g], depth[g], g * (kGBWarpsAll + 1), g * (kGBWarpsAll + 1), g};
+  std::stable_sort(graphs.begin(), graphs.end(), [](const GBGraph& x, const GBGraph& y) { return x.n > y.n; });
+  S.gblock_smem = std::min(cap, (size_t)2 * most * sizeof(double));
+  ACG_CUDA(cudaFuncSetAttribute(k_group_pcg<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cap));
+  ACG_CUDA(cudaFuncSetAttribute(k_group_pcg<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cap));
+  S.gb_graphs.upload(graphs, S.stream);
+  S.gb_tf.upload(gf, S.stream);
+  S.gb_tb.upload(gb, S.stream);
+  S.gb_of.upload(of, S.stream);
+  S.gb_ob.upload(ob, S.stream);
+  ACG_CUDA(cudaStreamSynchronize(S.stream));  // the uploads read this function's arrays
 }
 
 // Builds the device solver for one graph, or for the block-diagonal union of
@@ -1290,6 +1391,7 @@ void build_solver(SolverImpl& S, int64_t n64, const int64_t* a_colptr, const int
           ACG_CUDA(cudaFuncSetAttribute(k_tail<float, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, tb_bytes));
         }
       }
+      if (nseg > 1 && blank <= 0) build_gblock(S, plan, runs, af, ab, tf, tb);
       unproduced(tf);
       P.ntasks_f = (int)tf.size();
       P.tasks_f.upload(tf, S.stream);
@@ -2088,6 +2190,53 @@ GroupArgs group_args(const SolverImpl& S) {
                    S.gsh, S.nseg, S.n, S.sweep[0].nslots};
 }
 
+// Every graph's whole PCG, one block each.
+template <typename T>
+void enqueue_gblock(cudaStream_t s, const SolverImpl& S, double eps, int init) {
+  const TypedArrays<T> A = arrays_of<T>(S);
+  const DevSweep& D = S.sweep[0];
+  GBArgs<T> P = {};
+  P.graphs = S.gb_graphs.p;
+  P.lp = A.lp;
+  P.li = A.li;
+  P.lv = A.lv;
+  P.tf = S.gb_tf.p;
+  P.tb = S.gb_tb.p;
+  P.of = S.gb_of.p;
+  P.ob = S.gb_ob.p;
+  P.fi = D.f_idx.p;
+  P.bi = D.b_idx.p;
+  P.fc = D.coef<T>(true);
+  P.bc = D.coef<T>(false);
+  P.g = A.g;
+  if constexpr (sizeof(T) == 8) {
+    P.r = S.r64.p; P.p = S.p64.p; P.q = S.q64.p; P.x3 = S.x3_64.p; P.y = S.y64.p;
+  } else {
+    P.r = S.r32.p; P.p = S.p32.p; P.q = S.q32.p; P.x3 = S.x3_32.p; P.y = S.y32.p;
+  }
+  P.nall = S.n;
+  P.st = S.gstates;
+  P.eps = eps;
+  P.init = init;
+  P.smem_values = (int)(S.gblock_smem / sizeof(T));
+  k_group_pcg<T><<<S.nseg, kGBThreads, S.gblock_smem, s>>>(P);
+  ACG_CUDA(cudaGetLastError());
+}
+
+cudaGraphExec_t finish_group_graph(SolverImpl& S, cudaGraph_t top, const std::vector<cudaGraphNode_t>& deps) {
+  cudaStream_t s = S.stream;
+  const GroupArgs g = group_args(S);
+  begin_into(s, top, deps);
+  kg_take_best<double><<<S.nchunks, kVecThreads, 0, s>>>(S.n, S.x3_64.p, S.xf.p, g);
+  kg_true_residual<<<S.nchunks, kVecThreads, 0, s>>>(S.l_ptr.p, S.l_idx.p, S.l_v64.p, S.xf.p, S.bm.p, nullptr, g);
+  k_scatter_out<<<kVecBlocks, kVecThreads, 0, s>>>(S.n, S.perm.p, S.xf.p, S.x_ext.p);
+  end_into(s);
+  cudaGraphExec_t exec;
+  ACG_CUDA(cudaGraphInstantiate(&exec, top, 0));
+  cudaGraphDestroy(top);
+  return exec;
+}
+
 cudaGraphExec_t build_group_graph(SolverImpl& S) {
   cudaStream_t s = S.stream;
   const int n = S.n;
@@ -2095,9 +2244,9 @@ cudaGraphExec_t build_group_graph(SolverImpl& S) {
   const GroupArgs g = group_args(S);
   cudaGraph_t top;
   ACG_CUDA(cudaGraphCreate(&top, 0));
-  cudaGraphConditionalHandle h;
-  ACG_CUDA(cudaGraphConditionalHandleCreate(&h, top, 1u, cudaGraphCondAssignDefault));
-  LoopCtl ctl{h, 1};
+  cudaGraphConditionalHandle h{};
+  if (!S.gblock[0]) ACG_CUDA(cudaGraphConditionalHandleCreate(&h, top, 1u, cudaGraphCondAssignDefault));
+  LoopCtl ctl{h, S.gblock[0] ? 0 : 1};
   const TypedArrays<double> A = arrays_of<double>(S);
   begin_into(s, top, {});
   // tickets of graphs that stopped while blocks of the same launch were still
@@ -2105,6 +2254,10 @@ cudaGraphExec_t build_group_graph(SolverImpl& S) {
   ACG_CUDA(cudaMemsetAsync(S.seg_cnt.p, 0, sizeof(unsigned int) * 8 * S.nseg, s));
   kg_gather_in<<<nb, kVecThreads, 0, s>>>(S.perm.p, S.b_ext.p, S.bm.p, g);
   kg_center<double><<<nb, kVecThreads, 0, s>>>(S.bm.p, S.r64.p, S.x3_64.p, S.s64.p, S.y64.p, g, ctl, S.vs64, 0);
+  if (S.gblock[0]) {
+    enqueue_gblock<double>(s, S, kEps64, 1);
+    return finish_group_graph(S, top, capture_end(s));
+  }
   enqueue_sweeps<double>(s, S, S.r64.p, S.s64.p, S.y64.p, S.gflags);
   kg_ysum<double><<<nb, kVecThreads, 0, s>>>(S.y64.p, g, ctl, S.vs64);
   kg_zdot<double><<<nb, kVecThreads, 0, s>>>(S.y64.p, S.r64.p, S.p64.p, g, kEps64, 1, ctl, S.vs64);
@@ -2122,9 +2275,21 @@ cudaGraphExec_t build_group_graph(SolverImpl& S) {
   kg_zdot<double><<<nb, kVecThreads, 0, s>>>(S.y64.p, S.r64.p, S.p64.p, g, kEps64, 0, ctl, S.vs64);
   kg_pupdate<double><<<nb, kVecThreads, 0, s>>>(S.y64.p, S.p64.p, g, S.vs64);
   end_into(s);
-  begin_into(s, top, {wnode});
-  kg_take_best<double><<<nb, kVecThreads, 0, s>>>(n, S.x3_64.p, S.xf.p, g);
-  kg_true_residual<<<nb, kVecThreads, 0, s>>>(S.l_ptr.p, S.l_idx.p, S.l_v64.p, S.xf.p, S.bm.p, nullptr, g);
+  return finish_group_graph(S, top, {wnode});
+}
+
+cudaGraphExec_t finish_group_mixed_graph(SolverImpl& S, cudaGraph_t top, cudaGraph_t obody, cudaGraphNode_t onode,
+                                         LoopCtl octl, const std::vector<cudaGraphNode_t>& deps) {
+  cudaStream_t s = S.stream;
+  const int n = S.n, nb = S.nchunks;
+  const GroupArgs g = group_args(S);
+  begin_into(s, obody, deps);
+  kg_outer_correct<float><<<nb, kVecThreads, 0, s>>>(n, S.x3_32.p, S.xf.p, g);
+  kg_true_residual<<<nb, kVecThreads, 0, s>>>(S.l_ptr.p, S.l_idx.p, S.l_v64.p, S.xf.p, S.bm.p, S.r64.p, g);
+  kg_outer_decide<<<1, 256, 0, s>>>(g, octl);
+  end_into(s);
+
+  begin_into(s, top, {onode});
   k_scatter_out<<<kVecBlocks, kVecThreads, 0, s>>>(n, S.perm.p, S.xf.p, S.x_ext.p);
   end_into(s);
   cudaGraphExec_t exec;
@@ -2158,12 +2323,16 @@ cudaGraphExec_t build_group_mixed_graph(SolverImpl& S) {
 
   cudaGraph_t obody;
   cudaGraphNode_t onode = add_while(top, leaves, ho, &obody);
-  cudaGraphConditionalHandle hi;
-  ACG_CUDA(cudaGraphConditionalHandleCreate(&hi, obody, 1u, cudaGraphCondAssignDefault));
-  LoopCtl ictl{hi, 1};
+  cudaGraphConditionalHandle hi{};
+  if (!S.gblock[1]) ACG_CUDA(cudaGraphConditionalHandleCreate(&hi, obody, 1u, cudaGraphCondAssignDefault));
+  LoopCtl ictl{hi, S.gblock[1] ? 0 : 1};
   begin_into(s, obody, {});
   kg_outer_begin<<<1, 256, 0, s>>>(g, ictl);
   kg_outer_prep<float><<<nb, kVecThreads, 0, s>>>(S.r64.p, S.r32.p, S.x3_32.p, S.s32.p, S.y32.p, g, ictl, S.vs32);
+  if (S.gblock[1]) {
+    enqueue_gblock<float>(s, S, eps32, 2);
+    return finish_group_mixed_graph(S, top, obody, onode, octl, capture_end(s));
+  }
   enqueue_sweeps<float>(s, S, S.r32.p, S.s32.p, S.y32.p, S.gflags);
   kg_ysum<float><<<nb, kVecThreads, 0, s>>>(S.y32.p, g, ictl, S.vs32);
   kg_zdot<float><<<nb, kVecThreads, 0, s>>>(S.y32.p, S.r32.p, S.p32.p, g, eps32, 2, ictl, S.vs32);
@@ -2183,19 +2352,7 @@ cudaGraphExec_t build_group_mixed_graph(SolverImpl& S) {
   kg_pupdate<float><<<nb, kVecThreads, 0, s>>>(S.y32.p, S.p32.p, g, S.vs32);
   end_into(s);
 
-  begin_into(s, obody, {inode});
-  kg_outer_correct<float><<<nb, kVecThreads, 0, s>>>(n, S.x3_32.p, S.xf.p, g);
-  kg_true_residual<<<nb, kVecThreads, 0, s>>>(S.l_ptr.p, S.l_idx.p, S.l_v64.p, S.xf.p, S.bm.p, S.r64.p, g);
-  kg_outer_decide<<<1, 256, 0, s>>>(g, octl);
-  end_into(s);
-
-  begin_into(s, top, {onode});
-  k_scatter_out<<<kVecBlocks, kVecThreads, 0, s>>>(n, S.perm.p, S.xf.p, S.x_ext.p);
-  end_into(s);
-  cudaGraphExec_t exec;
-  ACG_CUDA(cudaGraphInstantiate(&exec, top, 0));
-  cudaGraphDestroy(top);
-  return exec;
+  return finish_group_mixed_graph(S, top, obody, onode, octl, {inode});
 }
 
 int solve_group(SolverImpl& S, const double* b, double* x, cudaMemcpyKind kin, cudaMemcpyKind kout, double tol,
@@ -2984,7 +3141,7 @@ int acg_solver_stats(const acg_solver* h, acg_stats* out) {
   add(S.b_ext); add(S.x_ext); add(S.bm); add(S.r64); add(S.s64); add(S.y64); add(S.p64); add(S.q64); add(S.x3_64);
   add(S.xf); add(S.r32); add(S.s32); add(S.y32); add(S.p32); add(S.q32); add(S.x3_32); add(S.partials);
   bytes += S.sweep[0].bytes() + S.sweep[1].bytes();
-  add(S.W64); add(S.W32); add(S.r64b); add(S.p64b); add(S.r32b); add(S.p32b); add(S.wt64); add(S.wt32); add(S.red);
+  add(S.W64); add(S.W32); add(S.r64b); add(S.p64b); add(S.r32b); add(S.p32b); add(S.wt64); add(S.wt32); add(S.red); add(S.gb_graphs); add(S.gb_tf); add(S.gb_tb); add(S.gb_of); add(S.gb_ob);
   add(S.bb_ext[0]); add(S.bx_ext[0]); add(S.bb_ext[1]); add(S.bx_ext[1]); add(S.bbm); add(S.br64); add(S.bxf); add(S.bpartials); add(S.br32); add(S.bs32);
   add(S.by32); add(S.bp32); add(S.bq32); add(S.bx3_32); add(S.bs64); add(S.by64); add(S.bp64); add(S.bq64);
   add(S.bx3_64);
