@@ -278,7 +278,7 @@ __device__ __forceinline__ T w_row(const T* __restrict__ Wr, const T* w, int ld,
   constexpr int V = 16 / sizeof(T);
   using VT = typename std::conditional<sizeof(T) == 8, double2, float4>::type;
   constexpr int U = 4;
-  T acc = T(0);
+  T acc[U] = {};
   const VT* a = reinterpret_cast<const VT*>(Wr);
   const VT* b = reinterpret_cast<const VT*>(w);
   const int m = ld / V;
@@ -292,17 +292,17 @@ __device__ __forceinline__ T w_row(const T* __restrict__ Wr, const T* w, int ld,
       if (j + 32 * u < m) {
         const VT z = b[j + 32 * u];
         if constexpr (sizeof(T) == 8) {
-          acc += x[u].x * z.x;
-          acc += x[u].y * z.y;
+          acc[u] += x[u].x * z.x;
+          acc[u] += x[u].y * z.y;
         } else {
-          acc += x[u].x * z.x;
-          acc += x[u].y * z.y;
-          acc += x[u].z * z.z;
-          acc += x[u].w * z.w;
+          acc[u] += x[u].x * z.x;
+          acc[u] += x[u].y * z.y;
+          acc[u] += x[u].z * z.z;
+          acc[u] += x[u].w * z.w;
         }
       }
   }
-  return group_sum_w(acc, 32);
+  return group_sum_w((acc[0] + acc[1]) + (acc[2] + acc[3]), 32);
 }
 
 // kWhole: W is the whole preconditioner (K = n): no sweeps, and an iteration is
@@ -592,32 +592,58 @@ __global__ void __launch_bounds__(kPersistThreads, 2) k_apply(const __grid_const
   for (int i = gtid; i < P.n; i += gsize) yext[perm[i]] = (double)P.y[(size_t)i * vs] - mean;
 }
 
-// W = M^T diag(g) M for the dense tail (or the whole graph): M is K x K
-// row-major lower triangular, W's rows are padded with zeros to ldw columns.
+// mean[k] = the mean of row k of M (K x K, row-major, lower triangular), a
+// warp a row.
+__global__ void __launch_bounds__(256) k_row_mean(int K, const double* __restrict__ M, double* __restrict__ mean) {
+  const int lane = threadIdx.x & 31, k = blockIdx.x * 8 + (threadIdx.x >> 5);
+  if (k >= K) return;
+  double sum = 0.0;
+  for (int i = lane; i <= k; i += 32) sum += M[(size_t)k * K + i];
+  sum = group_sum_w(sum, 32);
+  if (lane == 0) mean[k] = sum / K;
+}
+
+// W = (M - mean 1^T)^T diag(g) M for the dense tail (or the whole graph): M is
+// K x K row-major lower triangular, W's rows are padded with zeros to ldw
+// columns.  M^T diag(g) M is the operator; a constant in a column of W only
+// shifts all of y, which the mean removal takes out again, and the rows of M
+// near the root are nearly constant (all flows to the root, whose own row is
+// all ones and is left out).  With these constants in W its entries are far
+// larger than what they say of y, and the rounding of each row's sum shows:
+// on matchings of 60,000 vertices with lognormal weights one application was
+// 4.6e-14 from 64 bits without the means and the root taken out, 6e-16 with
+// the two triangular products.  The sums over k carry their rounding errors
+// along (two-sum and a product split by fma), since W is used many times.
 // 64 x 64 tiles, 4 x 4 entries a thread, FP64.  Run once per solver.
 constexpr int kWTile = 64;
 __global__ void __launch_bounds__(256) k_form_w(int K, int ldw, const double* __restrict__ M,
-                                                const double* __restrict__ g, double* __restrict__ W64,
-                                                float* __restrict__ W32) {
+                                                const double* __restrict__ mean, const double* __restrict__ g,
+                                                double* __restrict__ W64, float* __restrict__ W32) {
   __shared__ double A[16][kWTile + 1], B[16][kWTile + 1];
   const int i0 = blockIdx.y * kWTile, j0 = blockIdx.x * kWTile;
   const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-  double acc[4][4] = {};
-  // column i of M has entries in rows k >= i only
-  for (int k0 = (max(i0, j0) / 16) * 16; k0 < K; k0 += 16) {
+  double acc[4][4] = {}, low[4][4] = {};
+  const int rows = K - 1;  // without the root
+  // column j of M has entries in rows k >= j only
+  for (int k0 = (j0 / 16) * 16; k0 < rows; k0 += 16) {
     for (int e = threadIdx.x; e < 16 * kWTile; e += 256) {
       const int kk = e / kWTile, c = e % kWTile, k = k0 + kk;
-      const bool in = k < K;
-      A[kk][c] = in && i0 + c <= k ? M[(size_t)k * K + i0 + c] * g[k] : 0.0;
+      const bool in = k < rows;
+      A[kk][c] = in ? ((i0 + c <= k ? M[(size_t)k * K + i0 + c] : 0.0) - mean[k]) * g[k] : 0.0;
       B[kk][c] = in && j0 + c <= k ? M[(size_t)k * K + j0 + c] : 0.0;
     }
     __syncthreads();
-#pragma unroll
+#pragma unroll 4
     for (int kk = 0; kk < 16; ++kk)
 #pragma unroll
       for (int a = 0; a < 4; ++a)
 #pragma unroll
-        for (int b = 0; b < 4; ++b) acc[a][b] += A[kk][ty * 4 + a] * B[kk][tx * 4 + b];
+        for (int b = 0; b < 4; ++b) {
+          const double x = A[kk][ty * 4 + a], z = B[kk][tx * 4 + b], prod = x * z, old = acc[a][b];
+          const double sum = old + prod, t = sum - old;
+          low[a][b] += ((old - (sum - t)) + (prod - t)) + fma(x, z, -prod);
+          acc[a][b] = sum;
+        }
     __syncthreads();
   }
 #pragma unroll
@@ -626,7 +652,7 @@ __global__ void __launch_bounds__(256) k_form_w(int K, int ldw, const double* __
     for (int b = 0; b < 4; ++b) {
       const int i = i0 + ty * 4 + a, j = j0 + tx * 4 + b;
       if (i < K && j < ldw) {
-        const double v = j < K ? acc[a][b] : 0.0;
+        const double v = j < K ? acc[a][b] + low[a][b] : 0.0;
         W64[(size_t)i * ldw + j] = v;
         W32[(size_t)i * ldw + j] = (float)v;
       }

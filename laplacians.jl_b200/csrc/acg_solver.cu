@@ -1483,15 +1483,20 @@ void build_solver(SolverImpl& S, int64_t n64, const int64_t* a_colptr, const int
     S.w_v0 = w_whole ? 0 : S.dt_v0;
     if (S.w_K) {
       const int K = S.w_K, ldw = w_stride(K);
-      DevBuf<double> m;
+      DevBuf<double> m, mean;
       if (w_whole) m.upload(whole_m, s);
       S.W64.alloc((size_t)K * ldw);
       S.W32.alloc((size_t)K * ldw);
-      k_form_w<<<dim3(ldw / kWTile, (K + kWTile - 1) / kWTile), 256, 0, s>>>(
-          K, ldw, w_whole ? m.p : S.dt_M64.p, S.g64.p + S.w_v0, S.W64.p, S.W32.p);
+      mean.alloc(K);
+      const double* mp = w_whole ? m.p : S.dt_M64.p;
+      k_row_mean<<<(K + 7) / 8, 256, 0, s>>>(K, mp, mean.p);
+      ACG_CUDA(cudaGetLastError());
+      k_form_w<<<dim3(ldw / kWTile, (K + kWTile - 1) / kWTile), 256, 0, s>>>(K, ldw, mp, mean.p, S.g64.p + S.w_v0,
+                                                                             S.W64.p, S.W32.p);
       ACG_CUDA(cudaGetLastError());
       ACG_CUDA(cudaStreamSynchronize(s));
       m.free();
+      mean.free();
     }
     int sms = 0;
     ACG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, S.device));
