@@ -24,7 +24,7 @@ OUT = PKG / "acgpu" / "libacgpu.so"
 HOST_OUT = PKG / "acgpu" / "libacghost.so"
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 
-CU_SOURCES = ["acg_solver.cu"]
+CU_SOURCES = ["acg_solver.cu", "acg_persist.cu"]
 CPP_SOURCES = ["acg_rng.cpp", "acg_factor.cpp", "acg_factor_par.cpp", "acg_host_api.cpp", "acg_plan.cpp"]
 GENCODE = ["-gencode", "arch=compute_100a,code=sm_100a"]
 

@@ -261,7 +261,7 @@ __global__ void __launch_bounds__(kVecThreads) k_pupdate(int n, const T* __restr
 // ---- set-up and wrap-up kernels (FP64) ------------------------------------
 
 // b_int[i] = b_ext[perm[i]]; mean(b) -> st->mean.
-__global__ void __launch_bounds__(kVecThreads) k_gather_in(int n, const int* __restrict__ perm, const double* __restrict__ bext,
+static __global__ void __launch_bounds__(kVecThreads) k_gather_in(int n, const int* __restrict__ perm, const double* __restrict__ bext,
                                                            double* __restrict__ bint, PcgState* st, double* partials) {
   double acc[1] = {0.0};
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
@@ -356,7 +356,7 @@ __global__ void __launch_bounds__(kVecThreads) k_true_residual(int n, const int*
 }
 
 // x_ext[perm[i]] = xf[i]
-__global__ void __launch_bounds__(kVecThreads) k_scatter_out(int n, const int* __restrict__ perm, const double* __restrict__ xf,
+static __global__ void __launch_bounds__(kVecThreads) k_scatter_out(int n, const int* __restrict__ perm, const double* __restrict__ xf,
                                                              double* __restrict__ xext) {
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) xext[perm[i]] = xf[i];
 }
@@ -412,7 +412,7 @@ __global__ void __launch_bounds__(kVecThreads) k_outer_correct(int n, const T* _
 
 // After the true residual: account iterations, decide whether to refine again,
 // and give the next inner solve its tolerance and remaining iteration budget.
-__global__ void k_outer_decide(PcgState* st, LoopCtl outer_ctl) {
+static __global__ void k_outer_decide(PcgState* st, LoopCtl outer_ctl) {
   if (threadIdx.x != 0 || blockIdx.x != 0) return;
   st->total_its += st->itcnt;
   st->outer_its += 1;

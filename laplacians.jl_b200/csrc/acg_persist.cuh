@@ -7,9 +7,8 @@
 //
 //   update    x' = x + alpha p, r' = r - alpha q, |r'|^2, ...       -> reduce
 //   forward   the sweep plan's forward tasks (values are their own ready flags)
-//   tail      y_T = W w_T, W = M^T diag(g_T) M: the dense tail's two triangular
-//             products as one symmetric matrix (formed once in FP64; all its
-//             terms are non-negative, so nothing cancels)
+//   tail      y_T = W w_T, W = M^T diag(g_T) M up to a constant per column: the
+//             dense tail's two triangular products as one matrix (k_form_w)
 //   backward  the backward tasks; also sum y and y.r                -> reduce
 //   p         p' = (y - mean) + beta p                              -> reduce
 //   mat-vec   q = L p', p'.q                                        -> reduce
@@ -592,9 +591,21 @@ __global__ void __launch_bounds__(kPersistThreads, 2) k_apply(const __grid_const
   for (int i = gtid; i < P.n; i += gsize) yext[perm[i]] = (double)P.y[(size_t)i * vs] - mean;
 }
 
+// The one-vector kernels are compiled in acg_persist.cu alone.
+#define ACG_PERSIST_KERNELS(INST)                                                                                 \
+  INST __global__ void k_pcg<double, true>(const __grid_constant__ PersistArgs<double>);                          \
+  INST __global__ void k_pcg<double, false>(const __grid_constant__ PersistArgs<double>);                         \
+  INST __global__ void k_pcg<float, true>(const __grid_constant__ PersistArgs<float>);                            \
+  INST __global__ void k_pcg<float, false>(const __grid_constant__ PersistArgs<float>);                           \
+  INST __global__ void k_apply<double, true>(const __grid_constant__ PersistArgs<double>, const int*, double*);   \
+  INST __global__ void k_apply<double, false>(const __grid_constant__ PersistArgs<double>, const int*, double*);  \
+  INST __global__ void k_apply<float, true>(const __grid_constant__ PersistArgs<float>, const int*, double*);     \
+  INST __global__ void k_apply<float, false>(const __grid_constant__ PersistArgs<float>, const int*, double*);
+ACG_PERSIST_KERNELS(extern template)
+
 // mean[k] = the mean of row k of M (K x K, row-major, lower triangular), a
 // warp a row.
-__global__ void __launch_bounds__(256) k_row_mean(int K, const double* __restrict__ M, double* __restrict__ mean) {
+static __global__ void __launch_bounds__(256) k_row_mean(int K, const double* __restrict__ M, double* __restrict__ mean) {
   const int lane = threadIdx.x & 31, k = blockIdx.x * 8 + (threadIdx.x >> 5);
   if (k >= K) return;
   double sum = 0.0;
@@ -616,7 +627,7 @@ __global__ void __launch_bounds__(256) k_row_mean(int K, const double* __restric
 // along (two-sum and a product split by fma), since W is used many times.
 // 64 x 64 tiles, 4 x 4 entries a thread, FP64.  Run once per solver.
 constexpr int kWTile = 64;
-__global__ void __launch_bounds__(256) k_form_w(int K, int ldw, const double* __restrict__ M,
+static __global__ void __launch_bounds__(256) k_form_w(int K, int ldw, const double* __restrict__ M,
                                                 const double* __restrict__ mean, const double* __restrict__ g,
                                                 double* __restrict__ W64, float* __restrict__ W32) {
   __shared__ double A[16][kWTile + 1], B[16][kWTile + 1];
