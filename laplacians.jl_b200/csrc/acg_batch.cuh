@@ -580,65 +580,88 @@ __device__ __forceinline__ void sum_rows(const double* src, size_t qstride, int 
   }
 }
 
-// Sums, per column, the rows [0, rows) of NV tables of kp columns into `out`
-// of the threads below kp: the block's threads split the rows into
-// blockDim / kp contiguous parts, and the parts are added in order.
-template <int NV, int kTile>
-__device__ __forceinline__ void block_sum_rows(const double* src, size_t qstride, int kp, int rows,
-                                               double (&sm)[NV][kVecThreads * kTile], double (&out)[NV]) {
-  const int per = (int)blockDim.x / kp;
-  const int c = threadIdx.x % kp, part = threadIdx.x / kp;
-  double s[NV];
-  sum_rows<NV>(src, qstride, kp, c, (int)((long long)rows * part / per), (int)((long long)rows * (part + 1) / per), s);
+// Sums over the block, per column, of NV values when each thread holds VPT
+// consecutive columns (v[q][j] for column (VPT * threadIdx.x + j) mod kp): the
+// lanes of a warp with the same columns by shuffles, then the warps' rows in
+// order through shared memory.  Threads below kp get column threadIdx.x.  (All
+// threads' values through shared memory left kp threads with 256 * VPT / kp
+// dependent additions: 128 for 8 FP32 columns.)
+constexpr int kRedWarps = kVecThreads / 32;
+template <int NV, int VPT>
+__device__ __forceinline__ void block_columns(double (&v)[NV][VPT], int kp, double (&sm)[NV][kRedWarps * kMaxBatch],
+                                              double (&out)[NV]) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int cw = min(32 * VPT, kp);  // columns of a warp; a power of two, as kp and VPT are
+  for (int o = 16; o * VPT >= cw; o >>= 1)
 #pragma unroll
-  for (int q = 0; q < NV; ++q) sm[q][threadIdx.x] = s[q];
+    for (int q = 0; q < NV; ++q)
+#pragma unroll
+      for (int j = 0; j < VPT; ++j) v[q][j] += __shfl_xor_sync(0xffffffffu, v[q][j], o);
+  if (lane * VPT < cw) {
+#pragma unroll
+    for (int q = 0; q < NV; ++q)
+#pragma unroll
+      for (int j = 0; j < VPT; ++j) sm[q][w * cw + lane * VPT + j] = v[q][j];
+  }
   __syncthreads();
   if ((int)threadIdx.x < kp) {
 #pragma unroll
     for (int q = 0; q < NV; ++q) {
       double t = 0.0;
-      for (int j = 0; j < per; ++j) t += sm[q][threadIdx.x + j * kp];
+      for (int e = threadIdx.x; e < kRedWarps * cw; e += kp) t += sm[q][e];
       out[q] = t;
     }
   }
+  __syncthreads();
 }
 
-// The same reduction when each thread holds VPT consecutive columns
-// (v[q][j] for column (VPT * threadIdx.x + j) mod kp; blockDim * VPT and the
-// grid stride are multiples of kp), in two levels: the block's values are laid
-// out as VPT * blockDim virtual threads in shared memory and summed per column
-// into one row of partials per block; the last block to finish in each of up
-// to kRedGroups contiguous groups of blocks sums its group's rows into a group
-// row, and the last group to finish sums the group rows.  One block alone
-// would read every block's row (592 x NV x kp values) with a few loads in
-// flight per thread, tens of dependent L2 round trips; two levels take a
-// handful.  The order of every sum is fixed by the grid, so results repeat
-// bit for bit.  Threads below kp of the returning block get the totals of
-// column threadIdx.x in out.  partials holds NV * (gridDim + kRedGroups) * kp
-// values.
+// Sums, per column, the rows [0, rows) of NV tables of kp columns into `out`
+// of the threads below kp: the block's threads split the rows into
+// blockDim / kp contiguous parts.
+template <int NV>
+__device__ __forceinline__ void block_sum_rows(const double* src, size_t qstride, int kp, int rows,
+                                               double (&sm)[NV][kRedWarps * kMaxBatch], double (&out)[NV]) {
+  const int per = (int)blockDim.x / kp;
+  const int c = threadIdx.x % kp, part = threadIdx.x / kp;
+  double s[NV], v[NV][1];
+  sum_rows<NV>(src, qstride, kp, c, (int)((long long)rows * part / per), (int)((long long)rows * (part + 1) / per), s);
+#pragma unroll
+  for (int q = 0; q < NV; ++q) v[q][0] = s[q];
+  block_columns<NV, 1>(v, kp, sm, out);
+}
+
+// The reduction over the grid of what block_columns sums over a block, in up to
+// two levels: each block writes one row of partials; the last block to finish
+// in each of up to kRedGroups contiguous groups of blocks sums its group's rows
+// into a group row, and the last group to finish sums the group rows.  One
+// block alone would read every block's row (592 x NV x kp values) with a few
+// loads in flight per thread, tens of dependent L2 round trips; two levels take
+// a handful.  Where the last block's threads read at most kRedRows rows each
+// there is one level: two tickets and a row's way through L2 less. (us per
+// iteration with all values through shared memory and always two levels, and
+// now: 5 columns of a
+// 20,000-vertex matching graph 115.2 and 112.0, 64 mixed columns of 10^6 vertices
+// 2,525 and 2,508.)  The order
+// of every sum is fixed by the grid, so results repeat bit for bit.  Threads
+// below kp of the returning block get the totals of column threadIdx.x in out.
+// partials holds NV * (gridDim + kRedGroups) * kp values.
+constexpr int kRedRows = 8;
 template <int NV, int VPT>
 __device__ __forceinline__ bool batch_reduce_v(double (&v)[NV][VPT], int kp, double* partials, BatchShared* bs,
                                                int ci, double (&out)[NV]) {
-  constexpr int kTile = VPT > 4 ? VPT : 4;
-  __shared__ double sm[NV][kVecThreads * kTile];
+  __shared__ double sm[NV][kRedWarps * kMaxBatch];
   __shared__ bool am_last;
-#pragma unroll
-  for (int q = 0; q < NV; ++q)
-#pragma unroll
-    for (int j = 0; j < VPT; ++j) sm[q][threadIdx.x * VPT + j] = v[q][j];
-  __syncthreads();
   const int G = gridDim.x;
-  const int gs = (G + kRedGroups - 1) / kRedGroups;  // blocks per group
-  const int NG = (G + gs - 1) / gs;                   // groups
+  const int gs = G * kp <= kRedRows * kVecThreads ? G : (G + kRedGroups - 1) / kRedGroups;  // blocks per group
+  const int NG = (G + gs - 1) / gs;                                                         // groups
   const int g = blockIdx.x / gs, gb0 = g * gs, gb1 = min(G, gb0 + gs);
-  double* grows = partials + (size_t)NV * G * kp;     // group rows: [q][NG][kp]
-  const int per_v = (int)blockDim.x * VPT / kp;
-  if ((int)threadIdx.x < kp) {
+  double* grows = partials + (size_t)NV * G * kp;  // group rows: [q][NG][kp]
+  {
+    double t[NV];
+    block_columns<NV, VPT>(v, kp, sm, t);
+    if ((int)threadIdx.x < kp) {
 #pragma unroll
-    for (int q = 0; q < NV; ++q) {
-      double s = 0.0;
-      for (int j = 0; j < per_v; ++j) s += sm[q][threadIdx.x + j * kp];
-      partials[((size_t)q * G + blockIdx.x) * kp + threadIdx.x] = s;
+      for (int q = 0; q < NV; ++q) partials[((size_t)q * G + blockIdx.x) * kp + threadIdx.x] = t[q];
     }
   }
   __syncthreads();
@@ -652,7 +675,13 @@ __device__ __forceinline__ bool batch_reduce_v(double (&v)[NV][VPT], int kp, dou
   // the group's last block: its rows into the group row
   {
     double t[NV];
-    block_sum_rows<NV, kTile>(partials + (size_t)gb0 * kp, (size_t)G * kp, kp, gb1 - gb0, sm, t);
+    block_sum_rows<NV>(partials + (size_t)gb0 * kp, (size_t)G * kp, kp, gb1 - gb0, sm, t);
+    if (NG == 1) {
+#pragma unroll
+      for (int q = 0; q < NV; ++q) out[q] = t[q];
+      if (threadIdx.x == 0) bs->gcounter[ci][0] = 0u;
+      return true;
+    }
     if ((int)threadIdx.x < kp) {
 #pragma unroll
       for (int q = 0; q < NV; ++q) grows[((size_t)q * NG + g) * kp + threadIdx.x] = t[q];
@@ -667,7 +696,7 @@ __device__ __forceinline__ bool batch_reduce_v(double (&v)[NV][VPT], int kp, dou
   __syncthreads();
   if (!am_last) return false;
   __threadfence();
-  block_sum_rows<NV, kTile>(grows, (size_t)NG * kp, kp, NG, sm, out);
+  block_sum_rows<NV>(grows, (size_t)NG * kp, kp, NG, sm, out);
   if (threadIdx.x == 0) bs->counter[ci] = 0u;
   return true;
 }
