@@ -60,7 +60,7 @@ def build(force: bool = False, verbose: bool = False) -> Path:
     os.replace(host_tmp, HOST_OUT)
     for src in CU_SOURCES:
         obj = objdir / (src + ".o")
-        cmd = [NVCC, *common, *GENCODE, "-lineinfo", "-c", str(CSRC / src), "-o", str(obj)]
+        cmd = [NVCC, *common, *GENCODE, "-static-global-template-stub=false", "-lineinfo", "-c", str(CSRC / src), "-o", str(obj)]
         if verbose:
             cmd += ["-Xptxas", "-v", "-Wno-deprecated-gpu-targets"]
         _run(cmd, verbose)
