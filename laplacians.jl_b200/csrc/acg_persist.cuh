@@ -21,7 +21,10 @@
 // release (fence, then the slots), collecting an acquire (slots, then fence), so
 // a reduction is also a grid barrier for the vectors written before it.  A block
 // resets its slots once it has the totals; block 0 resets the totals of one
-// reduction when every block has published the next.
+// reduction when every block has published the next, before the fence with which
+// it publishes that one's totals.  So a block that has the totals of one
+// reduction finds those of the reduction before it pending or new, never old:
+// with two reductions an iteration (kWhole) these are the next that it polls.
 //
 // Graphs of up to kDenseWhole vertices have W for the whole graph (k_pcg's
 // kWhole): no sweeps and two reductions an iteration.
@@ -146,9 +149,10 @@ __device__ __forceinline__ void red_collect(double* red, int point, int last, do
     }
     __syncthreads();
     // every block has published `point`, so has the totals of `last`
-    if (wid == 0 && lane < kRedValues) {
-      fence_gpu();
-      st_relaxed(red + last * kRedValues + lane, pending_value<double>());
+    if (wid == 0) {
+      if (lane < kRedValues) st_relaxed(red + last * kRedValues + lane, pending_value<double>());
+      __syncwarp();
+      fence_gpu();  // the reset before the totals, for every lane's slot
       if (lane < NV) st_relaxed(red + point * kRedValues + lane, smem[lane]);
     }
   } else {
