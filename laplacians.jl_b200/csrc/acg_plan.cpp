@@ -128,13 +128,17 @@ void partition(Shared& s, int la, int lb, std::vector<Block>& out) {
 }
 
 // The vertex ranges of levels [l0, l1), one per graph (a graph's vertices are
-// numbered level by level, so consecutive levels join up).
+// numbered level by level, so consecutive levels join up; blocks of several
+// levels are made for one graph alone).  Ranges of one level are different
+// graphs' and stay apart: next to a graph of one level lies the next graph's
+// first, and a group's task tables are cut by graph.
 std::vector<std::pair<int, int>> ranges(const SweepDag& d, int l0, int l1) {
   std::vector<std::pair<int, int>> out;
   for (int l = l0; l < l1; ++l)
     for (const auto& r : (*d.level_runs)[l])
       if (r.second > r.first) out.push_back(r);
   std::sort(out.begin(), out.end());
+  if (l1 - l0 == 1) return out;
   size_t w = 0;
   for (size_t i = 0; i < out.size(); ++i) {
     if (w && out[w - 1].second == out[i].first)

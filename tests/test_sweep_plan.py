@@ -1,0 +1,94 @@
+"""The sweep plan (csrc/acg_plan.h) on the host, without a GPU.
+
+plan_check.cpp is compiled with the plan's source into a temporary library; the
+plans are built for factors of the host elimination and for DAGs made here, and
+their rows are walked in plain numpy.
+"""
+import ctypes
+import pathlib
+import subprocess
+import sys
+
+import numpy as np
+import pytest
+
+import acgpu
+from acgpu import generators as G
+
+HERE = pathlib.Path(__file__).parent
+CSRC = HERE.parent / "laplacians.jl_b200" / "csrc"
+VECTOR = (25000.0, 128.0, 0.4, 160, 64)
+BATCH = (10000.0, 32.0, 0.5, 0, 0)
+PART = 3  # kRowPart
+
+
+@pytest.fixture(scope="session")
+def lib_path(tmp_path_factory):
+    out = tmp_path_factory.mktemp("plan") / "plan_check.so"
+    subprocess.run(["g++", "-O2", "-std=c++17", "-ffp-contract=off", "-shared", "-fPIC", "-Wl,-Bsymbolic", "-I", CSRC,
+                    HERE / "plan_check.cpp", CSRC / "acg_plan.cpp", "-o", out, "-lpthread"], check=True)
+    return out
+
+
+class Dag:
+    """CSR of the in-edges (ascending) and of the column entries (descending);
+    `levels`: per level one vertex range per graph."""
+
+    def __init__(self, n, levels, dst, src, val, tail=None):
+        self.n, self.levels = n, levels
+        self.tail = len(levels) if tail is None else tail
+        o = np.lexsort((src, dst))
+        self.fptr = np.concatenate([[0], np.cumsum(np.bincount(dst, minlength=n))]).astype(np.int32)
+        self.fidx, self.fc = src[o].astype(np.int32), val[o].astype(np.float64)
+        o = np.lexsort((-dst, src))
+        self.bptr = np.concatenate([[0], np.cumsum(np.bincount(src, minlength=n))]).astype(np.int32)
+        self.bidx, self.bc = dst[o].astype(np.int32), val[o].astype(np.float64)
+
+    def build(self, path, cost, merge=True, fail=False):
+        lib = ctypes.CDLL(str(path))
+        lib.pc_build.restype = ctypes.c_void_p
+        runs = np.array([(i, a, b) for i, lv in enumerate(self.levels) for a, b in lv], np.int32)
+
+        def c(a):
+            return ctypes.c_void_p(a.ctypes.data)
+
+        cst = np.array(cost, np.float64)
+        h = lib.pc_build(self.n, len(self.levels), len(runs), c(runs), c(self.fptr), c(self.fidx), c(self.fc),
+                         c(self.bptr), c(self.bidx), c(self.bc), self.tail, c(cst), int(merge), int(fail))
+        if not h:
+            return None
+        h = ctypes.c_void_p(h)
+        dims = np.zeros(8, np.int64)
+        lib.pc_dims(h, c(dims))
+        out = {"slots": int(dims[0]), "blocks": int(dims[1])}
+        for d, name in enumerate(("fwd", "bwd")):
+            nr, rows, nnz = (int(v) for v in dims[2 + 3 * d:5 + 3 * d])
+            r, p, i, v = (np.empty((nr, 5), np.int32), np.empty(rows + 1, np.int32), np.empty(nnz, np.int32),
+                          np.empty(nnz, np.float64))
+            lib.pc_rows(h, d, c(r), c(p), c(i), c(v))
+            out[name] = (r, p, i, v)
+        lib.pc_free(h)
+        return out
+
+
+def layers(nlev, width, seed=0, fan=3):
+    """nlev levels of `width` vertices, each with `fan` inputs one level down."""
+    rng = np.random.default_rng(seed)
+    n = nlev * width
+    dst = np.repeat(np.arange(width, n), fan)
+    src = (dst // width - 1) * width + rng.integers(0, width, dst.shape[0])
+    pair = np.unique(np.stack([dst, src]), axis=1)
+    return Dag(n, [[(i * width, (i + 1) * width)] for i in range(nlev)], pair[0], pair[1],
+               rng.uniform(0.1, 0.3, pair.shape[1]))
+
+
+def test_a_run_of_rows_belongs_to_one_graph(lib_path):
+    """A group's task tables are cut by graph, so no run may hold rows of two: a
+    graph without factor entries (one level) lies next to the first level of the
+    one after it."""
+    # graph 0: vertices 0 and 1, no entries; graph 1: vertices 2 and 3, then 4
+    dag = Dag(5, [[(0, 2), (2, 4)], [(4, 5)]], np.array([4, 4]), np.array([2, 3]), np.array([0.5, 0.5]))
+    plan = dag.build(lib_path, VECTOR, merge=False)
+    for name in ("fwd", "bwd"):
+        for v0, count, *_ in plan[name][0]:
+            assert (v0 < 2) == (v0 + count - 1 < 2)
