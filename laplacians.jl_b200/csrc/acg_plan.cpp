@@ -2,7 +2,8 @@
 
 #include <algorithm>
 #include <cmath>
-#include <thread>
+
+#include "acg_threads.h"
 
 namespace acg {
 namespace {
@@ -234,11 +235,7 @@ SweepPlan build_sweep_plan(const SweepDag& d, const SweepCost& cost, bool merge)
     }
     cut.push_back(head);
     std::vector<std::vector<Block>> parts(cut.size() - 1);
-    std::vector<std::thread> pool;
-    for (size_t i = 1; i < parts.size(); ++i)
-      pool.emplace_back([&, i]() { partition(s, cut[i], cut[i + 1], parts[i]); });
-    partition(s, cut[0], cut[1], parts[0]);
-    for (auto& t : pool) t.join();
+    run_threads((int)parts.size(), [&](int i) { partition(s, cut[i], cut[i + 1], parts[i]); });
     size_t held = 0;
     for (auto& p : parts)
       for (auto& b : p) {

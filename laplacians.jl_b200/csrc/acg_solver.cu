@@ -20,6 +20,7 @@
 #include "../../include/acgpu.h"
 #include "acg_internal.h"
 #include "acg_plan.h"
+#include "acg_threads.h"
 #include "acg_batch.cuh"
 #include "acg_dense.cuh"
 #include "acg_gblock.cuh"
@@ -890,10 +891,7 @@ std::vector<double> triangular_inverse(const std::vector<int>& fptr, const std::
       }
     }
   };
-  std::vector<std::thread> pool;
-  for (int t = 1; t < nthreads; ++t) pool.emplace_back(work, t);
-  work(0);
-  for (auto& t : pool) t.join();
+  run_threads(nthreads, work);
   return m;
 }
 

@@ -92,3 +92,15 @@ def test_a_run_of_rows_belongs_to_one_graph(lib_path):
     for name in ("fwd", "bwd"):
         for v0, count, *_ in plan[name][0]:
             assert (v0 < 2) == (v0 + count - 1 < 2)
+
+
+def test_an_allocation_that_fails_on_a_thread_is_an_exception(lib_path):
+    """The plan of a DAG large enough for several threads, with allocations off the
+    calling thread failing: the caller gets std::bad_alloc (the C entries' error
+    code) and the process goes on.  In a process of its own, which an unhandled
+    exception would end."""
+    code = (f"import sys; sys.path[:0] = {sys.path!r}; import test_sweep_plan as t; "
+            f"d = t.layers(20, 15000); assert d.build({str(lib_path)!r}, t.VECTOR, fail=True) is None; "
+            f"assert d.build({str(lib_path)!r}, t.VECTOR)['blocks'] > 0; print('went on')")
+    res = subprocess.run([sys.executable, "-c", code], cwd=HERE, capture_output=True, text=True, timeout=300)
+    assert res.returncode == 0 and "went on" in res.stdout, res.stderr[-2000:]
