@@ -1,7 +1,9 @@
 #include "acg_plan.h"
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
+#include <limits>
 
 #include "acg_threads.h"
 
@@ -28,11 +30,13 @@ struct Shared {
   std::vector<int> where;  // a vertex's row in the block being grown
   std::vector<double> acc;
   std::vector<double> level_cost;  // rows and entries of a level, both directions averaged
+  std::atomic<size_t> held{0};     // entries of the blocks made so far, on all threads
 };
 
 // Greedy blocks over the levels [la, lb): from each level on, the length with
-// the largest saving in hand-overs.
-void partition(Shared& s, int la, int lb, std::vector<Block>& out) {
+// the largest saving in hand-overs.  Gives up once all threads' blocks hold more
+// than `limit` entries.
+void partition(Shared& s, int la, int lb, size_t limit, std::vector<Block>& out) {
   const SweepDag& d = s.d;
   const auto& runs = *d.level_runs;
   const double A = s.cost->entries_per_hop;
@@ -125,6 +129,8 @@ void partition(Shared& s, int la, int lb, std::vector<Block>& out) {
     }
     out.push_back(std::move(b));
     l = out.back().l1;
+    const size_t size = out.back().idx.size();
+    if (s.held.fetch_add(size, std::memory_order_relaxed) + size > limit) return;
   }
 }
 
@@ -202,9 +208,20 @@ int split_rows(SweepRows& R, int split, int part, int base) {
 
 }  // namespace
 
+size_t sweep_fill_limit(const SweepCost& cost, int n, size_t factor_entries) {
+  // A direction has at most E = factor + M_B entries, and rows of more than
+  // `split` entries add E / part + E / split parts, each an entry and a slot.
+  const size_t most = std::numeric_limits<int>::max();
+  const size_t per = cost.split ? (size_t)std::min(cost.part, cost.split) / 2 : most;
+  const size_t entries = most - most / (per + 1);  // E + E / per <= most
+  if (factor_entries >= entries || 2 * (size_t)n + entries / per > most) return 0;
+  const size_t want = std::max((size_t)(cost.fill * (double)factor_entries), cost.fill_min);
+  return std::min(want, entries - factor_entries);
+}
+
 SweepPlan build_sweep_plan(const SweepDag& d, const SweepCost& cost, bool merge) {
   Shared s{d, &cost, std::vector<int>(d.n, 0), std::vector<int>(d.n, -1), std::vector<int>(d.n, 0),
-           std::vector<double>(d.n, 0.0), std::vector<double>(d.nlev, 0.0)};
+           std::vector<double>(d.n, 0.0), std::vector<double>(d.nlev, 0.0), {}};
   const auto& runs = *d.level_runs;
   const int head = std::min(d.tail_level, d.nlev);
   for (int l = 0; l < d.nlev; ++l)
@@ -216,14 +233,17 @@ SweepPlan build_sweep_plan(const SweepDag& d, const SweepCost& cost, bool merge)
   // Blocks: stretches of levels of about equal cost are partitioned by their
   // own thread (the stretches depend on the graph alone).
   std::vector<Block> blocks;
-  // A DAG that fills in fast is merged less: the rows of M_B may hold at most
-  // six times the factor's entries (or 32M), else the blocks are cut again with
-  // dearer entries.
-  const size_t most = std::max((size_t)6 * d.fidx->size(), (size_t)32 << 20);
+  // A DAG that fills in fast is merged less: while the blocks hold more than the
+  // limit, they are cut again with dearer entries.  (Whether they do depends on
+  // the graph alone: the threads' total only grows.)
+  const size_t limit = sweep_fill_limit(cost, d.n, std::max(d.fidx->size(), d.bidx->size()));
+  if (limit == 0) merge = false;
   SweepCost c = cost;
   s.cost = &c;
-  for (int round = 0; merge && round < 6; ++round, c.entries_per_hop *= 0.25) {
+  for (int round = 0; merge; ++round, c.entries_per_hop *= 0.25) {
     blocks.clear();
+    s.held = 0;
+    std::fill(s.mark.begin(), s.mark.end(), -1);
     double total = 0.0;
     for (int l = 0; l < head; ++l) total += s.level_cost[l];
     const int stretches = std::max(1, std::min(8, (int)(total / 1e6)));
@@ -235,15 +255,13 @@ SweepPlan build_sweep_plan(const SweepDag& d, const SweepCost& cost, bool merge)
     }
     cut.push_back(head);
     std::vector<std::vector<Block>> parts(cut.size() - 1);
-    run_threads((int)parts.size(), [&](int i) { partition(s, cut[i], cut[i + 1], parts[i]); });
-    size_t held = 0;
-    for (auto& p : parts)
-      for (auto& b : p) {
-        held += b.idx.size();
-        blocks.push_back(std::move(b));
-      }
-    if (held <= most) break;
-    if (round == 5) merge = false;
+    run_threads((int)parts.size(), [&](int i) { partition(s, cut[i], cut[i + 1], limit, parts[i]); });
+    if (s.held <= limit) {
+      for (auto& p : parts)
+        for (auto& b : p) blocks.push_back(std::move(b));
+      break;
+    }
+    if (round == 7) merge = false;
   }
   if (!merge) {
     blocks.clear();

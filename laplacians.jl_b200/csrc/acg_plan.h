@@ -59,8 +59,12 @@ struct SweepCost {
   double entries_per_hop;  // entries all warps work through in the time of one hand-over
   double row_entries;      // entries of one row walked before it costs another load round trip
   double row_round;        // that round trip
-  int split = 0;           // rows longer than this are cut (one more hand-over); 0: none are
-  int part = 0;            // entries of a part
+  int split;               // rows longer than this are cut (one more hand-over); 0: none are
+  int part;                // entries of a part
+  // What the blocks' rows of M_B may hold at most: `fill` times the factor's
+  // entries, or fill_min entries where that is more.
+  double fill;
+  size_t fill_min;
 };
 
 // The DAG in internal vertex order (per graph: level by level): in-edges and
@@ -72,6 +76,10 @@ struct SweepDag {
   const std::vector<double>*fc, *bc;
   int tail_level;  // levels >= tail_level are the dense tail (nlev: none)
 };
+
+// Entries that the rows of all M_B together may hold: what `cost` allows, and
+// no more than leaves every entry, slot and row number of the plan an int.
+size_t sweep_fill_limit(const SweepCost& cost, int n, size_t factor_entries);
 
 // merge = false: every level is a block of its own.
 SweepPlan build_sweep_plan(const SweepDag& dag, const SweepCost& cost, bool merge);

@@ -776,8 +776,15 @@ namespace {
 // 812/851, 716/777, 778/842.  us per FP64 iteration with whole rows, rows cut
 // above 256 into parts of 128, above 256 and above 160 into parts of 64: matchings
 // of 150,000 vertices 321, 238, 230, 215; grid3(50) 208, 184, 179, 173.
-constexpr SweepCost kVectorCost{25000.0, 128.0, 0.4, 160, 64};
-constexpr SweepCost kBatchCost{10000.0, 32.0, 0.5, 0, 0};
+//
+// A plan holds its entries as indices and in both value types (16 bytes an entry
+// and direction), so deep factors are kept from filling in: up to 3 (2) times
+// the factor's entries, or 2M (1M) where that is more, which none of the grids,
+// geometric and matching graphs measured here reaches (at most 2.6 and 1.8 times
+// above that floor).  A path of 100,000 vertices took 12.7M entries without a
+// limit, 809 MB for both plans (3 MB for its factor alone), and takes 1.1M.
+constexpr SweepCost kVectorCost{25000.0, 128.0, 0.4, 160, 64, 3.0, (size_t)2 << 20};
+constexpr SweepCost kBatchCost{10000.0, 32.0, 0.5, 0, 0, 2.0, (size_t)1 << 20};
 
 // Groups: us per iteration of a graph's block (by depth and vertices, and by
 // vertices where p does not fit shared memory), and of the launches all graphs

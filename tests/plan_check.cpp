@@ -41,7 +41,7 @@ void* pc_build(int n, int nlev, int nrun, const int* levels, const int* fptr, co
   h->bidx.assign(bidx, bidx + bptr[n]);
   h->bc.assign(bc, bc + bptr[n]);
   const acg::SweepDag d{n, nlev, &h->runs, &h->fptr, &h->fidx, &h->bptr, &h->bidx, &h->fc, &h->bc, tail};
-  acg::SweepCost c{cost[0], cost[1], cost[2], (int)cost[3], (int)cost[4]};
+  acg::SweepCost c{cost[0], cost[1], cost[2], (int)cost[3], (int)cost[4], cost[5], (size_t)cost[6]};
   g_main = std::this_thread::get_id();
   g_fail = fail != 0;
   bool ok = true;
@@ -78,6 +78,12 @@ void pc_rows(const void* p, int dir, int* runs, int* ptr, int* idx, double* coef
   for (int v : R.ptr) *ptr++ = v;
   for (int v : R.idx) *idx++ = v;
   for (double v : R.coef) *coef++ = v;
+}
+
+// The entries a plan's blocks may hold for a factor of this size.
+long long pc_fill_limit(const double* cost, int n, long long entries) {
+  const acg::SweepCost c{cost[0], cost[1], cost[2], (int)cost[3], (int)cost[4], cost[5], (size_t)cost[6]};
+  return (long long)acg::sweep_fill_limit(c, n, (size_t)entries);
 }
 
 void pc_free(void* p) { delete static_cast<Handle*>(p); }

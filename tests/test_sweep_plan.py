@@ -17,8 +17,8 @@ from acgpu import generators as G
 
 HERE = pathlib.Path(__file__).parent
 CSRC = HERE.parent / "laplacians.jl_b200" / "csrc"
-VECTOR = (25000.0, 128.0, 0.4, 160, 64)
-BATCH = (10000.0, 32.0, 0.5, 0, 0)
+VECTOR = (25000.0, 128.0, 0.4, 160, 64, 3.0, 2 << 20)  # kVectorCost, kBatchCost
+BATCH = (10000.0, 32.0, 0.5, 0, 0, 2.0, 1 << 20)
 PART = 3  # kRowPart
 
 
@@ -92,6 +92,82 @@ def test_a_run_of_rows_belongs_to_one_graph(lib_path):
     for name in ("fwd", "bwd"):
         for v0, count, *_ in plan[name][0]:
             assert (v0 < 2) == (v0 + count - 1 < 2)
+
+
+def factor_dag(a, seed=1, dense_tail=2048):
+    """The DAG of a graph's factor, numbered as the solver numbers it: by level,
+    then by falling in-degree, then by elimination step; coefficients folded.
+    Also the plain factor's in-edges (the oracle of the sweeps)."""
+    acgpu.seed(seed)
+    f = acgpu.approx_chol(a)
+    n = a.shape[0]
+    col, ptr, row = f.col - 1, f.colptr - 1, f.rowval - 1
+    src = np.repeat(col, np.diff(ptr))
+    step = np.full(n, n - 1)
+    step[col] = np.arange(n - 1)
+    lev = np.zeros(n, np.int64)
+    val = np.empty(f.fval.shape[0])
+    for i, u in enumerate(col):
+        e = slice(ptr[i], ptr[i + 1])
+        lev[row[e]] = np.maximum(lev[row[e]], lev[u] + 1)
+        left = np.concatenate([[1.0], np.cumprod(1.0 - f.fval[e][:-1])])
+        val[e] = left * np.append(f.fval[e][:-1], 1.0)
+    indeg = np.bincount(row, minlength=n)
+    perm = np.lexsort((step, -indeg, lev))
+    num = np.empty(n, np.int64)
+    num[perm] = np.arange(n)
+    off = np.concatenate([[0], np.cumsum(np.bincount(lev))])
+    levels = [[(int(off[i]), int(off[i + 1]))] for i in range(len(off) - 1)]
+    tail = len(levels)
+    while tail > 0 and n - off[tail - 1] <= min(dense_tail, n // 4):
+        tail -= 1
+    if len(levels) - tail < 8:
+        tail = len(levels)
+    dst, s = num[row], num[src]
+    v0 = off[tail] if tail < len(levels) else n
+    keep = ~((dst >= v0) & (s >= v0))  # the sweeps keep the tail's inputs from the head
+    d = Dag(n, levels, dst[keep], s[keep], val[keep], tail)
+    full = Dag(n, levels, dst, s, val)
+    d.bptr, d.bidx, d.bc = full.bptr, full.bidx, full.bc
+    return d
+
+
+@pytest.mark.parametrize("cost", [VECTOR, BATCH])
+def test_deep_factors_do_not_fill_the_device(lib_path, cost):
+    """The blocks' entries stay within the limit however deep the DAG is: a path's
+    factor (one entry a column, as many levels as vertices) took 127 entries a
+    vertex."""
+    d = factor_dag(G.path_graph(60000))
+    factor = int(d.bptr[-1])
+    lib = ctypes.CDLL(str(lib_path))
+    lib.pc_fill_limit.restype = ctypes.c_longlong
+    c = np.array(cost, np.float64)
+    limit = lib.pc_fill_limit(ctypes.c_void_p(c.ctypes.data), d.n, ctypes.c_longlong(factor))
+    assert limit == max(cost[5] * factor, cost[6])
+    plan = d.build(lib_path, cost)
+    head = d.levels[d.tail][0][0]
+    assert plan["blocks"] < head  # still merged
+    for name in ("fwd", "bwd"):
+        assert len(plan[name][2]) <= (factor + limit) * (1 + 2 / 64)
+
+
+@pytest.mark.parametrize("cost", [VECTOR, BATCH])
+@pytest.mark.parametrize("n,factor", [(10**6, 8 * 10**6), (2 * 10**8, 10**9), (10**9, 10**9), (2 * 10**9, 2 * 10**9),
+                                      (10**6, 2**31 - 2), (1000, 2 * 10**9)])
+def test_plans_of_large_factors_stay_in_int_range(lib_path, cost, n, factor):
+    """Entries, slots and rows of a plan are ints: what a limit other than 0 (no
+    merging, no cutting) allows has to fit."""
+    lib = ctypes.CDLL(str(lib_path))
+    lib.pc_fill_limit.restype = ctypes.c_longlong
+    c = np.array(cost, np.float64)
+    limit = lib.pc_fill_limit(ctypes.c_void_p(c.ctypes.data), n, ctypes.c_longlong(factor))
+    if limit == 0:
+        assert factor + n > 10**9
+        return
+    entries = factor + limit
+    parts = -(-entries // cost[4]) + entries // cost[3] if cost[3] else 0
+    assert entries + parts < 2**31  # a long row's parts are entries of the row
+    assert 2 * n + parts < 2**31    # values, work values, parts; as many rows
 
 
 def test_an_allocation_that_fails_on_a_thread_is_an_exception(lib_path):
