@@ -157,52 +157,195 @@ std::vector<std::pair<int, int>> ranges(const SweepDag& d, int l0, int l1) {
   return out;
 }
 
-// Cuts the rows of R longer than `split` into parts of `part` entries with
-// slots from `base` on; returns the parts.
-int split_rows(SweepRows& R, int split, int part, int base) {
-  SweepRows out;
-  out.ptr.push_back(0);
-  out.idx.reserve(R.idx.size());
-  out.coef.reserve(R.coef.size());
-  std::vector<int> after(R.runs.size() + 1, 0);  // runs of out up to the end of run i
-  int parts = 0;
-  for (size_t i = 0; i < R.runs.size(); ++i) {
-    SweepRun run = R.runs[i];
-    const int first = parts;
-    for (int q = 0; q < run.count; ++q) {
-      const int k0 = R.ptr[run.row + q], k1 = R.ptr[run.row + q + 1];
-      if (k1 - k0 <= split) continue;
-      for (int k = k0; k < k1; k += part, ++parts) {
-        const int e = std::min(k1, k + part);
-        out.idx.insert(out.idx.end(), R.idx.begin() + k, R.idx.begin() + e);
-        out.coef.insert(out.coef.end(), R.coef.begin() + k, R.coef.begin() + e);
-        out.ptr.push_back((int)out.idx.size());
-      }
-    }
-    if (parts > first)  // v0 counts from 0: a part has no vertex
-      out.runs.push_back(SweepRun{0, parts - first, kRowPart, base + first, (int)out.ptr.size() - 1 - (parts - first)});
-    int next = first;
-    const int row = run.row;
-    run.row = (int)out.ptr.size() - 1;
-    for (int q = 0; q < run.count; ++q) {
-      const int k0 = R.ptr[row + q], k1 = R.ptr[row + q + 1];
-      if (k1 - k0 <= split) {
-        out.idx.insert(out.idx.end(), R.idx.begin() + k0, R.idx.begin() + k1);
-        out.coef.insert(out.coef.end(), R.coef.begin() + k0, R.coef.begin() + k1);
-      } else {
-        for (int k = k0; k < k1; k += part, ++next) {
-          out.idx.push_back(base + next);
-          out.coef.push_back(1.0);
-        }
-      }
-      out.ptr.push_back((int)out.idx.size());
-    }
-    out.runs.push_back(run);
-    after[i + 1] = (int)out.runs.size();
+// What the rows are made from.
+struct Layout {
+  const SweepDag& d;
+  const std::vector<int>& lev;
+  const std::vector<Block>& blocks;
+  const std::vector<int>& delta;  // of a vertex's work slot (0: it has none)
+  int head;                       // levels in blocks; the rest is the dense tail
+  int split, part, part_slot;     // rows longer than split are cut; the first part's slot
+};
+
+void add_run(SweepRows& R, const std::pair<int, int>& r, int kind, int delta) {
+  R.runs.push_back(SweepRun{r.first, r.second - r.first, kind, delta, (int)R.ptr.size() - 1});
+}
+
+// The factor's entries [k, e) as a row's, ending it.
+void add_row(SweepRows& R, const std::vector<int>& idx, const std::vector<double>& coef, int k, int e) {
+  R.idx.insert(R.idx.end(), idx.begin() + k, idx.begin() + e);
+  R.coef.insert(R.coef.end(), coef.begin() + k, coef.begin() + e);
+  R.ptr.push_back((int)R.idx.size());
+}
+
+void reserve_rows(SweepRows& R, const Layout& y, size_t entries) {
+  size_t rows = y.d.n;
+  for (const Block& b : y.blocks) {
+    entries += b.idx.size();
+    rows += b.vert.size();
   }
-  out.upto.resize(R.upto.size());
-  for (size_t l = 0; l < R.upto.size(); ++l) out.upto[l] = after[R.upto[l]];
-  R = std::move(out);
+  R.ptr.reserve(rows + 1);
+  R.idx.reserve(entries);
+  R.coef.reserve(entries);
+  R.ptr.push_back(0);
+  R.upto.assign(y.d.nlev, 0);
+}
+
+// Ends the last run: cuts its rows longer than y.split into parts, a run of
+// their own before it, with slots from y.part_slot + parts on.
+void end_run(const Layout& y, SweepRows& R, int& parts) {
+  SweepRun run = R.runs.back();
+  const int k = R.ptr[run.row];
+  bool any = false;
+  if (y.split)
+    for (int q = run.row; q < run.row + run.count && !any; ++q) any = R.ptr[q + 1] - R.ptr[q] > y.split;
+  if (!any) return;
+  const std::vector<int> ptr(R.ptr.begin() + run.row, R.ptr.end()), idx(R.idx.begin() + k, R.idx.end());
+  const std::vector<double> coef(R.coef.begin() + k, R.coef.end());
+  R.ptr.resize(run.row + 1);
+  R.idx.resize(k);
+  R.coef.resize(k);
+  R.runs.pop_back();
+  const int first = parts;
+  for (int q = 0; q < run.count; ++q) {
+    if (ptr[q + 1] - ptr[q] <= y.split) continue;
+    for (int a = ptr[q]; a < ptr[q + 1]; a += y.part, ++parts)
+      add_row(R, idx, coef, a - k, std::min(ptr[q + 1], a + y.part) - k);
+  }
+  // v0 counts from 0: a part has no vertex
+  R.runs.push_back(SweepRun{0, parts - first, kRowPart, y.part_slot + first, run.row});
+  run.row = (int)R.ptr.size() - 1;
+  R.runs.push_back(run);
+  int next = y.part_slot + first;
+  for (int q = 0; q < run.count; ++q) {
+    if (ptr[q + 1] - ptr[q] <= y.split) {
+      add_row(R, idx, coef, ptr[q] - k, ptr[q + 1] - k);
+      continue;
+    }
+    for (int a = ptr[q]; a < ptr[q + 1]; a += y.part) {
+      R.idx.push_back(next++);
+      R.coef.push_back(1.0);
+    }
+    R.ptr.push_back((int)R.idx.size());
+  }
+}
+
+// Blocks upwards, then the dense tail's rows (head inputs only).  Returns the
+// number of parts.
+int emit_forward(const Layout& y, SweepRows& F) {
+  int parts = 0;
+  const SweepDag& d = y.d;
+  const auto &fptr = *d.fptr, &fidx = *d.fidx;
+  const auto& fc = *d.fc;
+  std::vector<int> where(d.n);
+  reserve_rows(F, y, fidx.size());
+  for (const Block& b : y.blocks) {
+    const bool multi = b.l1 - b.l0 > 1;
+    for (const auto& r : ranges(d, b.l0, b.l0 + 1)) {
+      add_run(F, r, kRowPlain, multi ? y.delta[r.first] : 0);
+      for (int v = r.first; v < r.second; ++v) add_row(F, fidx, fc, fptr[v], fptr[v + 1]);
+      end_run(y, F, parts);
+    }
+    F.upto[b.l0] = (int)F.runs.size();
+    if (!multi) continue;
+    const auto rest = ranges(d, b.l0 + 1, b.l1);
+    for (const auto& r : rest) {
+      add_run(F, r, kRowWork, y.delta[r.first]);
+      for (int v = r.first; v < r.second; ++v) {  // the inputs before the block, which come first
+        int e = fptr[v];
+        while (e < fptr[v + 1] && y.lev[fidx[e]] < b.l0) ++e;
+        add_row(F, fidx, fc, fptr[v], e);
+      }
+      end_run(y, F, parts);
+    }
+    for (size_t i = 0; i < b.vert.size(); ++i) where[b.vert[i]] = (int)i;
+    for (const auto& r : rest) {
+      add_run(F, r, kRowFinal, y.delta[r.first]);
+      for (int v = r.first; v < r.second; ++v) {
+        const int row = where[v];
+        for (int e = b.ptr[row]; e < b.ptr[row + 1]; ++e) {
+          const int u = b.idx[e];
+          F.idx.push_back(y.lev[u] == b.l0 ? u : u + y.delta[u]);
+          F.coef.push_back(b.val[e]);
+        }
+        F.ptr.push_back((int)F.idx.size());
+      }
+      end_run(y, F, parts);
+    }
+    for (int l = b.l0 + 1; l < b.l1; ++l) F.upto[l] = (int)F.runs.size();
+  }
+  if (y.head < d.nlev) {
+    for (const auto& r : ranges(d, y.head, d.nlev)) {
+      add_run(F, r, kRowPlain, 0);
+      for (int v = r.first; v < r.second; ++v) add_row(F, fidx, fc, fptr[v], fptr[v + 1]);
+      end_run(y, F, parts);
+    }
+    for (int l = y.head; l < d.nlev; ++l) F.upto[l] = (int)F.runs.size();
+  }
+  return parts;
+}
+
+// Blocks downwards; a block's last level is its first step.
+int emit_backward(const Layout& y, SweepRows& B) {
+  int parts = 0;
+  const SweepDag& d = y.d;
+  const auto &bptr = *d.bptr, &bidx = *d.bidx;
+  const auto& bc = *d.bc;
+  std::vector<int> where(d.n), tptr, tidx, pos;
+  std::vector<double> tval;
+  reserve_rows(B, y, bidx.size());
+  for (auto it = y.blocks.rbegin(); it != y.blocks.rend(); ++it) {
+    const Block& b = *it;
+    const int top = b.l1 - 1;
+    const bool multi = top > b.l0;
+    for (const auto& r : ranges(d, top, b.l1)) {
+      add_run(B, r, kRowPlain, multi ? y.delta[r.first] : 0);
+      for (int v = r.first; v < r.second; ++v) add_row(B, bidx, bc, bptr[v], bptr[v + 1]);
+      end_run(y, B, parts);
+    }
+    B.upto[top] = (int)B.runs.size();
+    if (!multi) continue;
+    const auto rest = ranges(d, b.l0, top);
+    for (const auto& r : rest) {
+      add_run(B, r, kRowWork, y.delta[r.first]);
+      for (int v = r.first; v < r.second; ++v) {  // the targets after the block, which come first
+        int e = bptr[v];
+        while (e < bptr[v + 1] && y.lev[bidx[e]] >= b.l1) ++e;
+        add_row(B, bidx, bc, bptr[v], e);
+      }
+      end_run(y, B, parts);
+    }
+    // columns of M_B, targets descending (as the plain entries)
+    const int m = (int)b.vert.size();
+    for (int i = 0; i < m; ++i) where[b.vert[i]] = i;
+    tptr.assign(m + 1, 0);
+    for (int u : b.idx) tptr[where[u] + 1]++;
+    for (int i = 0; i < m; ++i) tptr[i + 1] += tptr[i];
+    tidx.resize(b.idx.size());
+    tval.resize(b.idx.size());
+    pos.assign(tptr.begin(), tptr.end() - 1);
+    for (int i = m - 1; i >= 0; --i)
+      for (int e = b.ptr[i]; e < b.ptr[i + 1]; ++e) {
+        const int c = where[b.idx[e]];
+        tidx[pos[c]] = b.vert[i];
+        tval[pos[c]] = b.val[e];
+        ++pos[c];
+      }
+    for (const auto& r : rest) {
+      add_run(B, r, kRowFinal, y.delta[r.first]);
+      for (int v = r.first; v < r.second; ++v) {
+        const int c = where[v];
+        for (int e = tptr[c]; e < tptr[c + 1]; ++e) {
+          const int u = tidx[e];
+          B.idx.push_back(y.lev[u] == top ? u : u + y.delta[u]);
+          B.coef.push_back(tval[e]);
+        }
+        B.ptr.push_back((int)B.idx.size());
+      }
+      end_run(y, B, parts);
+    }
+    for (int l = b.l0; l < top; ++l) B.upto[l] = (int)B.runs.size();
+  }
   return parts;
 }
 
@@ -280,130 +423,12 @@ SweepPlan build_sweep_plan(const SweepDag& d, const SweepCost& cost, bool merge)
       plan.nslots += r.second - r.first;
     }
   }
-  auto add_entry = [](SweepRows& R, int slot, double c) {
-    R.idx.push_back(slot);
-    R.coef.push_back(c);
-  };
-  auto add_run = [](SweepRows& R, int v0, int count, int kind, int del) {
-    R.runs.push_back(SweepRun{v0, count, kind, del, (int)R.ptr.size() - 1});
-  };
-  SweepRows &F = plan.fwd, &B = plan.bwd;
-  F.ptr.push_back(0);
-  B.ptr.push_back(0);
-  F.upto.assign(d.nlev, 0);
-  B.upto.assign(d.nlev, 0);
-
-  // ---- forward: blocks upwards, then the dense tail's rows (head inputs only)
-  for (const Block& b : blocks) {
-    const bool multi = b.l1 - b.l0 > 1;
-    for (const auto& r : ranges(d, b.l0, b.l0 + 1)) {
-      add_run(F, r.first, r.second - r.first, kRowPlain, multi ? delta[r.first] : 0);
-      for (int v = r.first; v < r.second; ++v) {
-        for (int k = (*d.fptr)[v]; k < (*d.fptr)[v + 1]; ++k) add_entry(F, (*d.fidx)[k], (*d.fc)[k]);
-        F.ptr.push_back((int)F.idx.size());
-      }
-    }
-    F.upto[b.l0] = (int)F.runs.size();
-    if (!multi) continue;
-    const auto rest = ranges(d, b.l0 + 1, b.l1);
-    for (const auto& r : rest) {
-      add_run(F, r.first, r.second - r.first, kRowWork, delta[r.first]);
-      for (int v = r.first; v < r.second; ++v) {
-        for (int k = (*d.fptr)[v]; k < (*d.fptr)[v + 1]; ++k) {
-          if (s.lev[(*d.fidx)[k]] >= b.l0) break;
-          add_entry(F, (*d.fidx)[k], (*d.fc)[k]);
-        }
-        F.ptr.push_back((int)F.idx.size());
-      }
-    }
-    for (size_t i = 0; i < b.vert.size(); ++i) s.where[b.vert[i]] = (int)i;
-    for (const auto& r : rest) {
-      add_run(F, r.first, r.second - r.first, kRowFinal, delta[r.first]);
-      for (int v = r.first; v < r.second; ++v) {
-        const int row = s.where[v];
-        for (int e = b.ptr[row]; e < b.ptr[row + 1]; ++e) {
-          const int u = b.idx[e];
-          add_entry(F, s.lev[u] == b.l0 ? u : u + delta[u], b.val[e]);
-        }
-        F.ptr.push_back((int)F.idx.size());
-      }
-    }
-    for (int l = b.l0 + 1; l < b.l1; ++l) F.upto[l] = (int)F.runs.size();
-  }
-  if (head < d.nlev) {
-    for (const auto& r : ranges(d, head, d.nlev)) {
-      add_run(F, r.first, r.second - r.first, kRowPlain, 0);
-      for (int v = r.first; v < r.second; ++v) {
-        for (int k = (*d.fptr)[v]; k < (*d.fptr)[v + 1]; ++k) add_entry(F, (*d.fidx)[k], (*d.fc)[k]);
-        F.ptr.push_back((int)F.idx.size());
-      }
-    }
-    for (int l = head; l < d.nlev; ++l) F.upto[l] = (int)F.runs.size();
-  }
-
-  // ---- backward: blocks downwards; a block's last level is its first step
-  std::vector<int> tptr, tidx;
-  std::vector<double> tval;
-  for (auto it = blocks.rbegin(); it != blocks.rend(); ++it) {
-    const Block& b = *it;
-    const int top = b.l1 - 1;
-    const bool multi = top > b.l0;
-    for (const auto& r : ranges(d, top, b.l1)) {
-      add_run(B, r.first, r.second - r.first, kRowPlain, multi ? delta[r.first] : 0);
-      for (int v = r.first; v < r.second; ++v) {
-        for (int k = (*d.bptr)[v]; k < (*d.bptr)[v + 1]; ++k) add_entry(B, (*d.bidx)[k], (*d.bc)[k]);
-        B.ptr.push_back((int)B.idx.size());
-      }
-    }
-    B.upto[top] = (int)B.runs.size();
-    if (!multi) continue;
-    const auto rest = ranges(d, b.l0, top);
-    for (const auto& r : rest) {
-      add_run(B, r.first, r.second - r.first, kRowWork, delta[r.first]);
-      for (int v = r.first; v < r.second; ++v) {
-        for (int k = (*d.bptr)[v]; k < (*d.bptr)[v + 1]; ++k) {
-          if (s.lev[(*d.bidx)[k]] < b.l1) break;
-          add_entry(B, (*d.bidx)[k], (*d.bc)[k]);
-        }
-        B.ptr.push_back((int)B.idx.size());
-      }
-    }
-    // columns of M_B, targets descending (as the plain entries)
-    const int m = (int)b.vert.size();
-    for (int i = 0; i < m; ++i) s.where[b.vert[i]] = i;
-    tptr.assign(m + 1, 0);
-    for (int u : b.idx) tptr[s.where[u] + 1]++;
-    for (int i = 0; i < m; ++i) tptr[i + 1] += tptr[i];
-    tidx.resize(b.idx.size());
-    tval.resize(b.idx.size());
-    {
-      std::vector<int> pos(tptr.begin(), tptr.end() - 1);
-      for (int i = m - 1; i >= 0; --i)
-        for (int e = b.ptr[i]; e < b.ptr[i + 1]; ++e) {
-          const int c = s.where[b.idx[e]];
-          tidx[pos[c]] = b.vert[i];
-          tval[pos[c]] = b.val[e];
-          ++pos[c];
-        }
-    }
-    for (const auto& r : rest) {
-      add_run(B, r.first, r.second - r.first, kRowFinal, delta[r.first]);
-      for (int v = r.first; v < r.second; ++v) {
-        const int c = s.where[v];
-        for (int e = tptr[c]; e < tptr[c + 1]; ++e) {
-          const int u = tidx[e];
-          add_entry(B, s.lev[u] == top ? u : u + delta[u], tval[e]);
-        }
-        B.ptr.push_back((int)B.idx.size());
-      }
-    }
-    for (int l = b.l0; l < top; ++l) B.upto[l] = (int)B.runs.size();
-  }
-  if (merge && cost.split) {  // s and y are vectors of their own: the same slots serve both
-    const int base = plan.nslots;
-    const int pf = split_rows(F, cost.split, cost.part, base), pb = split_rows(B, cost.split, cost.part, base);
-    plan.nslots += std::max(pf, pb);
-  }
+  // The directions share no state but the layout; s and y are vectors of their
+  // own, so the same slots serve the parts of both.
+  const Layout lay{d, s.lev, blocks, delta, head, merge ? cost.split : 0, cost.part, plan.nslots};
+  int parts[2] = {0, 0};
+  run_threads(2, [&](int i) { parts[i] = i == 0 ? emit_forward(lay, plan.fwd) : emit_backward(lay, plan.bwd); });
+  plan.nslots += std::max(parts[0], parts[1]);
   return plan;
 }
 

@@ -132,6 +132,57 @@ def factor_dag(a, seed=1, dense_tail=2048):
     return d
 
 
+GRAPHS = {
+    "path2": lambda: G.path_graph(2), "path3000": lambda: G.path_graph(3000), "star2000": lambda: G.star_graph(2000),
+    "tree4000": lambda: G.random_tree(4000, 4), "complete60": lambda: G.complete_graph(60),
+    "grid2_61x47": lambda: G.grid2(61, 47, weights="loguniform", seed=2),
+    "grid3_17": lambda: G.grid3(17, weights="loguniform", seed=3),
+    "matchings6000": lambda: G.path_plus_matchings(6000, seed=5),
+}
+
+
+def walk(plan, name, term, given):
+    """The plan's rows in their order, `term` a vertex's own term: every slot is
+    written once, and none is read before.  `given`: values there from the start
+    (NaN: none)."""
+    runs, ptr, idx, coef = plan[name]
+    out = np.full(plan["slots"], np.nan)
+    out[:given.shape[0]] = given
+    for v0, count, kind, delta, row in runs:
+        for i in range(count):
+            e = slice(ptr[row + i], ptr[row + i + 1])
+            total = float(coef[e] @ out[idx[e]]) + (term[v0 + i] if kind in (0, 1) else 0.0)
+            slot = v0 + i + (delta if kind in (1, PART) else 0)
+            assert np.isnan(out[slot]) and not np.isnan(total)
+            out[slot] = total
+    return out[:given.shape[0]]
+
+
+@pytest.mark.parametrize("cost,merge", [(VECTOR, True), (VECTOR[:3] + (16, 5) + VECTOR[5:], True), (BATCH, True),
+                                        (VECTOR, False)])
+@pytest.mark.parametrize("name", sorted(GRAPHS))
+def test_the_rows_are_the_substitutions(lib_path, name, cost, merge):
+    """Both directions against plain substitution over the DAG, to 1e-13 of the
+    largest value (a row sums at most a few thousand non-negative products)."""
+    d = factor_dag(GRAPHS[name]())
+    plan = d.build(lib_path, cost, merge)
+    rng = np.random.default_rng(1)
+    r, g = rng.uniform(0.5, 1.5, d.n), rng.uniform(0.5, 1.5, d.n)
+    v0 = d.levels[d.tail][0][0] if d.tail < len(d.levels) else d.n
+    s = r.copy()
+    for v in range(d.n):
+        e = slice(d.fptr[v], d.fptr[v + 1])
+        s[v] += d.fc[e] @ s[d.fidx[e]]
+    none = np.full(d.n, np.nan)
+    assert np.abs(walk(plan, "fwd", r, none) - s).max() <= 1e-13 * s.max()
+    y = g * s  # the tail's values are given
+    none[v0:] = y[v0:]
+    for v in range(v0 - 1, -1, -1):
+        e = slice(d.bptr[v], d.bptr[v + 1])
+        y[v] += d.bc[e] @ y[d.bidx[e]]
+    assert np.abs(walk(plan, "bwd", g * s, none) - y).max() <= 1e-13 * y.max()
+
+
 @pytest.mark.parametrize("cost", [VECTOR, BATCH])
 def test_deep_factors_do_not_fill_the_device(lib_path, cost):
     """The blocks' entries stay within the limit however deep the DAG is: a path's
