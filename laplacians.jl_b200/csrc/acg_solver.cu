@@ -109,6 +109,17 @@ struct DevSweep {
   }
 };
 
+// The DAG on the host, kept until the batched sweeps' plan is made from it.
+struct HostDag {
+  std::vector<std::vector<std::pair<int, int>>> runs;
+  std::vector<int> fptr, fidx, bptr, bidx;
+  std::vector<double> fc, bc;
+  int tail_level;
+  int heavy[2];    // rows with more entries get a whole warp: forward, backward
+  int unproduced;  // acg_options.test_unproduced_task
+  SweepDag view(int n) const { return {n, (int)runs.size(), &runs, &fptr, &fidx, &bptr, &bidx, &fc, &bc, tail_level}; }
+};
+
 // Graph capture and device (de)allocation are serialised across threads: an
 // allocation or free on one thread while another thread captures a stream can
 // invalidate that capture.  Graph launches do not take this lock.
@@ -140,12 +151,15 @@ struct SolverImpl {
   double min_inner_tol = 2e-5;       // mixed precision: floor of an inner solve's tolerance
   cudaEvent_t order_ev = nullptr;    // device entry points: after the legacy stream's work
   // sweep plans: [0] one vector, [1] batches (whose entries cost more, so their
-  // blocks are smaller); the per-level engine and the one-CTA tail need one
+  // blocks are smaller), made from `dag` with the first batch (a handle that
+  // solves single vectors needs neither its time nor its memory: 0.3 s and
+  // 274 MB for the 10^6-vertex grid); the per-level engine and the one-CTA tail need one
   // level per block and have plan 0 alone.  So does a group: some of its
   // members' PCG amplify a change of rounding to 1e-9 of x at tol 1e-8 (weights
   // of 1/distance), and a group's results stay those of its levels in turn.
   DevSweep sweep[2];
   bool two_plans = false;
+  std::unique_ptr<HostDag> dag;
   const DevSweep& batch_sweep() const { return sweep[two_plans ? 1 : 0]; }
 
   DevBuf<int> perm, lvl_off_d;
@@ -985,6 +999,91 @@ void build_gblock(SolverImpl& S, const SweepPlan& plan, const std::vector<std::v
   ACG_CUDA(cudaStreamSynchronize(S.stream));  // the uploads read this function's arrays
 }
 
+// Task records of a direction; after[i] = tasks up to the end of run i.
+std::vector<SweepTask> emit_tasks(const SweepRows& R, int heavy_min, std::vector<int>& after) {
+  std::vector<SweepTask> tasks;
+  after.reserve(R.runs.size());
+  for (const SweepRun& r : R.runs) {
+    int first = 0, cnt = 0;
+    auto push = [&](int i, int c, int heavy) {
+      SweepTask t = {};
+      t.v = r.v0 + i;
+      t.info = (r.kind << 4) | (c << 1) | heavy;
+      t.delta = r.delta;
+      for (int q = 0; q <= c; ++q) t.p[q] = R.ptr[r.row + i + q];
+      tasks.push_back(t);
+    };
+    for (int i = 0; i < r.count; ++i) {
+      if (R.ptr[r.row + i + 1] - R.ptr[r.row + i] > heavy_min) {
+        if (cnt) push(first, cnt, 0);
+        cnt = 0;
+        push(i, 1, 1);
+        continue;
+      }
+      if (cnt == 0) first = i;
+      if (++cnt == 4) {
+        push(first, 4, 0);
+        cnt = 0;
+      }
+    }
+    if (cnt) push(first, cnt, 0);
+    after.push_back((int)tasks.size());
+  }
+  return tasks;
+}
+
+// Testing only: blank one forward task record (it stores nothing), so the values
+// of its vertices are never produced and the waits on them run out after
+// spin_limit polls; the solve then reports ACG_ERR_TIMEOUT.  This is how the
+// bounded waits are tested without faulting or hanging the GPU.
+void unproduced_task(std::vector<SweepTask>& t, int blank) {
+  if (blank <= 0) return;
+  if (blank > (int)t.size()) throw InputError("test_unproduced_task is beyond the forward task tables");
+  t[blank - 1].info = 0;
+}
+
+void upload_rows(DevSweep& P, const SweepPlan& plan, cudaStream_t s) {
+  P.nslots = plan.nslots;
+  P.nnz_f = (int64_t)plan.fwd.idx.size();
+  P.nnz_b = (int64_t)plan.bwd.idx.size();
+  P.f_idx.upload(plan.fwd.idx, s);
+  P.f_c64.upload(plan.fwd.coef, s);
+  P.f_c32.upload(to_f32(plan.fwd.coef), s);
+  P.b_idx.upload(plan.bwd.idx, s);
+  P.b_c64.upload(plan.bwd.coef, s);
+  P.b_c32.upload(to_f32(plan.bwd.coef), s);
+}
+
+// The batched sweeps' task tables of a plan (its rows are on the device).
+void upload_batch_tasks(DevSweep& P, const SweepPlan& plan, int nlev, const int (&heavy)[2], int unproduced,
+                        cudaStream_t s) {
+  std::vector<int> af, ab;
+  std::vector<SweepTask> tf = emit_tasks(plan.fwd, heavy[0], af), tb = emit_tasks(plan.bwd, heavy[1], ab);
+  P.tfb_upto.assign(nlev, 0);
+  P.tbb_from.assign(nlev, 0);
+  for (int l = 0; l < nlev; ++l) {
+    if (plan.fwd.upto[l]) P.tfb_upto[l] = af[plan.fwd.upto[l] - 1];
+    if (plan.bwd.upto[l]) P.tbb_from[l] = ab[plan.bwd.upto[l] - 1];
+  }
+  unproduced_task(tf, unproduced);
+  P.ntasks_fb = (int)tf.size();
+  P.tasks_fb.upload(tf, s);
+  P.ntasks_bb = (int)tb.size();
+  P.tasks_bb.upload(tb, s);
+  ACG_CUDA(cudaStreamSynchronize(s));  // the uploads read this function's arrays
+}
+
+// The batched sweeps' plan: called with the solver's lock, before the first batch.
+// The planning is host work and does not hold up other threads' device work.
+void ensure_batch_plan(SolverImpl& S) {
+  if (!S.dag) return;
+  const SweepPlan plan = build_sweep_plan(S.dag->view(S.n), kBatchCost, true);
+  std::lock_guard<std::recursive_mutex> glk(g_device_mu);
+  upload_rows(S.sweep[1], plan, S.stream);
+  upload_batch_tasks(S.sweep[1], plan, S.nlev, S.dag->heavy, S.dag->unproduced, S.stream);
+  S.dag.reset();
+}
+
 // Builds the device solver for one graph, or for the block-diagonal union of
 // several graphs (seg_off: G+1 vertex offsets of contiguous diagonal blocks,
 // null for one graph).  The factor has ncol eliminated columns; the vertices
@@ -1206,7 +1305,7 @@ void build_solver(SolverImpl& S, int64_t n64, const int64_t* a_colptr, const int
   // Laplacian rows in internal order; diagonal = a*ones summed in column order
   std::vector<int> lptr(n + 1, 0), lidx(m + n);
   std::vector<double> lv(m + n);
-  {
+  auto laplacian = [&]() {
     std::vector<std::pair<int, double>> row;
     for (int i = 0; i < n; ++i) {
       const int u = perm[i];
@@ -1230,7 +1329,21 @@ void build_solver(SolverImpl& S, int64_t n64, const int64_t* a_colptr, const int
         lv[lptr[i] + k] = row[k].second;
       }
     }
-  }
+  };
+  // the one-vector sweeps' plan, beside it on a thread of its own
+  S.sweep_mode = (opts && opts->sweep_lanes == 1 && nseg == 1) ? 1 : 0;
+  const bool merge = S.sweep_mode == 0 && !(opts && opts->tail == 2) && nseg == 1;
+  SweepPlan plan;
+  auto planning = [&]() {
+    const SweepDag dag{n, nlev, &runs, &fptr, &fidx, &bptr, &bidx, &fc, &bc, S.dt_K ? S.dt_L0 : nlev};
+    SweepCost cost = kVectorCost;
+    plan = build_sweep_plan(dag, cost, merge);
+    if (n <= ACG_NOALLOC_MAX_N && plan.nslots > 3 * ACG_NOALLOC_MAX_N) {
+      cost.split = 0;  // the fixed scratch of acg_ldlsolve_noalloc holds two slots a vertex and more
+      plan = build_sweep_plan(dag, cost, merge);
+    }
+  };
+  run_threads(2, [&](int i) { i == 0 ? laplacian() : planning(); });
   S.nnz_l = m + n;
   S.nnz_f = F;
   // ---- tuning knobs
@@ -1275,136 +1388,64 @@ void build_solver(SolverImpl& S, int64_t n64, const int64_t* a_colptr, const int
   // ---- sweep plans and their task tables: a row with more than sweep_heavy
   // entries (default 16; batched 8) is a task of its own on a whole warp, other
   // rows go four to a task within one run
-  S.sweep_mode = (opts && opts->sweep_lanes == 1 && nseg == 1) ? 1 : 0;
-  const bool merge = S.sweep_mode == 0 && !(opts && opts->tail == 2) && nseg == 1;
+  // (From here on the solver allocates on the device.)
+  std::lock_guard<std::recursive_mutex> glk(g_device_mu);
   S.two_plans = merge;
-  int phases = nlev;
-  for (int w = 0; w < (S.two_plans ? 2 : 1); ++w) {
-    DevSweep& P = S.sweep[w];
-    const SweepDag dag{n, nlev, &runs, &fptr, &fidx, &bptr, &bidx, &fc, &bc, S.dt_K ? S.dt_L0 : nlev};
-    SweepCost cost = w == 0 ? kVectorCost : kBatchCost;
-    SweepPlan plan = build_sweep_plan(dag, cost, merge);
-    if (w == 0 && n <= ACG_NOALLOC_MAX_N && plan.nslots > 3 * ACG_NOALLOC_MAX_N) {
-      cost.split = 0;  // the fixed scratch of acg_ldlsolve_noalloc holds two slots a vertex and more
-      plan = build_sweep_plan(dag, cost, merge);
-    }
-    P.nslots = plan.nslots;
-    P.nnz_f = (int64_t)plan.fwd.idx.size();
-    P.nnz_b = (int64_t)plan.bwd.idx.size();
-    P.f_idx.upload(plan.fwd.idx, S.stream);
-    P.f_c64.upload(plan.fwd.coef, S.stream);
-    P.f_c32.upload(to_f32(plan.fwd.coef), S.stream);
-    P.b_idx.upload(plan.bwd.idx, S.stream);
-    P.b_c64.upload(plan.bwd.coef, S.stream);
-    P.b_c32.upload(to_f32(plan.bwd.coef), S.stream);
-    // tasks of a direction; after[i] = tasks up to the end of run i
-    auto emit = [](const SweepRows& R, int heavy_min, std::vector<int>& after) {
-      std::vector<SweepTask> tasks;
-      for (const SweepRun& r : R.runs) {
-        int first = 0, cnt = 0;
-        auto push = [&](int i, int c, int heavy) {
-          SweepTask t = {};
-          t.v = r.v0 + i;
-          t.info = (r.kind << 4) | (c << 1) | heavy;
-          t.delta = r.delta;
-          for (int q = 0; q <= c; ++q) t.p[q] = R.ptr[r.row + i + q];
-          tasks.push_back(t);
-        };
-        for (int i = 0; i < r.count; ++i) {
-          if (R.ptr[r.row + i + 1] - R.ptr[r.row + i] > heavy_min) {
-            if (cnt) push(first, cnt, 0);
-            cnt = 0;
-            push(i, 1, 1);
-            continue;
-          }
-          if (cnt == 0) first = i;
-          if (++cnt == 4) {
-            push(first, 4, 0);
-            cnt = 0;
-          }
-        }
-        if (cnt) push(first, cnt, 0);
-        after.push_back((int)tasks.size());
-      }
-      return tasks;
-    };
-    std::vector<int> af, ab, afb, abb;
-    const int sheavy = (opts && opts->sweep_heavy > 0) ? opts->sweep_heavy : 16;
-    const int bheavy = (opts && opts->batch_bwd_heavy > 0) ? opts->batch_bwd_heavy : 8;
-    const int fheavy = (opts && opts->batch_fwd_heavy > 0) ? opts->batch_fwd_heavy : 8;
-    std::vector<SweepTask> tfb = emit(plan.fwd, fheavy, afb), tbb = emit(plan.bwd, bheavy, abb);
-    P.tfb_upto.assign(nlev, 0);
-    P.tbb_from.assign(nlev, 0);
+  DevSweep& P = S.sweep[0];
+  upload_rows(P, plan, S.stream);
+  const int blank = opts ? opts->test_unproduced_task : 0;
+  const int bheavy[2] = {(opts && opts->batch_fwd_heavy > 0) ? opts->batch_fwd_heavy : 8,
+                         (opts && opts->batch_bwd_heavy > 0) ? opts->batch_bwd_heavy : 8};
+  if (!S.two_plans) upload_batch_tasks(P, plan, nlev, bheavy, blank, S.stream);
+  const int sheavy = (opts && opts->sweep_heavy > 0) ? opts->sweep_heavy : 16;
+  std::vector<int> af, ab;
+  std::vector<SweepTask> tf = emit_tasks(plan.fwd, sheavy, af), tb = emit_tasks(plan.bwd, sheavy, ab);
+  const int phases = merge ? 2 * plan.blocks : (S.dt_K ? S.dt_L0 : nlev);
+  // the tail: the longest run of final levels with at most 32 tasks in both
+  // tables whose values fit in shared memory (FP64 sizes, so both precisions fit)
+  if (!merge && nseg == 1 && opts->tail == 2) {
+    std::vector<int2> lf(nlev), lb(nlev);  // {first task, count} per level
     for (int l = 0; l < nlev; ++l) {
-      if (plan.fwd.upto[l]) P.tfb_upto[l] = afb[plan.fwd.upto[l] - 1];
-      if (plan.bwd.upto[l]) P.tbb_from[l] = abb[plan.bwd.upto[l] - 1];
+      const int f1 = af[plan.fwd.upto[l] - 1], f0 = l ? af[plan.fwd.upto[l - 1] - 1] : 0;
+      const int b1 = ab[plan.bwd.upto[l] - 1], b0 = l + 1 < nlev ? ab[plan.bwd.upto[l + 1] - 1] : 0;
+      lf[l] = make_int2(f0, f1 - f0);
+      lb[l] = make_int2(b0, b1 - b0);
     }
-    // Testing only: blank one forward task record (it stores nothing), so
-    // the values of its vertices are never produced and the waits on them
-    // run out after spin_limit polls; the solve then reports
-    // ACG_ERR_TIMEOUT.  This is how the bounded waits are tested without
-    // faulting or hanging the GPU.
-    const int blank = opts ? opts->test_unproduced_task : 0;
-    auto unproduced = [&](std::vector<SweepTask>& t) {
-      if (blank <= 0) return;
-      if (blank > (int)t.size()) throw InputError("test_unproduced_task is beyond the forward task tables");
-      t[blank - 1].info = 0;
-    };
-    unproduced(tfb);
-    P.ntasks_fb = (int)tfb.size();
-    P.tasks_fb.upload(tfb, S.stream);
-    P.ntasks_bb = (int)tbb.size();
-    P.tasks_bb.upload(tbb, S.stream);
-    if (w == 0) {
-      std::vector<SweepTask> tf = emit(plan.fwd, sheavy, af), tb = emit(plan.bwd, sheavy, ab);
-      phases = merge ? 2 * plan.blocks : (S.dt_K ? S.dt_L0 : nlev);
-      // the tail: the longest run of final levels with at most 32 tasks in both
-      // tables whose values fit in shared memory (FP64 sizes, so both precisions fit)
-      if (!merge && nseg == 1 && opts->tail == 2) {
-        std::vector<int2> lf(nlev), lb(nlev);  // {first task, count} per level
-        for (int l = 0; l < nlev; ++l) {
-          const int f1 = af[plan.fwd.upto[l] - 1], f0 = l ? af[plan.fwd.upto[l - 1] - 1] : 0;
-          const int b1 = ab[plan.bwd.upto[l] - 1], b0 = l + 1 < nlev ? ab[plan.bwd.upto[l + 1] - 1] : 0;
-          lf[l] = make_int2(f0, f1 - f0);
-          lb[l] = make_int2(b0, b1 - b0);
-        }
-        int optin = 0;
-        ACG_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, S.device));
-        const size_t cap = optin > 8192 ? (size_t)optin - 4096 : 0;
-        int lt = nlev, nv = 0;
-        while (lt > 0) {
-          const int l = lt - 1;
-          const int wd = S.lvl_off[l + 1] - S.lvl_off[l];
-          if (lf[l].y > kTailWarps || lb[l].y > kTailWarps) break;
-          if (tail_smem_bytes<double>(nv + wd, nlev - l) > cap) break;
-          nv += wd;
-          lt = l;
-        }
-        if (nlev - lt >= 8) {
-          S.tail_nl = nlev - lt;
-          S.tail_v0 = S.lvl_off[lt];
-          S.tail_nv = n - S.tail_v0;
-          S.tail_tf0 = lf[lt].x;
-          S.tail_tb0 = lb[lt].x + lb[lt].y;
-          std::vector<int2> tlf(lf.begin() + lt, lf.end()), tlb(lb.begin() + lt, lb.end());
-          S.tail_lvl_f.upload(tlf, S.stream);
-          S.tail_lvl_b.upload(tlb, S.stream);
-          const int tb_bytes = (int)tail_smem_bytes<double>(S.tail_nv, S.tail_nl);
-          ACG_CUDA(cudaFuncSetAttribute(k_tail<double, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, tb_bytes));
-          ACG_CUDA(cudaFuncSetAttribute(k_tail<double, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, tb_bytes));
-          ACG_CUDA(cudaFuncSetAttribute(k_tail<float, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, tb_bytes));
-          ACG_CUDA(cudaFuncSetAttribute(k_tail<float, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, tb_bytes));
-        }
-      }
-      if (nseg > 1 && blank <= 0) build_gblock(S, plan, runs, af, ab, tf, tb);
-      unproduced(tf);
-      P.ntasks_f = (int)tf.size();
-      P.tasks_f.upload(tf, S.stream);
-      P.ntasks_b = (int)tb.size();
-      P.tasks_b.upload(tb, S.stream);
+    int optin = 0;
+    ACG_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, S.device));
+    const size_t cap = optin > 8192 ? (size_t)optin - 4096 : 0;
+    int lt = nlev, nv = 0;
+    while (lt > 0) {
+      const int l = lt - 1;
+      const int wd = S.lvl_off[l + 1] - S.lvl_off[l];
+      if (lf[l].y > kTailWarps || lb[l].y > kTailWarps) break;
+      if (tail_smem_bytes<double>(nv + wd, nlev - l) > cap) break;
+      nv += wd;
+      lt = l;
     }
-    ACG_CUDA(cudaStreamSynchronize(S.stream));  // the uploads read this iteration's arrays
+    if (nlev - lt >= 8) {
+      S.tail_nl = nlev - lt;
+      S.tail_v0 = S.lvl_off[lt];
+      S.tail_nv = n - S.tail_v0;
+      S.tail_tf0 = lf[lt].x;
+      S.tail_tb0 = lb[lt].x + lb[lt].y;
+      std::vector<int2> tlf(lf.begin() + lt, lf.end()), tlb(lb.begin() + lt, lb.end());
+      S.tail_lvl_f.upload(tlf, S.stream);
+      S.tail_lvl_b.upload(tlb, S.stream);
+      const int tb_bytes = (int)tail_smem_bytes<double>(S.tail_nv, S.tail_nl);
+      ACG_CUDA(cudaFuncSetAttribute(k_tail<double, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, tb_bytes));
+      ACG_CUDA(cudaFuncSetAttribute(k_tail<double, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, tb_bytes));
+      ACG_CUDA(cudaFuncSetAttribute(k_tail<float, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, tb_bytes));
+      ACG_CUDA(cudaFuncSetAttribute(k_tail<float, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, tb_bytes));
+    }
   }
+  if (nseg > 1 && blank <= 0) build_gblock(S, plan, runs, af, ab, tf, tb);
+  unproduced_task(tf, blank);
+  P.ntasks_f = (int)tf.size();
+  P.tasks_f.upload(tf, S.stream);
+  P.ntasks_b = (int)tb.size();
+  P.tasks_b.upload(tb, S.stream);
+  ACG_CUDA(cudaStreamSynchronize(S.stream));  // the uploads read these arrays
   {
     int sms = 0;
     ACG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, S.device));
@@ -1545,6 +1586,11 @@ void build_solver(SolverImpl& S, int64_t n64, const int64_t* a_colptr, const int
     ACG_CUDA(cudaMallocHost(&S.h_gstates, sizeof(PcgState) * S.nseg));
   }
   ACG_CUDA(cudaStreamSynchronize(s));
+  if (S.two_plans) {
+    S.dag.reset(new HostDag{std::move(runs), std::move(fptr), std::move(fidx), std::move(bptr), std::move(bidx),
+                            std::move(fc), std::move(bc), S.dt_K ? S.dt_L0 : nlev, {bheavy[0], bheavy[1]}, blank});
+    if (blank > 0) ensure_batch_plan(S);  // refuses a record beyond the batched tables
+  }
 }
 
 // ---- small kernels for the one-shot entry points ---------------------------
@@ -2052,6 +2098,7 @@ void order_after_legacy_stream(SolverImpl& S) {
 }
 
 void ensure_batch(SolverImpl& S, int kp) {
+  ensure_batch_plan(S);
   if (!S.bst) {
     ACG_CUDA(cudaMalloc(&S.bst, sizeof(PcgState) * kMaxBatch));
     ACG_CUDA(cudaMalloc(&S.bsh, sizeof(BatchShared)));
@@ -2162,6 +2209,7 @@ int solve_batch(SolverImpl& S, const double* B, int64_t ldb, double* X, int64_t 
   cudaStream_t s = S.stream;
   const int kp = round_kp(k);
   drain_async(S);  // the asynchronous slots share the batch buffers
+  ensure_batch_plan(S);
   std::unique_lock<std::recursive_mutex> glk(g_device_mu);
   ensure_batch(S, std::max(kp, S.batch_kp));
   cudaGraphExec_t ge = batch_graph(S, 0, precision, kp);
@@ -2799,6 +2847,7 @@ int submit_async(acg_solver* h, const double* B, double* X, int k, int64_t ld, d
                  double maxtime, int stag_test, int precision, acg_request** out) {
   SolverImpl& S = h->impl;
   const int kp = round_kp(k);
+  ensure_batch_plan(S);
   std::unique_lock<std::recursive_mutex> glk(g_device_mu);
   ensure_async(S);
   if (kp > S.batch_kp) drain_async(S);  // growing the blocks frees the ones in flight
@@ -3096,16 +3145,21 @@ int acg_create(int64_t n, const int64_t* a_colptr, const int64_t* a_rowval, cons
   rc = check_device();
   if (rc != ACG_OK) return rc;
   return guarded("acg_create", [&]() {
-    std::lock_guard<std::recursive_mutex> glk(acg::g_device_mu);
     auto* h = new acg_solver();
     try {
       ACG_CUDA(cudaGetDevice(&h->impl.device));
-      ACG_CUDA(cudaStreamCreateWithFlags(&h->impl.stream, cudaStreamNonBlocking));
+      {
+        std::lock_guard<std::recursive_mutex> glk(acg::g_device_mu);
+        ACG_CUDA(cudaStreamCreateWithFlags(&h->impl.stream, cudaStreamNonBlocking));
+      }
+      // takes the lock once its host work is done
       acg::build_solver(h->impl, n, a_colptr, a_rowval, a_nzval, ldli_col, n - 1, ldli_colptr, ldli_rowval, ldli_fval,
                         ldli_d, ldli_nnz, index_base, opts);
       // set-up of the allocation-free entry point, with this device current
+      std::lock_guard<std::recursive_mutex> glk(acg::g_device_mu);
       h->impl.noalloc_scratch = acg::noalloc_scratch_for_current_device(h->impl.device);
     } catch (...) {
+      std::lock_guard<std::recursive_mutex> glk(acg::g_device_mu);
       delete h;
       throw;
     }
@@ -3272,14 +3326,18 @@ int acg_create_group(int64_t ngraphs, const int64_t* offsets, int64_t n, const i
   rc = check_device();
   if (rc != ACG_OK) return rc;
   return guarded("acg_create_group", [&]() {
-    std::lock_guard<std::recursive_mutex> glk(acg::g_device_mu);
     auto* h = new acg_solver();
     try {
       ACG_CUDA(cudaGetDevice(&h->impl.device));
-      ACG_CUDA(cudaStreamCreateWithFlags(&h->impl.stream, cudaStreamNonBlocking));
+      {
+        std::lock_guard<std::recursive_mutex> glk(acg::g_device_mu);
+        ACG_CUDA(cudaStreamCreateWithFlags(&h->impl.stream, cudaStreamNonBlocking));
+      }
+      // takes the lock once its host work is done
       acg::build_solver(h->impl, n, a_colptr, a_rowval, a_nzval, ldli_col, ncol, ldli_colptr, ldli_rowval, ldli_fval,
                         ldli_d, ldli_nnz, index_base, opts, ngraphs, offsets);
     } catch (...) {
+      std::lock_guard<std::recursive_mutex> glk(acg::g_device_mu);
       delete h;
       throw;
     }
@@ -3505,9 +3563,10 @@ int acg_serve_open(acg_solver* h, int precision, int slots, int queue, acg_serve
   return guarded("acg_serve_open", [&]() {
     acg::SolverImpl& S = h->impl;
     std::lock_guard<std::mutex> lk(S.mu);
+    ACG_CUDA(cudaSetDevice(S.device));
+    acg::ensure_batch_plan(S);
     std::lock_guard<std::recursive_mutex> glk(acg::g_device_mu);
     if (S.serving) throw acg::InputError("the solver already has a serving loop");
-    ACG_CUDA(cudaSetDevice(S.device));
     acg::drain_async(S);
     auto srv = std::make_unique<acg_server>();
     srv->h = h;
