@@ -52,6 +52,10 @@ template <typename T>
 struct DevBuf {
   T* p = nullptr;
   size_t n = 0;
+  DevBuf() = default;
+  DevBuf(const DevBuf&) = delete;
+  DevBuf& operator=(const DevBuf&) = delete;
+  ~DevBuf() { free(); }
   void alloc(size_t count) {
     free();
     if (count == 0) count = 1;
@@ -1541,8 +1545,6 @@ void build_solver(SolverImpl& S, int64_t n64, const int64_t* a_colptr, const int
                                                                              S.W64.p, S.W32.p);
       ACG_CUDA(cudaGetLastError());
       ACG_CUDA(cudaStreamSynchronize(s));
-      m.free();
-      mean.free();
     }
     int sms = 0;
     ACG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, S.device));
@@ -3059,7 +3061,7 @@ void serve_manager(acg_server* srv) {
     }
     bool busy = false;
     for (int e = 0; e < srv->capacity && !busy; ++e) busy = srv->owner[e].first != nullptr;
-    if (srv->closing && !busy && !srv->launched) break;
+    if (srv->closing && !srv->launched && (!busy || srv->err != ACG_OK)) break;
     if (srv->launched || busy) {
       // the loop runs: poll the done flags
       lk.unlock();
@@ -3096,6 +3098,41 @@ int guarded(const char* where, F&& fn) {
     acg::set_last_error(std::string(where) + ": " + e.what());
     return ACG_ERR_INVALID;
   }
+}
+
+// Ends the loop once the published requests are served and frees it; while
+// tickets are still to be waited, all but their results.
+int serve_stop(acg_server* srv) {
+  {
+    std::lock_guard<std::mutex> lk(srv->mu);
+    srv->closing = true;
+    srv->cv.notify_all();
+  }
+  if (srv->manager.joinable()) srv->manager.join();
+  acg::SolverImpl& S = srv->h->impl;
+  std::lock_guard<std::mutex> lk(S.mu);
+  cudaStreamSynchronize(srv->loop_stream);
+  if (srv->exec) cudaGraphExecDestroy(srv->exec);
+  for (int e = 0; e < srv->capacity; ++e) {
+    cudaFree(srv->bstage[e]);
+    cudaFree(srv->xstage[e]);
+  }
+  cudaFree(srv->slots);
+  cudaFreeHost(srv->ring_h);
+  cudaFreeHost(srv->reqs_h);
+  cudaEventDestroy(srv->loop_done);
+  cudaStreamDestroy(srv->loop_stream);
+  cudaStreamDestroy(srv->in_stream);
+  cudaStreamDestroy(srv->out_stream);
+  S.serving = false;
+  S.server = nullptr;
+  std::unique_lock<std::mutex> slk(srv->mu);
+  srv->h = nullptr;
+  const int rc = srv->err;
+  const bool last = srv->outstanding == 0;  // else the last acg_serve_wait frees it
+  slk.unlock();
+  if (last) delete srv;
+  return rc;
 }
 
 int check_device() {
@@ -3170,7 +3207,9 @@ int acg_create(int64_t n, const int64_t* a_colptr, const int64_t* a_rowval, cons
 
 void acg_destroy(acg_solver* h) {
   if (!h) return;
-  if (h->impl.server) acg_serve_close(h->impl.server);
+  // a loop whose tickets are still to be waited serves them first; the last wait
+  // then frees what is left of it
+  if (acg_server* srv = h->impl.server; srv && acg_serve_close(srv) == ACG_ERR_BUSY) serve_stop(srv);
   std::lock_guard<std::recursive_mutex> glk(acg::g_device_mu);
   {
     std::lock_guard<std::mutex> lk(h->impl.mu);
@@ -3712,9 +3751,11 @@ int acg_serve_wait(acg_ticket* t, acg_solve_info* info) {
   }
   std::unique_ptr<acg_ticket> own(t);
   acg_server* srv = t->srv;
+  std::unique_ptr<acg_server> last;  // freed after the lock
   std::unique_lock<std::mutex> lk(srv->mu);
   srv->cv.wait(lk, [&]() { return t->remaining == 0 || srv->err != ACG_OK; });
   srv->outstanding -= 1;
+  if (!srv->h && srv->outstanding == 0) last.reset(srv);
   if (t->remaining != 0) {
     acg::set_last_error(srv->err_msg);
     return srv->err;
@@ -3743,32 +3784,8 @@ int acg_serve_close(acg_server* srv) {
       acg::set_last_error("acg_serve_close: " + std::to_string(srv->outstanding) + " tickets not yet waited");
       return ACG_ERR_BUSY;
     }
-    srv->closing = true;  // requests already published are still served
-    srv->cv.notify_all();
   }
-  if (srv->manager.joinable()) srv->manager.join();
-  acg::SolverImpl& S = srv->h->impl;
-  const int rc = srv->err;
-  {
-    std::lock_guard<std::mutex> lk(S.mu);
-    cudaStreamSynchronize(srv->loop_stream);
-    if (srv->exec) cudaGraphExecDestroy(srv->exec);
-    for (int e = 0; e < srv->capacity; ++e) {
-      cudaFree(srv->bstage[e]);
-      cudaFree(srv->xstage[e]);
-    }
-    cudaFree(srv->slots);
-    cudaFreeHost(srv->ring_h);
-    cudaFreeHost(srv->reqs_h);
-    cudaEventDestroy(srv->loop_done);
-    cudaStreamDestroy(srv->loop_stream);
-    cudaStreamDestroy(srv->in_stream);
-    cudaStreamDestroy(srv->out_stream);
-    S.serving = false;
-    S.server = nullptr;
-  }
-  delete srv;
-  return rc;
+  return serve_stop(srv);
 }
 
 }  // extern "C"
