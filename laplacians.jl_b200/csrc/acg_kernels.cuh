@@ -65,7 +65,7 @@ struct PcgState {
   int sweep_error;             // a bounded wait of a sync-free sweep gave up
   long long nvert;             // vertices of this system (graphs of a group)
   int entering;                // joined a running serving loop: this pass is its pre-loop step
-  int pad1;
+  int resumed;                 // one-launch solves: left unfinished, the next launch goes on
   double pq_dot;               // batched loop: p.q summed by the mat-vec
   double elapsed;              // one-launch solves: seconds since t_start, as every block reads them
   unsigned int counter[16];    // last-block tickets of the reducing kernels

@@ -26,6 +26,15 @@
 // reduction finds those of the reduction before it pending or new, never old:
 // with two reductions an iteration (kWhole) these are the next that it polls.
 //
+// While it runs, a grid of two blocks per SM leaves next to no registers to other
+// streams, so a launch leaves after slice_s seconds, at the end of an iteration,
+// and a WHILE node launches the next, which goes on where it left (the vectors,
+// the scalars and the reduction slots are in device memory): work that waits gets
+// the SMs in between.  A 2048^3 matrix product (0.4 ms alone) beside solves of
+// 216,000 vertices (12 ms) took 0.5 ms between the launches of a kernel per step,
+// 12 ms beside one launch, and takes 1.5 ms beside launches of a millisecond;
+// these cost a solve alone 0.4 to 1 % (grid3(100) 28.07 -> 28.20 ms).
+//
 // Graphs of up to kDenseWhole vertices have W for the whole graph (k_pcg's
 // kWhole): no sweeps and two reductions an iteration.
 //
@@ -67,6 +76,7 @@ struct PersistArgs {
   int poll_mode;
   unsigned spin_limit;                 // polls of a sweep value
   unsigned red_limit;                  // polls of a reduction slot
+  double slice_s;                      // seconds after which a launch leaves
 };
 
 __device__ __forceinline__ bool gave_up(const PcgState* st) { return *((volatile const int*)&st->sweep_error) != 0; }
@@ -324,22 +334,25 @@ __global__ void __launch_bounds__(kPersistThreads, 2) k_pcg(const __grid_constan
   __shared__ double red_sm[kRedValues * kPersistThreads / 32];
   __shared__ PcgState ls;
   PcgState* gst = P.st;
-  if (gst->done) return;  // set before this launch: the same in every block
+  if (gst->done) return;  // set before this launch, as resumed: the same in every block
   const int tid = threadIdx.x, lane = tid & 31;
   const int gtid = blockIdx.x * blockDim.x + tid, gsize = gridDim.x * blockDim.x;
   const int n = P.n, K = P.K;
   const int ldw = w_stride(K);
   const size_t vs = P.vs;
+  bool first = kWhole || !gst->resumed;
+  __shared__ double since;  // ls.elapsed in this launch's first iteration
   if (tid == 0) {
     ls = *gst;
-    if (P.init == 1) ls.t_start = globaltimer_ns();
+    ls.resumed = 0;
+    since = -1.0;
+    if (P.init == 1 && first) ls.t_start = globaltimer_ns();
   }
   __syncthreads();
   const T* r = P.r0;  // the residual before the update (kWhole), and the current one
   T* rw = kWhole ? P.r1 : P.r0;
   const T* po = P.p0;
   T* pw = kWhole ? P.p1 : P.p0;
-  bool first = true;
   for (;;) {
     // ---- update: x', r' and their norms
     const double alpha = first ? 0.0 : ls.alpha;
@@ -521,10 +534,15 @@ __global__ void __launch_bounds__(kPersistThreads, 2) k_pcg(const __grid_constan
           ls.sum_abs_z = red_sm[3];
           stop = pcg_scalar_tail(&ls, P.eps, ls.elapsed);
         }
-        if (!stop) pcg_scalar_pq(&ls, red_sm[0], red_sm[1], red_sm[2], P.eps);
+        if (!stop) stop = pcg_scalar_pq(&ls, red_sm[0], red_sm[1], red_sm[2], P.eps);
+        if constexpr (!kWhole) {
+          // the same in every block: elapsed is block 0's, through a reduction
+          if (since < 0.0) since = ls.elapsed;
+          if (!stop && ls.elapsed - since > P.slice_s) ls.resumed = 1;
+        }
       }
       __syncthreads();
-      if (ls.done) break;
+      if (ls.done || (!kWhole && ls.resumed)) break;
     }
     if constexpr (kWhole) {
       const T* t = po;
@@ -593,6 +611,14 @@ __global__ void __launch_bounds__(kPersistThreads, 2) k_apply(const __grid_const
   red_collect<1>(P.red, 0, 1, red_sm, P.st, P.red_limit);
   const double mean = red_sm[0] / (double)P.n;
   for (int i = gtid; i < P.n; i += gsize) yext[perm[i]] = (double)P.y[(size_t)i * vs] - mean;
+}
+
+// Ends the loop around k_pcg's launches once the solve is done.  A kernel of its
+// own: with the call that sets the condition in k_pcg an iteration took 15 to
+// 30 % longer, also where no launch left early (200 x 200 grid 56 -> 68 us,
+// matchings of 150,000 vertices 213 -> 278).
+static __global__ void k_pcg_loop(const PcgState* st, LoopCtl ctl) {
+  if (st->done) clear_loop(ctl);
 }
 
 // The one-vector kernels are compiled in acg_persist.cu alone.

@@ -561,6 +561,14 @@ PersistArgs<T> persist_args(const SolverImpl& S) {
   return P;
 }
 
+// Seconds after which k_pcg leaves its SMs to others.
+constexpr double kPersistSlice = 1e-3;
+
+// The whole PCG is one launch without a loop around it: graphs whose
+// preconditioner is W alone.  They run one block per SM and leave half of it to
+// other streams.
+bool one_launch(const SolverImpl& S) { return S.persist && S.w_K == S.n; }
+
 // A cooperative launch of the solver's persistent grid.
 template <typename T, typename... KArgs, typename... Args>
 void launch_persist(cudaStream_t s, const SolverImpl& S, void (*kern)(KArgs...), Args... args) {
@@ -578,13 +586,19 @@ void launch_persist(cudaStream_t s, const SolverImpl& S, void (*kern)(KArgs...),
 }
 
 // The whole PCG of one right-hand side (r, x buffer 0 and the state set up by
-// k_center or k_outer_prep) as one cooperative launch.
+// k_center or k_outer_prep) as one cooperative launch, or as the body of the
+// WHILE node `ctl` whose launches go on where the one before left.
 template <typename T>
-void enqueue_persist(cudaStream_t s, const SolverImpl& S, double eps, int init) {
+void enqueue_persist(cudaStream_t s, const SolverImpl& S, double eps, int init, LoopCtl ctl) {
   PersistArgs<T> P = persist_args<T>(S);
   P.eps = eps;
   P.init = init;
+  P.slice_s = kPersistSlice;
   launch_persist<T>(s, S, S.w_K == S.n ? k_pcg<T, true> : k_pcg<T, false>, P);
+  if (ctl.use_handle) {
+    k_pcg_loop<<<1, 1, 0, s>>>(P.st, ctl);
+    ACG_CUDA(cudaGetLastError());
+  }
 }
 
 // One preconditioner application in the caller's vertex order.
@@ -677,28 +691,34 @@ cudaGraphExec_t build_fp64_graph(SolverImpl& S) {
   cudaGraph_t top;
   ACG_CUDA(cudaGraphCreate(&top, 0));
   cudaGraphConditionalHandle h{};
-  if (!S.persist) ACG_CUDA(cudaGraphConditionalHandleCreate(&h, top, 1u, cudaGraphCondAssignDefault));
-  LoopCtl ctl{h, S.persist ? 0 : 1};
+  const bool loop = !one_launch(S);
+  if (loop) ACG_CUDA(cudaGraphConditionalHandleCreate(&h, top, 1u, cudaGraphCondAssignDefault));
+  LoopCtl ctl{h, loop ? 1 : 0};
 
   begin_into(s, top, {});
   k_gather_in<<<kVecBlocks, kVecThreads, 0, s>>>(n, S.perm.p, S.b_ext.p, S.bm.p, S.st, S.partials.p);
   k_center<double><<<kVecBlocks, kVecThreads, 0, s>>>(n, S.bm.p, S.r64.p, S.x3_64.p, S.s64.p, S.y64.p, S.st,
                                                       S.partials.p, ctl, S.vs64, mark_args<double>(S));
-  if (S.persist) {
-    enqueue_persist<double>(s, S, kEps64, 1);
+  if (!loop) {
+    enqueue_persist<double>(s, S, kEps64, 1, ctl);
     return finish_fp64_graph(S, top, capture_end(s));
   }
-  enqueue_sweeps<double>(s, S, S.r64.p, S.s64.p, S.y64.p, S.st);
-  k_ysum<double><<<kVecBlocks, kVecThreads, 0, s>>>(n, S.y64.p, S.st, S.partials.p, ctl, S.vs64);
-  k_zdot<double><<<kVecBlocks, kVecThreads, 0, s>>>(n, S.y64.p, S.r64.p, S.p64.p, S.st, S.partials.p, kEps64, 1, ctl,
-                                                   S.vs64);
+  if (!S.persist) {
+    enqueue_sweeps<double>(s, S, S.r64.p, S.s64.p, S.y64.p, S.st);
+    k_ysum<double><<<kVecBlocks, kVecThreads, 0, s>>>(n, S.y64.p, S.st, S.partials.p, ctl, S.vs64);
+    k_zdot<double><<<kVecBlocks, kVecThreads, 0, s>>>(n, S.y64.p, S.r64.p, S.p64.p, S.st, S.partials.p, kEps64, 1,
+                                                     ctl, S.vs64);
+  }
   std::vector<cudaGraphNode_t> leaves = capture_leaves(s);
   end_into(s);
 
   cudaGraph_t body;
   cudaGraphNode_t wnode = add_while(top, leaves, h, &body);
   begin_into(s, body, {});
-  enqueue_pcg_iteration<double>(s, S, S.r64.p, S.s64.p, S.y64.p, S.p64.p, S.q64.p, S.x3_64.p, kEps64, ctl);
+  if (S.persist)
+    enqueue_persist<double>(s, S, kEps64, 1, ctl);
+  else
+    enqueue_pcg_iteration<double>(s, S, S.r64.p, S.s64.p, S.y64.p, S.p64.p, S.q64.p, S.x3_64.p, kEps64, ctl);
   end_into(s);
   return finish_fp64_graph(S, top, {wnode});
 }
@@ -749,27 +769,33 @@ cudaGraphExec_t build_mixed_graph(SolverImpl& S) {
   cudaGraph_t obody;
   cudaGraphNode_t onode = add_while(top, leaves, ho, &obody);
   cudaGraphConditionalHandle hi{};
-  if (!S.persist) ACG_CUDA(cudaGraphConditionalHandleCreate(&hi, obody, 1u, cudaGraphCondAssignDefault));
-  LoopCtl ictl{hi, S.persist ? 0 : 1};
+  const bool loop = !one_launch(S);
+  if (loop) ACG_CUDA(cudaGraphConditionalHandleCreate(&hi, obody, 1u, cudaGraphCondAssignDefault));
+  LoopCtl ictl{hi, loop ? 1 : 0};
 
   begin_into(s, obody, {});
   k_outer_prep<float><<<kVecBlocks, kVecThreads, 0, s>>>(n, S.r64.p, S.r32.p, S.x3_32.p, S.s32.p, S.y32.p, S.st,
                                                          S.partials.p, ictl, S.vs32, mark_args<float>(S));
-  if (S.persist) {
-    enqueue_persist<float>(s, S, eps32, 2);
+  if (!loop) {
+    enqueue_persist<float>(s, S, eps32, 2, ictl);
     return finish_mixed_graph(S, top, obody, onode, octl, capture_end(s));
   }
-  enqueue_sweeps<float>(s, S, S.r32.p, S.s32.p, S.y32.p, S.st);
-  k_ysum<float><<<kVecBlocks, kVecThreads, 0, s>>>(n, S.y32.p, S.st, S.partials.p, ictl, S.vs32);
-  k_zdot<float><<<kVecBlocks, kVecThreads, 0, s>>>(n, S.y32.p, S.r32.p, S.p32.p, S.st, S.partials.p, eps32, 2, ictl,
-                                                  S.vs32);
+  if (!S.persist) {
+    enqueue_sweeps<float>(s, S, S.r32.p, S.s32.p, S.y32.p, S.st);
+    k_ysum<float><<<kVecBlocks, kVecThreads, 0, s>>>(n, S.y32.p, S.st, S.partials.p, ictl, S.vs32);
+    k_zdot<float><<<kVecBlocks, kVecThreads, 0, s>>>(n, S.y32.p, S.r32.p, S.p32.p, S.st, S.partials.p, eps32, 2, ictl,
+                                                    S.vs32);
+  }
   std::vector<cudaGraphNode_t> ol = capture_leaves(s);
   end_into(s);
 
   cudaGraph_t ibody;
   cudaGraphNode_t inode = add_while(obody, ol, hi, &ibody);
   begin_into(s, ibody, {});
-  enqueue_pcg_iteration<float>(s, S, S.r32.p, S.s32.p, S.y32.p, S.p32.p, S.q32.p, S.x3_32.p, eps32, ictl);
+  if (S.persist)
+    enqueue_persist<float>(s, S, eps32, 2, ictl);
+  else
+    enqueue_pcg_iteration<float>(s, S, S.r32.p, S.s32.p, S.y32.p, S.p32.p, S.q32.p, S.x3_32.p, eps32, ictl);
   end_into(s);
 
   return finish_mixed_graph(S, top, obody, onode, octl, {inode});
