@@ -122,7 +122,10 @@ typedef struct acg_solver acg_solver;
 /* Optional tuning knobs of acg_create (0 = automatic). */
 typedef struct {
   int sweep_lanes;     /* sweep engine: 0 = sync-free dataflow sweep (one cooperative
-                          launch per sweep), 1 = one launch per level          */
+                          launch per sweep), 1 = one launch per level; groups:
+                          2 = launches that all graphs share, 3 = one block per
+                          graph (up to 131,072 vertices each), else the cheaper
+                          form by their sizes; the results are the same bits     */
   int spmv_lanes;      /* lanes per row in the Laplacian mat-vec: 2, 4, 8 or 16     */
   int wide_level_min;  /* levels at least this wide get a grid launch each; runs of
                           narrower levels whose values fit in shared memory run in

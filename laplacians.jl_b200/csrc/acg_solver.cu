@@ -946,12 +946,16 @@ std::vector<double> triangular_inverse(const std::vector<int>& fptr, const std::
   return m;
 }
 
+// acg_options.sweep_lanes of a group: either form, where the rule does not decide
+constexpr int kGroupShared = 2, kGroupBlocks = 3;
+
 // Decides whether the group's graphs run one block each (acg_gblock.cuh), and
 // cuts the union's task tables by graph and warp.  af / ab: tasks up to the end
 // of each run of the plan (a run is one level of one graph).
 void build_gblock(SolverImpl& S, const SweepPlan& plan, const std::vector<std::vector<std::pair<int, int>>>& level_runs,
                   const std::vector<int>& af, const std::vector<int>& ab, const std::vector<SweepTask>& tf,
-                  const std::vector<SweepTask>& tb) {
+                  const std::vector<SweepTask>& tb, int form) {
+  if (form == kGroupShared) return;
   const int nseg = S.nseg;
   std::vector<int> depth(nseg, 0), seg_of(S.n);
   int most = 0;
@@ -984,7 +988,7 @@ void build_gblock(SolverImpl& S, const SweepPlan& plan, const std::vector<std::v
     }
     // the slowest block, or several rounds of blocks with a half-empty last one
     const double blocks = nseg <= sms ? longest : std::max(longest, total / sms + 0.5 * longest);
-    S.gblock[w] = blocks < c.all_level * (double)level_runs.size() + c.all_vertex * (double)S.n;
+    S.gblock[w] = form == kGroupBlocks || blocks < c.all_level * (double)level_runs.size() + c.all_vertex * (double)S.n;
   }
   if (!S.gblock[0] && !S.gblock[1]) return;
   auto cut = [&](const SweepRows& R, const std::vector<int>& after, const std::vector<SweepTask>& all,
@@ -1469,7 +1473,7 @@ void build_solver(SolverImpl& S, int64_t n64, const int64_t* a_colptr, const int
       ACG_CUDA(cudaFuncSetAttribute(k_tail<float, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, tb_bytes));
     }
   }
-  if (nseg > 1 && blank <= 0) build_gblock(S, plan, runs, af, ab, tf, tb);
+  if (nseg > 1 && blank <= 0) build_gblock(S, plan, runs, af, ab, tf, tb, opts ? opts->sweep_lanes : 0);
   unproduced_task(tf, blank);
   P.ntasks_f = (int)tf.size();
   P.tasks_f.upload(tf, S.stream);
