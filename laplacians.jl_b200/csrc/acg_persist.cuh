@@ -654,7 +654,9 @@ static __global__ void __launch_bounds__(256) k_row_mean(int K, const double* __
 // on matchings of 60,000 vertices with lognormal weights one application was
 // 4.6e-14 from 64 bits without the means and the root taken out, 6e-16 with
 // the two triangular products.  The sums over k carry their rounding errors
-// along (two-sum and a product split by fma), since W is used many times.
+// along (two-sum and a product split by fma), since W is used many times; the
+// intrinsics keep the compiler from contracting a product into the additions
+// around it, which would count its rounding error twice.
 // 64 x 64 tiles, 4 x 4 entries a thread, FP64.  Run once per solver.
 constexpr int kWTile = 64;
 static __global__ void __launch_bounds__(256) k_form_w(int K, int ldw, const double* __restrict__ M,
@@ -680,9 +682,10 @@ static __global__ void __launch_bounds__(256) k_form_w(int K, int ldw, const dou
       for (int a = 0; a < 4; ++a)
 #pragma unroll
         for (int b = 0; b < 4; ++b) {
-          const double x = A[kk][ty * 4 + a], z = B[kk][tx * 4 + b], prod = x * z, old = acc[a][b];
-          const double sum = old + prod, t = sum - old;
-          low[a][b] += ((old - (sum - t)) + (prod - t)) + fma(x, z, -prod);
+          const double x = A[kk][ty * 4 + a], z = B[kk][tx * 4 + b], old = acc[a][b];
+          const double prod = __dmul_rn(x, z), sum = __dadd_rn(old, prod), t = __dsub_rn(sum, old);
+          const double err = __dadd_rn(__dsub_rn(old, __dsub_rn(sum, t)), __dsub_rn(prod, t));
+          low[a][b] = __dadd_rn(low[a][b], __dadd_rn(err, __fma_rn(x, z, -prod)));
           acc[a][b] = sum;
         }
     __syncthreads();
