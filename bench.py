@@ -422,9 +422,11 @@ def run_acgpu(args):
 
     # our kernel launches per step: set-up/wrap-up 3; per refinement the
     # outer kernels (6) and one preconditioner application (forward and
-    # backward launches); per inner iteration the library's count
-    per_it = kt["launches_per_iteration"]
-    per_ref = 6 + 2 * kt["forward_launches"]
+    # backward launches); per inner iteration the library's count.  One
+    # right-hand side: the inner solve is one launch and the kernel that ends
+    # its loop (more of both where a solve takes longer than a millisecond)
+    per_it = kt["launches_per_iteration"] if k > 1 else 0
+    per_ref = 6 + 2 * kt["forward_launches"] if k > 1 else 6
     launches = args.steps * (3 + refs.max() * per_ref + its.max() * per_it)
 
     extras = {}
@@ -465,8 +467,8 @@ def run_acgpu(args):
                          "algorithmic_bytes_per_launch": sweep_bytes, "launch_ms": sweep_ms,
                          "forward_sweep_ms": kt["forward_sweep_ms"], "backward_sweep_ms": kt["backward_sweep_ms"],
                          "dense_tail_ms": kt["dense_ms"], "dense_tail_vertices": stats["dense_vertices"],
-                         # the sweep walks the DAG's head levels one after another: time per level
-                         "swept_levels": swept_levels, "us_per_level": 1e3 * sweep_ms / max(1, swept_levels),
+                         # DAG levels before the dense tail; the sweep plan merges runs of them into blocks
+                         "swept_levels": swept_levels,
                          "spmv_ms": kt["spmv_ms"], "spmv_gbs": kt["spmv_bytes"] / (kt["spmv_ms"] * 1e-3) / 1e9},
             # every kernel of a batched solve, each timed alone (CUDA events, ms per launch)
             "kernel_ms": ({key: round(kt[key + "_ms"], 4) for key in
@@ -843,7 +845,7 @@ def matchings_2m_record(n=2_000_000):
     for prec in ("mixed", "fp64"):
         for _ in range(2):
             x, info = _device_solve(dev, b, prec, TOL)
-        kt = dev.time_kernels(prec, reps=3)
+        kt = dev.time_kernels(prec, reps=3)  # the sweeps as launches of their own
         out[prec] = {"solve_ms": info.solve_ms, "its": info.iterations, "refinements": info.refinements,
                      "true_relres": info.true_relres, "status": info.status,
                      "forward_ms": kt["forward_ms"], "backward_ms": kt["backward_ms"],

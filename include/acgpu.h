@@ -200,8 +200,9 @@ typedef struct {
   double iteration_ms;      /* the kernels of one PCG iteration              */
   int launches_per_iteration;
   int forward_launches;
-  /* algorithmic bytes per call: every structure entry, task record and vector
-     element the kernel must touch once (re-reads not counted) */
+  /* algorithmic bytes per call: every entry of the matrix or the factor, row
+     pointer and vector element once (re-reads, task records and what the merged
+     levels add to the factor's entries are not counted) */
   double spmv_bytes, forward_bytes, backward_bytes;
   /* the sweep kernel alone, without the dense tail products (equal to
      forward_ms / backward_ms when the solver has no dense tail) */

@@ -93,7 +93,6 @@ struct SweepStep {
 // tables of the one-vector sweeps (k_sweep) and of the batched ones (kb_sweep).
 struct DevSweep {
   int nslots = 0;                    // values of a sweep vector: n + the blocks' work slots
-  int64_t nnz_f = 0, nnz_b = 0;
   DevBuf<int> f_idx, b_idx;
   DevBuf<double> f_c64, b_c64;
   DevBuf<float> f_c32, b_c32;
@@ -134,6 +133,7 @@ struct SolverImpl {
   cudaStream_t stream = nullptr;
   int n = 0;
   int64_t nnz_l = 0, nnz_f = 0;
+  int64_t nnz_fsweep = 0, nnz_bsweep = 0;  // the factor's entries that the sweeps apply, without the dense tail's
   int nlev = 0;
   int vl_spmv = 8;
   int thin_max_width = 2048;
@@ -1078,8 +1078,6 @@ void unproduced_task(std::vector<SweepTask>& t, int blank) {
 
 void upload_rows(DevSweep& P, const SweepPlan& plan, cudaStream_t s) {
   P.nslots = plan.nslots;
-  P.nnz_f = (int64_t)plan.fwd.idx.size();
-  P.nnz_b = (int64_t)plan.bwd.idx.size();
   P.f_idx.upload(plan.fwd.idx, s);
   P.f_c64.upload(plan.fwd.coef, s);
   P.f_c32.upload(to_f32(plan.fwd.coef), s);
@@ -1380,6 +1378,8 @@ void build_solver(SolverImpl& S, int64_t n64, const int64_t* a_colptr, const int
   run_threads(2, [&](int i) { i == 0 ? laplacian() : planning(); });
   S.nnz_l = m + n;
   S.nnz_f = F;
+  S.nnz_fsweep = fptr[n];
+  S.nnz_bsweep = bptr[S.dt_K ? S.dt_v0 : n];
   // ---- tuning knobs
   S.vl_spmv = choose_vl((double)(m + n) / n);
   S.thin_max_width = 2048;
@@ -1860,10 +1860,10 @@ void time_kernels_t(SolverImpl& S, int reps, acg_kernel_times* out, T* r, T* sv,
   const double vb = sizeof(T), nv = S.n;
   // mat-vec: row pointers, (index, value) per entry, x once, y (FP64) out
   out->spmv_bytes = 4.0 * (nv + 1) + (double)S.nnz_l * (4.0 + vb) + nv * vb + nv * 8.0;
-  // sweeps: (index, coefficient) per entry, one 32-byte task record per task,
-  // aux (r or g) in, own forward value (backward), each input value once, output
-  out->forward_sweep_bytes = (double)S.sweep[0].nnz_f * (4.0 + vb) + 32.0 * S.sweep[0].ntasks_f + (nv + 2.0 * ns) * vb;
-  out->backward_sweep_bytes = (double)S.sweep[0].nnz_b * (4.0 + vb) + 32.0 * S.sweep[0].ntasks_b + 2.0 * (nv + ns) * vb;
+  // sweeps: (index, coefficient) per entry of the factor, row pointers, aux (r or g)
+  // in, own forward value (backward), each input value once, output
+  out->forward_sweep_bytes = (double)S.nnz_fsweep * (4.0 + vb) + 4.0 * (nv + 1) + 3.0 * nv * vb;
+  out->backward_sweep_bytes = (double)S.nnz_bsweep * (4.0 + vb) + 4.0 * (nv + 1) + 4.0 * nv * vb;
   // dense tail: the K(K+1)/2 entries of M once per product
   const double kk = (double)S.dt_K;
   out->dense_bytes = 2.0 * kk * (kk + 1.0) / 2.0 * vb;
@@ -2697,8 +2697,8 @@ void time_batch_t(SolverImpl& S, int reps, acg_kernel_times* out, T* r, T* sv, T
   out->forward_launches = 1 + dense_launches;
   const double vb = sizeof(T), nv = S.n;
   out->spmv_bytes = 4.0 * (nv + 1) + (double)S.nnz_l * (4.0 + vb) + 2.0 * nv * kp * vb;
-  out->forward_sweep_bytes = (double)P.nnz_f * (4.0 + vb) + 32.0 * P.ntasks_fb + (nv + 2.0 * P.nslots) * kp * vb;
-  out->backward_sweep_bytes = (double)P.nnz_b * (4.0 + vb) + 32.0 * P.ntasks_bb + nv * vb + (nv + 2.0 * P.nslots) * kp * vb;
+  out->forward_sweep_bytes = (double)S.nnz_fsweep * (4.0 + vb) + 4.0 * (nv + 1) + 3.0 * nv * kp * vb;
+  out->backward_sweep_bytes = (double)S.nnz_bsweep * (4.0 + vb) + 4.0 * (nv + 1) + nv * vb + 3.0 * nv * kp * vb;
   const double kk = (double)S.dt_K;
   out->dense_bytes = 2.0 * kk * (kk + 1.0) / 2.0 * vb;
   out->forward_bytes = out->forward_sweep_bytes + out->dense_bytes / 2.0;
@@ -3269,7 +3269,7 @@ int acg_solver_stats(const acg_solver* h, acg_stats* out) {
   out->sweep_lanes = acg::kLightLanes;
   size_t bytes = 0;
   auto add = [&](const auto& b) { bytes += b.n * sizeof(*b.p); };
-  add(S.perm); add(S.lvl_off_d); add(S.l_ptr); add(S.l_idx); add(S.f_ptr); add(S.f_idx); add(S.b_ptr); add(S.b_idx);
+  add(S.perm); add(S.iperm); add(S.dt_M64); add(S.dt_M32); add(S.dt_part); add(S.lvl_off_d); add(S.l_ptr); add(S.l_idx); add(S.f_ptr); add(S.f_idx); add(S.b_ptr); add(S.b_idx);
   add(S.l_v64); add(S.f_c64); add(S.b_c64); add(S.g64); add(S.l_v32); add(S.f_c32); add(S.b_c32); add(S.g32);
   add(S.b_ext); add(S.x_ext); add(S.bm); add(S.r64); add(S.s64); add(S.y64); add(S.p64); add(S.q64); add(S.x3_64);
   add(S.xf); add(S.r32); add(S.s32); add(S.y32); add(S.p32); add(S.q32); add(S.x3_32); add(S.partials);
