@@ -142,14 +142,26 @@ class SolveServer:
             self._graphs[gid] = _GraphEntry(gid, a, ldli)
 
     def _estimate_bytes(self, e: _GraphEntry) -> int:
+        """What e's solver, its batch buffers and its loop hold on the device, at
+        most: the sweep plans are counted as full as they may be (kVectorCost and
+        kBatchCost in csrc/acg_solver.cu), since only building one tells."""
         n = e.a.shape[0]
-        nnz_l = e.a.nnz + n
         F = e.ldli.nnz
-        structure = nnz_l * 16 + 2 * F * 16 + n * 64
-        vectors = n * 8 * 30
-        batch = n * self.slots * (9 * 8 + 3 * 8 + 8 * 4)
+        kp = next(k for k in (8, 16, 32, 64) if k >= min(self.slots, 64))
+        pairs = n * n // 2
+        fill = [min(max(3 * F, 2 << 20), pairs), min(max(2 * F, 1 << 20), pairs)]
+        slots = 2 * n + (F + fill[0]) // 53  # values, work values, parts of long rows
+        structure = (e.a.nnz + n) * 16 + n * 32
+        # per direction: an index and two coefficients an entry, 32 bytes a task
+        plans = sum(2 * 16 * (F + m) + 2 * 32 * 2 * n for m in fill)
+        vectors = n * 104 + slots * 4 * 32  # the sweeps' four hold a sector a slot
+        K = min(2048, n // 4)
+        W = n if n <= 2048 else K
+        dense = 12 * K * K + (K // 256 + 1) * K * 64 * 8 + 12 * W * (W + 63)
+        batch = n * kp * (10 * 8 + 6 * 4) + 2 * n * kp * (2 * 8 + 2 * 4)
         staging = 0 if self.unbatched else n * 8 * 2 * (self.slots + self.queue)
-        return int(structure + vectors + batch + staging)
+        reductions = 4 << 20
+        return int(structure + plans + vectors + dense + batch + staging + reductions)
 
     def _reserve(self, e: _GraphEntry) -> bool:
         """With the lock held: reserve e's bytes, evicting idle graphs (least
