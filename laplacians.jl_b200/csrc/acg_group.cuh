@@ -37,7 +37,6 @@ struct GroupArgs {
   PcgState* gst;          // group flags: done (all stopped), sweep_error
   GroupShared* gsh;
   int nseg;
-  int n, nslots;          // vertices and sweep slots of the union
 };
 
 // Block reduction of NV values; the last block of the chunk's graph gets the
@@ -127,7 +126,6 @@ __global__ void __launch_bounds__(kVecThreads) kg_update(int n, T* x3, const T* 
   const T* xc = x3 + (size_t)sc->xcur * n;
   T* xn = x3 + (size_t)sc->xnext * n;
   const T pend = pending_value<T>();
-  mark_work_slots(n, g.nslots, s_out, y_out, vs);
   double acc[3] = {0.0, 0.0, 0.0};
   for (int i = c.start + threadIdx.x; i < c.end; i += blockDim.x) {
     s_out[(size_t)i * vs] = pend;
@@ -227,7 +225,6 @@ __global__ void __launch_bounds__(kVecThreads) kg_center(double* __restrict__ bm
   const SegChunk c = g.chunks[blockIdx.x];
   const double mu = g.st[c.seg].mean;
   const T pend = pending_value<T>();
-  mark_work_slots(g.n, g.nslots, s_out, y_out, vs);
   double acc[2] = {0.0, 0.0};
   for (int i = c.start + threadIdx.x; i < c.end; i += blockDim.x) {
     const double v = bm[i] - mu;
@@ -344,7 +341,6 @@ __global__ void __launch_bounds__(kVecThreads) kg_outer_prep(const double* __res
   const SegChunk c = g.chunks[blockIdx.x];
   PcgState* s = &g.st[c.seg];
   const T pend = pending_value<T>();
-  mark_work_slots(g.n, g.nslots, s_out, y_out, vs);
   if (s->outer_done) {
     for (int i = c.start + threadIdx.x; i < c.end; i += blockDim.x) {
       s_out[(size_t)i * vs] = pend;

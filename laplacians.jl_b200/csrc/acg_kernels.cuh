@@ -412,12 +412,6 @@ __device__ __noinline__ T wait_value_slow(const T* p, PcgState* st, int poll_mod
   }
 }
 
-template <typename T>
-__device__ __forceinline__ T wait_value(const T* p, PcgState* st, int poll_mode, unsigned spin_limit) {
-  const T x = ld_relaxed(p);
-  return is_pending(x) ? wait_value_slow(p, st, poll_mode, spin_limit) : x;
-}
-
 // A task record (32 bytes): {first vertex, kind << 4 | count << 1 | heavy,
 // p[0..4], delta}: the task's rows are p[i]..p[i+1], so a lane finds its entry
 // range without another dependent load.  A heavy task is one row on 32 lanes,
@@ -694,22 +688,14 @@ struct MarkArgs {
   int nwt;
 };
 template <typename T>
-__device__ __forceinline__ void mark_work_slots(int n, int nslots, T* s, T* y, int vs);
-template <typename T>
 __device__ __forceinline__ void mark_all(int n, const MarkArgs<T>& m, T* s, T* y, int vs) {
-  mark_work_slots(n, m.nslots, s, y, vs);
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < m.nred; i += gridDim.x * blockDim.x)
-    m.red[i] = pending_value<double>();
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < m.nwt; i += gridDim.x * blockDim.x)
-    m.wt[i] = pending_value<T>();
-}
-template <typename T>
-__device__ __forceinline__ void mark_work_slots(int n, int nslots, T* s, T* y, int vs) {
-  const T pv = pending_value<T>();
-  for (int i = n + blockIdx.x * blockDim.x + threadIdx.x; i < nslots; i += gridDim.x * blockDim.x) {
-    s[(size_t)i * vs] = pv;
-    y[(size_t)i * vs] = pv;
+  const int i0 = blockIdx.x * blockDim.x + threadIdx.x, S = gridDim.x * blockDim.x;
+  for (int i = n + i0; i < m.nslots; i += S) {
+    s[(size_t)i * vs] = pending_value<T>();
+    y[(size_t)i * vs] = pending_value<T>();
   }
+  for (int i = i0; i < m.nred; i += S) m.red[i] = pending_value<double>();
+  for (int i = i0; i < m.nwt; i += S) m.wt[i] = pending_value<T>();
 }
 
 // Shared memory bytes of a thin run with nv vertices and nl levels.

@@ -191,11 +191,9 @@ __global__ void __launch_bounds__(kVecThreads) k_spmv_pq(int n, const int* __res
 template <typename T>
 __global__ void __launch_bounds__(kVecThreads) k_update(int n, T* x3, const T* __restrict__ p, const T* __restrict__ q,
                                                         T* __restrict__ r, T* __restrict__ s_out, T* __restrict__ y_out,
-                                                        PcgState* st, double* partials, LoopCtl ctl, int vs,
-                                                        int nslots) {
+                                                        PcgState* st, double* partials, LoopCtl ctl, int vs) {
   if (st->done) return;
   const T pend = pending_value<T>();
-  mark_work_slots(n, nslots, s_out, y_out, vs);
   const double al = st->alpha;
   const T* xc = x3 + (size_t)st->xcur * n;
   T* xn = x3 + (size_t)st->xnext * n;

@@ -16,7 +16,7 @@
 //
 // w and w' have their own slots behind the n values of the swept vector: a
 // vertex v of a block of several levels has slot v + delta (delta one per run
-// of consecutive vertices).  Rows come in three kinds, each a sweep task:
+// of consecutive vertices).  Rows come in four kinds, each a sweep task:
 //   kRowPlain  out[v] = aux(v) + sum          (a block's first level)
 //   kRowWork   out[v + delta] = aux(v) + sum  (the other levels' w or w')
 //   kRowFinal  out[v] = sum                   (the same vertices' M_B row)
@@ -45,7 +45,7 @@ struct SweepRows {
   std::vector<SweepRun> runs;
   std::vector<int> ptr, idx;
   std::vector<double> coef;
-  std::vector<int> upto;  // per DAG level: rows up to the last one the level needs
+  std::vector<int> upto;  // per DAG level: runs up to the last one the level needs
 };
 
 struct SweepPlan {

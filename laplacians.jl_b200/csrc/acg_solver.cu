@@ -490,8 +490,7 @@ void enqueue_pcg_iteration(cudaStream_t s, const SolverImpl& S, T* r, T* sv, T* 
   const TypedArrays<T> A = arrays_of<T>(S);
   ACG_VL_SWITCH(S.vl_spmv, spmv_pq_vl, s, S, A, p, q, S.st, eps, ctl);
   const int vs = vstride<T>(S);
-  k_update<T><<<kVecBlocks, kVecThreads, 0, s>>>(S.n, x3, p, q, r, sv, y, S.st, S.partials.p, ctl, vs,
-                                                 S.sweep[0].nslots);
+  k_update<T><<<kVecBlocks, kVecThreads, 0, s>>>(S.n, x3, p, q, r, sv, y, S.st, S.partials.p, ctl, vs);
   enqueue_sweeps<T>(s, S, r, sv, y, S.st);
   k_ysum<T><<<kVecBlocks, kVecThreads, 0, s>>>(S.n, y, S.st, S.partials.p, ctl, vs);
   k_zdot<T><<<kVecBlocks, kVecThreads, 0, s>>>(S.n, y, r, p, S.st, S.partials.p, eps, 0, ctl, vs);
@@ -2277,7 +2276,7 @@ int solve_batch(SolverImpl& S, const double* B, int64_t ldb, double* X, int64_t 
 
 GroupArgs group_args(const SolverImpl& S) {
   return GroupArgs{S.chunks.p, S.seg_first.p, S.seg_nchunk.p, S.seg_cnt.p, S.gpartials.p, S.gstates, S.gflags,
-                   S.gsh, S.nseg, S.n, S.sweep[0].nslots};
+                   S.gsh, S.nseg};
 }
 
 // Every graph's whole PCG, one block each.
