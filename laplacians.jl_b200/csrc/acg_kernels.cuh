@@ -456,7 +456,7 @@ __device__ __forceinline__ SweepTask load_task(const SweepTask* __restrict__ tas
   return r;
 }
 
-template <typename T, bool kForward, bool kLoadAux = true, int U = kEntryUnroll>
+template <typename T, bool kForward, bool kLoadAux = true, int U = kEntryUnroll, bool kPlain = false>
 __device__ __forceinline__ void load_entries(SweepEntries<T, U>& e, const SweepTask& r, int lane,
                                              const int* __restrict__ idx, const T* __restrict__ coef,
                                              const T* __restrict__ aux, const T* __restrict__ sfwd, int vs = 1) {
@@ -476,7 +476,7 @@ __device__ __forceinline__ void load_entries(SweepEntries<T, U>& e, const SweepT
   if (!active) k0 = k1 = 0;
   e.k0 = k0 + gl;
   e.k1 = k1;
-  const bool term = kLoadAux && active && e.term();
+  const bool term = kLoadAux && active && (kPlain || e.term());
   e.a = term ? __ldg(&aux[e.v]) : T(0);
   e.own = (!kForward && term) ? __ldg(&sfwd[(size_t)e.v * vs]) : T(0);
 #pragma unroll
@@ -543,8 +543,9 @@ __device__ __forceinline__ void gather_entries(T& acc, const int (&id)[U], const
 
 // Warp w runs tasks w, w+W, w+2W, ... (W warps in the grid).  Task records
 // are loaded two tasks ahead and entries one task ahead, so only the waits on
-// input values sit on the dependency chain.
-template <typename T, bool kForward>
+// input values sit on the dependency chain.  kPlain: all rows are of that kind
+// (one level per block).
+template <typename T, bool kForward, bool kPlain>
 __global__ void __launch_bounds__(kSweepThreads) k_sweep(int ntasks, const SweepTask* __restrict__ tasks,
                                                          const int* __restrict__ idx, const T* __restrict__ coef,
                                                          const T* __restrict__ aux, const T* __restrict__ sfwd, T* out,
@@ -558,17 +559,31 @@ __global__ void __launch_bounds__(kSweepThreads) k_sweep(int ntasks, const Sweep
   SweepEntries<T> e0;
   {
     const SweepTask r0 = load_task(tasks, t, ntasks);
-    load_entries<T, kForward>(e0, r0, lane, idx, coef, aux, sfwd, vs);
+    load_entries<T, kForward, true, kEntryUnroll, kPlain>(e0, r0, lane, idx, coef, aux, sfwd, vs);
   }
   for (; t < ntasks; t += W) {
     const SweepTask r2 = load_task(tasks, t + 2 * W, ntasks);
     SweepEntries<T> e1;
-    load_entries<T, kForward>(e1, r1, lane, idx, coef, aux, sfwd, vs);
+    load_entries<T, kForward, true, kEntryUnroll, kPlain>(e1, r1, lane, idx, coef, aux, sfwd, vs);
     const int gw = e0.gw();
     T acc = T(0);
-    // a row longer than the prefetched entries goes on in chunks of the same
-    // size: one value round trip per chunk, not per round of entries
-    for (int k = e0.k0; k < e0.k1;) {
+    // A row longer than the prefetched entries goes on in chunks of the same size
+    // (one value round trip per chunk, not per round of entries), except in FP64
+    // without merged levels: there rows are shorter and levels wider, and the
+    // chunks' registers cost more than the round trips.  ms per solve of a group of
+    // 90 grids and geometric graphs, chunks and rounds: FP64 58.6 / 56.5, mixed
+    // 114.5 / 116.7.  (One kernel for rows of all kinds: 59.7 and 116.8; 256 graphs
+    // 142.1 and 417, against 125.9 and 409 with kPlain.)
+    constexpr bool kChunks = !kPlain || sizeof(T) == 4;
+    if constexpr (!kChunks) {
+      gather_entries<T, kEntryUnroll>(acc, e0.id, e0.c, out, vs, st, poll_mode, spin_limit);
+      for (int k = e0.k0 + kEntryUnroll * gw; k < e0.k1; k += gw) {
+        const T* p = &out[(size_t)__ldg(&idx[k]) * vs];
+        const T c = __ldg(&coef[k]), x = ld_relaxed(p);
+        acc += c * (is_pending(x) ? wait_value_slow(p, st, poll_mode, spin_limit) : x);
+      }
+    }
+    for (int k = e0.k0; kChunks && k < e0.k1;) {
       gather_entries<T, kEntryUnroll>(acc, e0.id, e0.c, out, vs, st, poll_mode, spin_limit);
       k += kEntryUnroll * gw;
       if (k >= e0.k1) break;
@@ -581,7 +596,8 @@ __global__ void __launch_bounds__(kSweepThreads) k_sweep(int ntasks, const Sweep
     }
     __syncwarp();  // reconverge after the divergent waits before the shuffles
     acc = group_sum_w(acc, gw);
-    if (e0.active(lane) && (lane & (gw - 1)) == 0) st_relaxed(&out[(size_t)e0.slot() * vs], kForward ? e0.a + acc : e0.a * e0.own + acc);
+    if (e0.active(lane) && (lane & (gw - 1)) == 0)
+      st_relaxed(&out[(size_t)(kPlain ? e0.v : e0.slot()) * vs], kForward ? e0.a + acc : e0.a * e0.own + acc);
     e0 = e1;
     r1 = r2;
   }

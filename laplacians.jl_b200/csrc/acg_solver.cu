@@ -381,7 +381,8 @@ void enqueue_syncfree(cudaStream_t s, const SolverImpl& S, const T* aux, const T
   cfg.numAttrs = 1;
   const DevSweep& P = S.sweep[0];
   const SweepTask* tasks = (kForward ? P.tasks_f.p : P.tasks_b.p) + t0;
-  ACG_CUDA(cudaLaunchKernelEx(&cfg, k_sweep<T, kForward>, t1 - t0, tasks,
+  const auto kern = S.two_plans ? k_sweep<T, kForward, false> : k_sweep<T, kForward, true>;
+  ACG_CUDA(cudaLaunchKernelEx(&cfg, kern, t1 - t0, tasks,
                               (const int*)(kForward ? P.f_idx.p : P.b_idx.p), P.coef<T>(kForward), aux, sfwd, out, st,
                               S.poll_mode, vs, S.spin_limit));
 }
@@ -1483,10 +1484,13 @@ void build_solver(SolverImpl& S, int64_t n64, const int64_t* a_colptr, const int
     int sms = 0;
     ACG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, S.device));
     int occ[4] = {0, 0, 0, 0};
-    ACG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ[0], k_sweep<double, true>, kSweepThreads, 0));
-    ACG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ[1], k_sweep<double, false>, kSweepThreads, 0));
-    ACG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ[2], k_sweep<float, true>, kSweepThreads, 0));
-    ACG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ[3], k_sweep<float, false>, kSweepThreads, 0));
+    auto fit = [&](int& n, auto merged, auto plain) {
+      ACG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, merge ? merged : plain, kSweepThreads, 0));
+    };
+    fit(occ[0], k_sweep<double, true, false>, k_sweep<double, true, true>);
+    fit(occ[1], k_sweep<double, false, false>, k_sweep<double, false, true>);
+    fit(occ[2], k_sweep<float, true, false>, k_sweep<float, true, true>);
+    fit(occ[3], k_sweep<float, false, false>, k_sweep<float, false, true>);
     // Resident blocks (8 warps each) per SM: a deep, narrow DAG gains nothing
     // from more warps (they add polling traffic without shortening the chains),
     // a wide one is throughput-bound in its wide levels and gains from them.
