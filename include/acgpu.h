@@ -313,8 +313,8 @@ int acg_ldlsolve(acg_solver* h, const double* r, double* y, int precision);
 int acg_lap_mul(acg_solver* h, const double* x, double* y, int precision);
 /* Time the solve's kernels: each captured `reps` times into a CUDA graph and
  * timed with CUDA events on the solver's stream (no reference counterpart).
- * One-vector solves run their whole PCG in one launch; the times here are of
- * the same phases as separate launches. */
+ * One-vector solves run their PCG in launches of up to a millisecond; the
+ * times here are of the same phases as separate launches. */
 int acg_time_kernels(acg_solver* h, int precision, int reps, acg_kernel_times* out);
 /* The same for the batched kernels with nrhs (<= 64) right-hand sides
  * (iteration_ms is not measured there). */
@@ -360,7 +360,8 @@ int acg_time_sweep_levels(acg_solver* h, int precision, int nrhs, int reps, int 
  *     next request relaunches it) and right-hand sides finished.
  *   acg_serve_close: waits for the loop to go idle and frees it; every
  *     ticket must have been waited (else ACG_ERR_BUSY).  acg_destroy closes a
- *     solver's open loop. */
+ *     solver's open loop after serving the requests it holds; their tickets
+ *     are waited as ever, the server itself is gone with the last. */
 typedef struct acg_server acg_server;
 typedef struct acg_ticket acg_ticket;
 int acg_serve_open(acg_solver* h, int precision, int slots, int queue, acg_server** out);
